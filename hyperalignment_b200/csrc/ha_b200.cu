@@ -8,6 +8,7 @@
 
 #include "../../include/hyperalignment_b200.h"
 #include "ha_b200_kernels.cuh"
+#include "ha_b200_dgemm.cuh"
 #include "ha_b200_grid.cuh"
 #include "ha_b200_mlp.cuh"
 #include "ha_b200_tc.cuh"
@@ -592,6 +593,8 @@ int set_smem_attrs() {
 	HA_CUDA(cudaFuncSetAttribute(k_reduce<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
 	HA_CUDA(cudaFuncSetAttribute(k_reduce<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
 	HA_CUDA(cudaFuncSetAttribute(k_pattern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
+	HA_CUDA(cudaFuncSetAttribute(k_ridge_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
+	HA_CUDA(cudaFuncSetAttribute(k_ridge_chol, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRidgeSmem));
 	HA_CUDA(cudaFuncSetAttribute(k_pchol<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kPcholNb * kGridMaxN * 8)));
 	HA_CUDA(cudaFuncSetAttribute(k_pchol<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kPcholNb * kGridMaxN * 4)));
 	done = true;
@@ -1400,9 +1403,13 @@ int run_ridge(HaB200Plan *P, const double *d_X, const double *d_Y, double alpha,
 			const Bucket &b = ch.b64[bi];
 			const cudaStream_t bs = g_fan.at((int)bi);
 			const SlWork *wk = ch.d_w64 + b.first;
-			{ HA_LAUNCH(kHaB200KXcov64, bs); k_xcov<double, 16><<<b.count, kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_X, nt, nt, G, P->stats.p, 0); }
-			{ HA_LAUNCH(kHaB200KXcov64, bs); k_xcov<double, 16><<<b.count, kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_Y, nt, nt, R, P->stats.p, 0); }
-			{ HA_LAUNCH(kHaB200KRidge, bs); k_ridge_chol<<<b.count, kBlock, 0, bs>>>(wk, G, R, P->scrT64.p, alpha, rowmajor, P->stats.p); }
+			// a bucket's items are sorted by size, the widest first: at most 65,535 of them per launch
+			const int tw = (ch.w64[b.first].n + kDgTile - 1) / kDgTile, tiles = tw * (tw + 1) / 2 + tw * tw;
+			for (int x = 0; x < b.count; x += 65535) {
+				HA_LAUNCH(kHaB200KXcov64, bs);
+				k_ridge_gram<<<dim3(tiles, std::min(b.count - x, 65535)), kDgThreads, kDgSmem, bs>>>(wk + x, P->idx.p, d_X, d_Y, nt, G, R);
+			}
+			{ HA_LAUNCH(kHaB200KRidge, bs); k_ridge_chol<<<b.count, kDgThreads, kRidgeSmem, bs>>>(wk, G, R, P->scrT64.p, alpha, rowmajor, P->stats.p); }
 		}
 		if ((rc = g_fan.end(st)) != kHaSuccess) return rc;
 		{ HA_LAUNCH(kHaB200KScale, st); k_scale<<<(nsl + 127) / 128, 128, 0, st>>>(ch.d_w64, nsl, P->idx.p, nullptr, P->stats.p, nt, 0, P->scale.p); }

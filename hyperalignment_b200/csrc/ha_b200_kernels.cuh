@@ -1331,88 +1331,6 @@ __global__ void __launch_bounds__(256) k_reduce(const int64_t *__restrict__ vl_p
 }
 
 // ---------------------------------------------------------------------------------------------
-// ridge  beta_s = (X_s^T X_s + alpha I)^-1 X_s^T Y_s   (csrc/ha_ridge.c:13-54, float64)
-// ---------------------------------------------------------------------------------------------
-// The reference computes V diag(s / (alpha + s^2)) U^T Y from the thin SVD X_s = U diag(s) V^T;
-// for alpha > 0 that is exactly the solution of the regularised normal equations, solved here
-// by a Cholesky factorisation of G + alpha I (G = X_s^T X_s in the A scratch, column-major) and
-// two triangular solves with the n right-hand sides X_s^T Y_s (in the V scratch, column-major:
-// column j holds right-hand side j).  One CTA per searchlight, float64 throughout, the factor
-// overwriting G in place.  beta is written (float64) in the T layout: row-major for CSR output
-// (row i = source vertex i), column-major for CSC output.  A non-positive pivot (alpha = 0 with a
-// rank-deficient X_s) marks the searchlight kFlagUnconverged and writes zeros.
-__global__ void __launch_bounds__(256) k_ridge_chol(const SlWork *__restrict__ work, double *__restrict__ Gscr,
-                                                    double *__restrict__ Rscr, double *__restrict__ Bout, double alpha,
-                                                    int t_rowmajor, SlStats *__restrict__ stats) {
-	const SlWork w = work[blockIdx.x];
-	const int n = w.n;
-	double *G = Gscr + w.aofs;  // G[c * n + r] = G(r, c); lower triangle used
-	double *R = Rscr + w.aofs;  // R[j * n + i] = rhs(i, j)
-	__shared__ int bad;
-	__shared__ double piv;
-	if (threadIdx.x == 0) bad = 0;
-	for (int k = threadIdx.x; k < n; k += blockDim.x) G[(int64_t)k * n + k] += alpha;
-	__syncthreads();
-	// right-looking Cholesky, column k at a time
-	for (int k = 0; k < n; k++) {
-		if (threadIdx.x == 0) {
-			double d = G[(int64_t)k * n + k];
-			if (!(d > 0.0)) {
-				bad = 1;
-				d = 1.0;
-			}
-			piv = sqrt(d);
-			G[(int64_t)k * n + k] = piv;
-		}
-		__syncthreads();
-		const double p = piv;
-		for (int r = k + 1 + threadIdx.x; r < n; r += blockDim.x) G[(int64_t)k * n + r] /= p;
-		__syncthreads();
-		const int m = n - k - 1;
-		for (int64_t e = threadIdx.x; e < (int64_t)m * m; e += blockDim.x) {
-			const int c = k + 1 + (int)(e / m), r = k + 1 + (int)(e % m);
-			if (r >= c) G[(int64_t)c * n + r] -= G[(int64_t)k * n + r] * G[(int64_t)k * n + c];
-		}
-		__syncthreads();
-	}
-	// forward solve L Z = rhs (all n right-hand sides), Z over R
-	for (int k = 0; k < n; k++) {
-		const double lkk = G[(int64_t)k * n + k];
-		for (int j = threadIdx.x; j < n; j += blockDim.x) R[(int64_t)j * n + k] /= lkk;
-		__syncthreads();
-		const int m = n - k - 1;
-		for (int64_t e = threadIdx.x; e < (int64_t)m * n; e += blockDim.x) {
-			const int j = (int)(e / m), r = k + 1 + (int)(e % m);
-			R[(int64_t)j * n + r] -= G[(int64_t)k * n + r] * R[(int64_t)j * n + k];
-		}
-		__syncthreads();
-	}
-	// backward solve L^T beta = Z
-	for (int k = n - 1; k >= 0; k--) {
-		const double lkk = G[(int64_t)k * n + k];
-		for (int j = threadIdx.x; j < n; j += blockDim.x) R[(int64_t)j * n + k] /= lkk;
-		__syncthreads();
-		for (int64_t e = threadIdx.x; e < (int64_t)k * n; e += blockDim.x) {
-			const int j = (int)(e / k), r = (int)(e % k);
-			R[(int64_t)j * n + r] -= G[(int64_t)r * n + k] * R[(int64_t)j * n + k];
-		}
-		__syncthreads();
-	}
-	double *Bo = Bout + w.tofs;
-	const int64_t ti = t_rowmajor ? n : 1, tj = t_rowmajor ? 1 : n;
-	for (int64_t e = threadIdx.x; e < (int64_t)n * n; e += blockDim.x) {
-		const int j = (int)(e / n), i = (int)(e % n);
-		Bo[i * ti + j * tj] = bad ? 0.0 : R[e];
-	}
-	if (threadIdx.x == 0) {
-		SlStats st = stats[w.slot];
-		st.s_sum = 0.0;
-		st.flags = bad ? (kFlagUnconverged | kFlagFP64) : kFlagFP64;
-		stats[w.slot] = st;
-	}
-}
-
-// ---------------------------------------------------------------------------------------------
 // template loop helpers (csrc/ha_template.c:14-114 with searchlight solves)
 // ---------------------------------------------------------------------------------------------
 

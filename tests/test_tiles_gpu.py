@@ -1,0 +1,60 @@
+"""The blocked kernels at the edges of their tiles, against the CPU oracle."""
+
+import numpy as np
+import pytest
+
+from hyperalignment_b200 import _lib as L
+from hyperalignment_b200.plan import Plan
+from oracle import ha_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def one_each(sizes, nt, seed):
+    """Gaussian series and one searchlight of every size over a common vertex set."""
+    rng = np.random.default_rng(seed)
+    nv = max(sizes)
+    X, Y = rng.standard_normal((nt, nv)), rng.standard_normal((nt, nv))
+    idx = np.concatenate([np.sort(rng.choice(nv, n, replace=False)) for n in sizes]).astype(np.int32)
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    return X, Y, idx, off
+
+
+def upload(X):
+    import torch
+    return torch.from_numpy(np.asfortranarray(X).ravel(order="F")).cuda()
+
+
+# A Gaussian X of 700 samples has cond(X^T X) < 200 for n <= 512, so normal equations solved in
+# float64 carry at most about 200 * 512 * 2.2e-16 = 2e-11; four times that is allowed.
+@pytest.mark.parametrize("csc", [False, True])
+def test_ridge_tile_edges(gpu, csc):
+    import torch
+    sizes = [1, 2, 31, 63, 64, 65, 127, 128, 129, 200, 255, 257, 511, 512]
+    X, Y, idx, off = one_each(sizes, 700, 3)
+    dX, dY = upload(X), upload(Y)
+    for s, n in enumerate(sizes):
+        sl = idx[off[s]:off[s + 1]]
+        plan = Plan(700, X.shape[1], sl, np.array([0, n]), weights=np.ones(n))
+        vals = torch.zeros(plan.nnz, dtype=torch.float64, device="cuda")
+        plan.ridge_device(dX.data_ptr(), dY.data_ptr(), vals.data_ptr(), 0.5,
+                          out_kind=L.OUT_CSC if csc else L.OUT_CSR)
+        got = vals.cpu().numpy().reshape(n, n)
+        plan.close()
+        ref = O.ridge(X[:, sl], Y[:, sl], 0.5)
+        err = np.linalg.norm((got.T if csc else got) - ref) / np.linalg.norm(ref)
+        assert err <= 8e-11, (n, err)
+
+
+def test_ridge_without_penalty_on_singular_data_writes_zeros(gpu):
+    import torch
+    rng = np.random.default_rng(4)
+    X, Y = rng.standard_normal((300, 130)), rng.standard_normal((300, 130))
+    X[:, 100] = 0.0
+    dX, dY = upload(X), upload(Y)
+    plan = Plan(300, 130, np.arange(130), np.array([0, 130]), weights=np.ones(130))
+    vals = torch.zeros(plan.nnz, dtype=torch.float64, device="cuda")
+    plan.ridge_device(dX.data_ptr(), dY.data_ptr(), vals.data_ptr(), 0.0)
+    assert plan.stats()["n_unconverged"] == 1
+    assert not vals.any()
+    plan.close()
