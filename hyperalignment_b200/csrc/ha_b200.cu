@@ -9,6 +9,8 @@
 #include "../../include/hyperalignment_b200.h"
 #include "ha_b200_kernels.cuh"
 #include "ha_b200_dgemm.cuh"
+#include "ha_b200_eig.cuh"
+#include "ha_b200_polar.cuh"
 #include "ha_b200_grid.cuh"
 #include "ha_b200_mlp.cuh"
 #include "ha_b200_tc.cuh"
@@ -260,6 +262,40 @@ int jacobi_threads(int bsz, bool fp64) {
 	(void)fp64;
 	warps = std::max(8, std::min(16, warps));
 	return warps * 32;
+}
+
+// Eigen decompositions of the matrices of a work list sorted by order, the largest first (orders:
+// their orders in that sequence), cut into size classes that run on the side streams.
+int launch_eig(const EigWork *d_work, const std::vector<int> &orders, double *A, double *Q, double *S, double *lam,
+               cudaStream_t st) {
+	int rc = g_fan.begin(st);
+	if (rc != kHaSuccess) return rc;
+	int i = 0, cls = 0;
+	for (int lo : {384, 256, 192, 128, 64, 0}) {
+		int j = i;
+		while (j < (int)orders.size() && orders[j] > lo) j++;
+		for (; i < j; i += std::min(j - i, 65535)) {
+			const int cnt = std::min(j - i, 65535), p = orders[i];
+			const cudaStream_t bs = g_fan.at(cls);
+			const size_t sm = eig_tridiag_smem(p);
+			{
+				HA_LAUNCH(kHaB200KJacobi64, bs);
+				if (lo == 384) k_eig_tridiag<16><<<cnt, kEigThreads, sm, bs>>>(d_work + i, A, Q, S);
+				else if (lo == 256) k_eig_tridiag<12><<<cnt, kEigThreads, sm, bs>>>(d_work + i, A, Q, S);
+				else if (lo == 192) k_eig_tridiag<8><<<cnt, kEigThreads, sm, bs>>>(d_work + i, A, Q, S);
+				else if (lo == 128) k_eig_tridiag<6><<<cnt, kEigThreads, sm, bs>>>(d_work + i, A, Q, S);
+				else if (lo == 64) k_eig_tridiag<4><<<cnt, kEigThreads, sm, bs>>>(d_work + i, A, Q, S);
+				else k_eig_tridiag<2><<<cnt, kEigThreads, sm, bs>>>(d_work + i, A, Q, S);
+			}
+			for (int r = 1; r <= kEigRounds; r++) {
+				{ HA_LAUNCH(kHaB200KJacobi64, bs); k_eig_ql<<<cnt, 32, (size_t)2 * p * sizeof(double), bs>>>(d_work + i, S, lam, r); }
+				{ HA_LAUNCH(kHaB200KJacobi64, bs); k_eig_rotate<<<dim3((p + kEigRows - 1) / kEigRows, cnt), 32, 0, bs>>>(d_work + i, A, Q, S, r); }
+			}
+		}
+		cls++;
+	}
+	HA_CUDA(cudaGetLastError());
+	return g_fan.end(st);
 }
 
 struct Chunk {
@@ -593,6 +629,17 @@ int set_smem_attrs() {
 	HA_CUDA(cudaFuncSetAttribute(k_reduce<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
 	HA_CUDA(cudaFuncSetAttribute(k_reduce<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
 	HA_CUDA(cudaFuncSetAttribute(k_pattern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
+	HA_CUDA(cudaFuncSetAttribute(k_eig_tridiag<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)eig_tridiag_smem(512)));
+	HA_CUDA(cudaFuncSetAttribute(k_eig_tridiag<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)eig_tridiag_smem(384)));
+	HA_CUDA(cudaFuncSetAttribute(k_eig_tridiag<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)eig_tridiag_smem(256)));
+	HA_CUDA(cudaFuncSetAttribute(k_eig_tridiag<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)eig_tridiag_smem(192)));
+	HA_CUDA(cudaFuncSetAttribute(k_eig_tridiag<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)eig_tridiag_smem(128)));
+	HA_CUDA(cudaFuncSetAttribute(k_eig_tridiag<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)eig_tridiag_smem(64)));
+	HA_CUDA(cudaFuncSetAttribute(k_polar_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
+	HA_CUDA(cudaFuncSetAttribute(k_polar_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
+	HA_CUDA(cudaFuncSetAttribute(k_pca_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
+	HA_CUDA(cudaFuncSetAttribute(k_pca_b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
+	HA_CUDA(cudaFuncSetAttribute(k_pca_contrib, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
 	HA_CUDA(cudaFuncSetAttribute(k_ridge_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
 	HA_CUDA(cudaFuncSetAttribute(k_ridge_chol, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRidgeSmem));
 	HA_CUDA(cudaFuncSetAttribute(k_pchol<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kPcholNb * kGridMaxN * 8)));
@@ -812,6 +859,79 @@ std::vector<NsStep> ns_schedule() {
 		l = std::min(1.0, 0.5 * a * l * (3.0 - a * a * l * l));
 	}
 	return out;
+}
+
+// Work lists and device buffers of a batch of float64 polar factors (ha_b200_polar.cuh).
+struct PolarBufs {
+	DevArr<PolarWork> work;
+	DevArr<PolarTile> low, all;
+	DevArr<PolarState> state;
+	DevArr<double> part;
+	DevArr<int32_t> left;
+	void release() { work.release(); low.release(); all.release(); state.release(); part.release(); left.release(); }
+};
+
+// Polar factors of the matrices B into T (float), flags into stats; items sorted by size, the
+// largest first.  The host waits for the count of unfinished matrices every other iteration from the
+// first plain step on, so it enqueues no iteration that no matrix needs.
+int polar_solve(PolarBufs &pb, std::vector<PolarWork> &items, const double *B, double *S, float *T, SlStats *stats,
+                cudaStream_t st) {
+	const int n = (int)items.size();
+	std::vector<PolarTile> low, all;
+	int parts = 0;
+	for (int q = 0; q < n; q++) {
+		const int t = (items[q].n + kDgTile - 1) / kDgTile;
+		items[q].part = parts;
+		for (int i = 0; i < t * (t + 1) / 2; i++) low.push_back({q, i});
+		for (int i = 0; i < t * t; i++) all.push_back({q, i});
+		parts += t * (t + 1) / 2;
+	}
+	int rc;
+	if ((rc = pb.work.ensure(n)) != kHaSuccess || (rc = pb.low.ensure(low.size())) != kHaSuccess ||
+	    (rc = pb.all.ensure(all.size())) != kHaSuccess || (rc = pb.state.ensure(2 * (size_t)n)) != kHaSuccess ||
+	    (rc = pb.part.ensure(parts)) != kHaSuccess || (rc = pb.left.ensure(1)) != kHaSuccess)
+		return rc;
+	HA_CUDA(cudaMemcpyAsync(pb.work.p, items.data(), n * sizeof(PolarWork), cudaMemcpyHostToDevice, st));
+	HA_CUDA(cudaMemcpyAsync(pb.low.p, low.data(), low.size() * sizeof(PolarTile), cudaMemcpyHostToDevice, st));
+	HA_CUDA(cudaMemcpyAsync(pb.all.p, all.data(), all.size() * sizeof(PolarTile), cudaMemcpyHostToDevice, st));
+	PolarArgs a = {};
+	a.work = pb.work.p;
+	a.B = B;
+	a.S = S;
+	a.T = T;
+	a.part = pb.part.p;
+	a.left = pb.left.p;
+	a.out = pb.state.p;
+	{ HA_LAUNCH(kHaB200KPca, st); k_polar_init<<<n, 256, 0, st>>>(a); }
+	const std::vector<NsStep> sched = ns_schedule();
+	const int maxit = (int)sched.size();
+	int k = 0;
+	for (; k < maxit; k++) {
+		a.in = pb.state.p + (k & 1) * (size_t)n;
+		a.out = pb.state.p + ((k + 1) & 1) * (size_t)n;
+		a.odd = k & 1;
+		a.c1 = sched[k].c1;
+		a.c3 = sched[k].c3;
+		a.plain = sched[k].plain;
+		a.last = k == maxit - 1;
+		HA_CUDA(cudaMemsetAsync(pb.left.p, 0, sizeof(int32_t), st));
+		a.tiles = pb.low.p;
+		{ HA_LAUNCH(kHaB200KPca, st); k_polar_gram<<<(int)low.size(), kDgThreads, kDgSmem, st>>>(a); }
+		a.tiles = pb.all.p;
+		{ HA_LAUNCH(kHaB200KPca, st); k_polar_update<<<(int)all.size(), kDgThreads, kDgSmem, st>>>(a); }
+		if (sched[k].plain && (k & 1)) {
+			int32_t left = 0;
+			HA_CUDA(cudaMemcpyAsync(&left, pb.left.p, sizeof(left), cudaMemcpyDeviceToHost, st));
+			HA_CUDA(cudaStreamSynchronize(st));
+			if (left == 0) {
+				k++;
+				break;
+			}
+		}
+	}
+	{ HA_LAUNCH(kHaB200KPca, st); k_polar_finish<<<(n + 127) / 128, 128, 0, st>>>(pb.work.p, n, pb.state.p + (k & 1) * (size_t)n, stats); }
+	HA_CUDA(cudaGetLastError());
+	return kHaSuccess;
 }
 
 // Residual ||G - I||_F / sqrt(n) below which a plain step is the last (HA_B200_NS_TOL).  The
@@ -2400,8 +2520,8 @@ int template_impl(const double *dms, int ns, int nt, int nv, const int32_t *idx,
 
 // Searchlight PCA template (src/hyperalignment/searchlight.py:215-236, tpl_kind="pca"), float64
 // throughout.  Consecutive searchlights form batches sized to the scratch budget; per batch: the
-// Gram of the smaller side (k_pca_gram), its pivoted Cholesky factor and eigenvector-mode Jacobi,
-// the template and B = tmpl^T M (k_pca_tmpl), the float64 Jacobi polar of B, C = tmpl R
+// Gram of the smaller side (k_pca_gram), its eigen decomposition, the template (k_pca_tmpl) and
+// B = tmpl^T M (k_pca_b), the float64 polar factor of B, C = tmpl R
 // (k_pca_contrib) and the weighted per-vertex reduction into the template (k_pca_reduce).
 int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *idx, const int32_t *off,
                       const double *dists, int count, double radius, double *tpl_out) {
@@ -2427,14 +2547,14 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 		nn[s] = n;
 		mg[s] = n > 0 ? m : nt;
 		if (n == 0) { region[s] = ptot[s] = 0; bytes[s] = 0; continue; }
-		int be, ke, bp, kp;
-		size_t me, mp;
-		jacobi_layout(m, true, be, ke, me, kSmemMax, false);
+		int bp, kp;
+		size_t mp;
 		jacobi_layout(n, true, bp, kp, mp);
-		int64_t r = std::max<int64_t>((int64_t)m * std::max(m, be * ke), (int64_t)n * kp * bp);
+		int64_t r = std::max<int64_t>((int64_t)m * m, (int64_t)n * kp * bp);
 		region[s] = (r + 31) & ~(int64_t)31;
 		ptot[s] = PcaLayout::make(nt, n, m, m != nt).total;
-		bytes[s] = (size_t)(2 * region[s] + ptot[s] + m + 2 * n) * 8 + (size_t)n * n * 4 + 2 * sizeof(SlStats);
+		bytes[s] = (size_t)(2 * region[s] + ptot[s] + m + 2 * n + EigScratch::make(m).total) * 8 + (size_t)n * n * 4 +
+		           2 * sizeof(SlStats);
 	}
 	// batches of consecutive searchlights
 	const size_t budget = scratch_budget_bytes();
@@ -2450,12 +2570,13 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 		}
 		bstart.push_back(count);
 	}
-	int64_t maxR = 1, maxP = 1, maxT = 1, maxUV = 1;
+	int64_t maxR = 1, maxP = 1, maxT = 1, maxUV = 1, maxE = 1;
 	int maxS = 1;
 	for (size_t b = 0; b + 1 < bstart.size(); b++) {
-		int64_t R = 0, Pt = 0, Tt = 0, U = 0;
+		int64_t R = 0, Pt = 0, Tt = 0, U = 0, E = 0;
 		for (int s = bstart[b]; s < bstart[b + 1]; s++) {
 			R += region[s];
+			E += nn[s] > 0 ? EigScratch::make(mg[s]).total : 0;
 			Pt += ptot[s];
 			Tt += (int64_t)nn[s] * nn[s];
 			U += nn[s] > 0 ? mg[s] + 2 * nn[s] : 0;
@@ -2464,27 +2585,30 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 		maxP = std::max(maxP, Pt);
 		maxT = std::max(maxT, Tt);
 		maxUV = std::max(maxUV, U);
+		maxE = std::max(maxE, E);
 		maxS = std::max(maxS, bstart[b + 1] - bstart[b]);
 	}
 	const size_t m1 = (size_t)nt * nv;
-	DevArr<double> D, eA, eV, Pw, uvb, tpl;
+	DevArr<double> D, eA, eV, eS, Pw, uvb, tpl;
 	DevArr<float> T;
-	DevArr<SlStats> stE, stP;
-	DevArr<SlWork> dwe, dwp, dwes, dwps;
+	DevArr<SlStats> stP;
+	DevArr<SlWork> dwe, dwp, dwps;
+	DevArr<EigWork> deig;
+	PolarBufs polar;
 	DevArr<int64_t> dpofs;
 	DevArr<int32_t> dmg;
 	auto done = [&](int code) {
-		D.release(); eA.release(); eV.release(); Pw.release(); uvb.release(); tpl.release(); T.release();
-		stE.release(); stP.release(); dwe.release(); dwp.release(); dwes.release(); dwps.release();
+		D.release(); eA.release(); eV.release(); eS.release(); Pw.release(); uvb.release(); tpl.release(); T.release();
+		stP.release(); dwe.release(); dwp.release(); dwps.release(); deig.release(); polar.release();
 		dpofs.release(); dmg.release();
 		return code;
 	};
 	if ((rc = D.ensure(m1 * ns)) != kHaSuccess || (rc = tpl.ensure(m1)) != kHaSuccess ||
 	    (rc = eA.ensure((size_t)maxR)) != kHaSuccess || (rc = eV.ensure((size_t)maxR)) != kHaSuccess ||
 	    (rc = Pw.ensure((size_t)maxP)) != kHaSuccess || (rc = uvb.ensure((size_t)maxUV)) != kHaSuccess ||
-	    (rc = T.ensure((size_t)maxT)) != kHaSuccess || (rc = stE.ensure((size_t)maxS)) != kHaSuccess ||
+	    (rc = T.ensure((size_t)maxT)) != kHaSuccess || (rc = eS.ensure((size_t)maxE)) != kHaSuccess ||
 	    (rc = stP.ensure((size_t)maxS)) != kHaSuccess || (rc = dwe.ensure((size_t)maxS)) != kHaSuccess ||
-	    (rc = dwp.ensure((size_t)maxS)) != kHaSuccess || (rc = dwes.ensure((size_t)maxS)) != kHaSuccess ||
+	    (rc = dwp.ensure((size_t)maxS)) != kHaSuccess || (rc = deig.ensure((size_t)maxS)) != kHaSuccess ||
 	    (rc = dwps.ensure((size_t)maxS)) != kHaSuccess || (rc = dpofs.ensure((size_t)maxS)) != kHaSuccess ||
 	    (rc = dmg.ensure((size_t)maxS)) != kHaSuccess)
 		return done(rc);
@@ -2492,14 +2616,13 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 	if (cudaMemcpyAsync(D.p, dms, m1 * ns * 8, cudaMemcpyHostToDevice, st) != cudaSuccess ||
 	    cudaMemsetAsync(tpl.p, 0, m1 * 8, st) != cudaSuccess)
 		return done(kHaErrorInternal);
-	const JacobiParams jpe = eig_params(false);
 	JacobiParams jpp;
 	jpp.max_sweeps = 40;
 	jpp.t_rowmajor = 0;
 	jpp.ill_ratio = 0.0;
 	jpp.weak = weak_factor();
 	jpp.eig = 0;
-	jpp.only_flagged = 0;
+	jpp.only_flagged = 1;
 	jpp.keep_v = 0;
 	jpp.warm = 0;
 	jpp.stop_cos = fp64_stop_cos();
@@ -2508,7 +2631,9 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 		std::vector<SlWork> we, wp;
 		std::vector<int64_t> pofs(s_hi - s_lo, 0);
 		std::vector<int32_t> mgb(s_hi - s_lo);
-		int64_t ro = 0, po = 0, to = 0, uo = 0;
+		std::vector<EigWork> eig;
+		std::vector<PolarWork> pol;
+		int64_t ro = 0, po = 0, to = 0, uo = 0, eo = 0;
 		for (int s = s_lo; s < s_hi; s++) {
 			const int q = s - s_lo, n = nn[s], m = mg[s];
 			mgb[q] = m;
@@ -2524,11 +2649,13 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 			{
 				int bb, kk;
 				size_t mm;
-				jacobi_layout(m, true, bb, kk, mm, kSmemMax, false);
-				e.bsz = bb; e.nblk = kk;
 				jacobi_layout(n, true, bb, kk, mm);
-				p.bsz = bb; p.nblk = kk;
+				p.bsz = e.bsz = bb;
+				p.nblk = e.nblk = kk;
 			}
+			eig.push_back({ro, ro, eo, uo, m, 0});
+			pol.push_back({ro, eo, eo + (int64_t)n * n, eo + 2 * (int64_t)n * n, to, n, q, 0, 0});
+			eo += EigScratch::make(m).total;
 			e.uvofs = uo;
 			p.uvofs = uo + m;
 			we.push_back(e);
@@ -2541,26 +2668,39 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 		}
 		const int nb = (int)we.size();
 		if (nb == 0) continue;
-		std::vector<SlWork> wes = we, wps = wp;
-		const std::vector<Bucket> be = bucketize(wes, 2), bp = bucketize(wps, 1);
+		std::vector<SlWork> wps = wp;
+		const std::vector<Bucket> bp = bucketize(wps, 1);
+		std::stable_sort(eig.begin(), eig.end(), [](const EigWork &a, const EigWork &b) { return a.p > b.p; });
+		std::stable_sort(pol.begin(), pol.end(), [](const PolarWork &a, const PolarWork &b) { return a.n > b.n; });
+		std::vector<int> orders(eig.size());
+		for (size_t k = 0; k < eig.size(); k++) orders[k] = eig[k].p;
 		if (cudaMemcpyAsync(dwe.p, we.data(), nb * sizeof(SlWork), cudaMemcpyHostToDevice, st) != cudaSuccess ||
 		    cudaMemcpyAsync(dwp.p, wp.data(), nb * sizeof(SlWork), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-		    cudaMemcpyAsync(dwes.p, wes.data(), nb * sizeof(SlWork), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+		    cudaMemcpyAsync(deig.p, eig.data(), nb * sizeof(EigWork), cudaMemcpyHostToDevice, st) != cudaSuccess ||
 		    cudaMemcpyAsync(dwps.p, wps.data(), nb * sizeof(SlWork), cudaMemcpyHostToDevice, st) != cudaSuccess ||
 		    cudaMemcpyAsync(dpofs.p, pofs.data(), pofs.size() * 8, cudaMemcpyHostToDevice, st) != cudaSuccess ||
 		    cudaMemcpyAsync(dmg.p, mgb.data(), mgb.size() * 4, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-		    cudaMemsetAsync(stE.p, 0, (size_t)(s_hi - s_lo) * sizeof(SlStats), st) != cudaSuccess ||
 		    cudaMemsetAsync(stP.p, 0, (size_t)(s_hi - s_lo) * sizeof(SlStats), st) != cudaSuccess)
 			return done(kHaErrorInternal);
-		{ HA_LAUNCH(kHaB200KPca, st); k_pca_gram<16><<<nb, kBlock, 0, st>>>(dwe.p, P->idx.p, P->off.p, D.p, ns, nt, nv, eV.p); }
-		for (const Bucket &k : be) {
-			const SlWork *wk = dwes.p + k.first;
-			{ HA_LAUNCH(kHaB200KRidge, st); k_pchol<double><<<k.count, kBlock, pchol_smem(k.rpl), st>>>(wk, eV.p, eA.p, stE.p); }
-			HA_LAUNCH(kHaB200KJacobi64, st);
-			if ((rc = launch_jacobi<double>(k.rpl, k.count, k.threads, k.smem, st, wk, eA.p, eV.p, T.p, stE.p, uvb.p, jpe)) != kHaSuccess)
-				return done(rc);
+		int nw = 1, mw = 1;  // widest searchlight and Gram order of the batch
+		for (int k = 0; k < nb; k++) {
+			nw = std::max(nw, wp[k].n);
+			mw = std::max(mw, we[k].n);
 		}
-		{ HA_LAUNCH(kHaB200KPca, st); k_pca_tmpl<<<nb, kBlock, 0, st>>>(dwe.p, dwp.p, P->idx.p, D.p, ns, nt, nv, eV.p, uvb.p, dpofs.p, Pw.p, eA.p); }
+		const int tn = (nw + kDgTile - 1) / kDgTile, tm = (mw + kDgTile - 1) / kDgTile, tt = (nt + kDgTile - 1) / kDgTile;
+		for (int x = 0; x < nb; x += 65535) {
+			HA_LAUNCH(kHaB200KPca, st);
+			k_pca_gram<<<dim3(tm * (tm + 1) / 2, std::min(nb - x, 65535)), kDgThreads, kDgSmem, st>>>(dwe.p + x, P->idx.p, P->off.p, D.p, ns, nt, nv, eV.p);
+		}
+		if ((rc = launch_eig(deig.p, orders, eV.p, eA.p, eS.p, uvb.p, st)) != kHaSuccess) return done(rc);
+		{ HA_LAUNCH(kHaB200KPca, st); k_pca_tmpl<<<nb, kBlock, 0, st>>>(dwe.p, dwp.p, P->idx.p, D.p, ns, nt, nv, eV.p, uvb.p, dpofs.p, Pw.p); }
+		for (int x = 0; x < nb; x += 65535) {
+			HA_LAUNCH(kHaB200KPca, st);
+			k_pca_b<<<dim3(tn * tn, std::min(nb - x, 65535)), kDgThreads, kDgSmem, st>>>(dwe.p + x, dwp.p + x, nt, dpofs.p, Pw.p, eA.p);
+		}
+		// the eigen decomposition's scratch holds the iterates (it is at least 4 m^2 per searchlight)
+		if ((rc = polar_solve(polar, pol, eA.p, eS.p, T.p, stP.p, st)) != kHaSuccess) return done(rc);
+		// the flagged ones by Jacobi
 		for (const Bucket &k : bp) {
 			const SlWork *wk = dwps.p + k.first;
 			{
@@ -2568,9 +2708,13 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 				if ((rc = launch_jacobi<double>(k.rpl, k.count, k.threads, k.smem, st, wk, eA.p, eV.p, T.p, stP.p, uvb.p, jpp)) != kHaSuccess)
 					return done(rc);
 			}
-			if (k.blocked) { HA_LAUNCH(kHaB200KFormT64, st); k_form_t_global<double><<<k.count, kBlock, 0, st>>>(wk, eA.p, eV.p, T.p, stP.p, 0, 0); }
+			if (k.blocked) { HA_LAUNCH(kHaB200KFormT64, st); k_form_t_global<double><<<k.count, kBlock, 0, st>>>(wk, eA.p, eV.p, T.p, stP.p, 0, 1); }
 		}
-		{ HA_LAUNCH(kHaB200KPca, st); k_pca_contrib<<<nb, kBlock, 0, st>>>(dwe.p, dwp.p, T.p, nt, dpofs.p, Pw.p); }
+		{ HA_LAUNCH(kHaB200KPca, st); k_pca_widen<<<nb, kBlock, 0, st>>>(dwe.p, dwp.p, T.p, nt, dpofs.p, Pw.p); }
+		for (int x = 0; x < nb; x += 65535) {
+			HA_LAUNCH(kHaB200KPca, st);
+			k_pca_contrib<<<dim3(tt * tn, std::min(nb - x, 65535)), kDgThreads, kDgSmem, st>>>(dwe.p + x, dwp.p + x, nt, dpofs.p, Pw.p);
+		}
 		{ HA_LAUNCH(kHaB200KPca, st); k_pca_reduce<<<nv, kBlock, 0, st>>>(P->vlptr.p, P->vlent.p, P->off.p, P->has_weights ? P->w.p : nullptr,
 		                                                              dpofs.p, dmg.p, Pw.p, nt, s_lo, s_hi, tpl.p); }
 		// the host work lists are rebuilt for the next batch

@@ -45,8 +45,9 @@ __device__ __forceinline__ void dg_cp8(double *dst, const double *src, bool ok) 
 }
 
 // The thread's share of an operand tile: 8 elements of every K slice.
-template <bool KC>
+template <bool KC_>
 struct DgLoader {
+	static constexpr bool KC = KC_;
 	const double *p[KC ? 8 : 1];
 	int64_t ld;
 	uint32_t ok;  // rows inside the operand (KC: one bit per element)
@@ -103,22 +104,21 @@ __device__ __forceinline__ void dg_mma(double (&c)[4], const double (&a)[4], con
 // acc(i, j) += sum_k A(m0 + i, k) B(n0 + j, k) over k in [0, K) for this thread's 32 elements of the
 // 64 x 64 tile: warp w covers rows 32 (w & 1).. and columns 32 (w >> 1).., acc[u][v][e] is row
 // 16 u + g + 8 (e >> 1), column 8 v + 2 t + (e & 1) of that 32 x 32 block (g = lane / 4, t = lane % 4).
-// Ends with a barrier, so the stages may be reused at once.
-template <bool AKC, bool BKC>
-__device__ __forceinline__ void dgemm_tile(const DgOperand &A, int m0, const DgOperand &B, int n0, int K, double *sm,
+// Ends with a barrier, so the stages may be reused at once.  la and lb load the operands' K slices
+// (their rows already placed at m0 and n0); `safe` is any readable address, the source of the
+// zero-size copies of elements outside an operand.
+template <typename LA, typename LB>
+__device__ __forceinline__ void dgemm_core(const LA &la, const LB &lb, int K, const double *safe, double *sm,
                                            double (&acc)[2][4][4]) {
+	constexpr bool AKC = LA::KC, BKC = LB::KC;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int g = lane >> 2, t = lane & 3, wm = 32 * (warp & 1), wn = 32 * (warp >> 1);
-	DgLoader<AKC> la;
-	DgLoader<BKC> lb;
-	la.init(A, m0, tid);
-	lb.init(B, n0, tid);
 	const int nk = (K + kDgK - 1) / kDgK;
 	auto fill = [&](int s) {
 		if (s < nk) {
 			double *st = sm + (s % kDgStages) * 2 * kDgOperand;
-			la.load(st, s * kDgK, K, A.base);
-			lb.load(st + kDgOperand, s * kDgK, K, B.base);
+			la.load(st, s * kDgK, K, safe);
+			lb.load(st + kDgOperand, s * kDgK, K, safe);
 		}
 		asm volatile("cp.async.commit_group;" ::: "memory");
 	};
@@ -148,6 +148,23 @@ __device__ __forceinline__ void dgemm_tile(const DgOperand &A, int m0, const DgO
 	}
 	asm volatile("cp.async.wait_group 0;" ::: "memory");
 	__syncthreads();
+}
+
+template <bool AKC, bool BKC>
+__device__ __forceinline__ void dgemm_tile(const DgOperand &A, int m0, const DgOperand &B, int n0, int K, double *sm,
+                                           double (&acc)[2][4][4]) {
+	DgLoader<AKC> la;
+	DgLoader<BKC> lb;
+	la.init(A, m0, threadIdx.x);
+	lb.init(B, n0, threadIdx.x);
+	dgemm_core(la, lb, K, A.base, sm, acc);
+}
+
+// Lower tile b of a T x T grid: row ti holds ti + 1 tiles.
+__device__ __forceinline__ void dg_lower(int b, int &ti, int &tj) {
+	ti = 0;
+	while (b > ti) b -= ++ti;
+	tj = b;
 }
 
 __device__ __forceinline__ void dg_zero(double (&acc)[2][4][4]) {
@@ -193,9 +210,7 @@ __global__ void __launch_bounds__(kDgThreads) k_ridge_gram(const SlWork *__restr
 	const bool gram = b < low;
 	int ti, tj;
 	if (gram) {
-		ti = 0;
-		while (b > ti) b -= ++ti;  // row ti holds ti + 1 tiles
-		tj = b;
+		dg_lower(b, ti, tj);
 	} else {
 		b -= low;
 		ti = b % T;

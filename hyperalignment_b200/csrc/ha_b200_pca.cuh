@@ -7,8 +7,8 @@
 //   the top n singular pairs of X from the smaller Gram (m = min(nt, ns n) <= 512):
 //     time side   (m = nt):   X X^T = U diag(lambda) U^T,   tmpl = U_n diag(sqrt(lambda_n)) / sqrt(ns)
 //     vertex side (m = ns n): X^T X = W diag(lambda) W^T,   tmpl = X W_n / sqrt(ns)
-//   both by the pivoted Cholesky factor of the Gram and the eigenvector-mode Jacobi (k_pchol,
-//   k_jacobi); then M = sum_j D_j[:, sl], R = polar(tmpl^T M) by the float64 Jacobi polar, and
+//   both by the batched eigen decomposition (ha_b200_eig.cuh); then M = sum_j D_j[:, sl],
+//   R = polar(tmpl^T M) by the float64 Newton-Schulz iteration (ha_b200_polar.cuh), and
 //   template[:, sl] += (tmpl R) diag(w_s) with the searchlight weights, reduced per vertex in
 //   searchlight order.
 // tmpl R depends only on the top-n singular subspace of X (signs and rotations inside a degenerate
@@ -19,11 +19,11 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "ha_b200_kernels.cuh"
+#include "ha_b200_dgemm.cuh"
 
 namespace hab200 {
 
-constexpr int kPcaMaxM = 512;  // Gram order limit (the pivoted Cholesky's shared rank arrays)
+constexpr int kPcaMaxM = 512;  // Gram order limit (kEigMaxP)
 
 // Per-searchlight scratch of the PCA template (float64 elements from the searchlight's base):
 // tmpl (nt x n), M (nt x n), then a work area that first holds the gathered X (nt x m) and the
@@ -49,99 +49,98 @@ __device__ __forceinline__ int64_t pca_col(const int32_t *sl, int n, int64_t pla
 	return (int64_t)j * plane + (int64_t)sl[k - j * n] * nt;
 }
 
-// The Gram of every searchlight of a batch into the V scratch at wm.aofs (m x m, leading dimension
-// m, wm.n = m): X X^T (m = nt, reduction over the ns n columns) or X^T X (m = ns n < nt, reduction
-// over time).  64 x 64 output tiles, the reduction staged KT at a time, loads along time.
-template <int KT>
-__global__ void __launch_bounds__(256) k_pca_gram(const SlWork *__restrict__ wm, const int32_t *__restrict__ sl_idx,
-                                                  const int32_t *__restrict__ off, const double *__restrict__ D,
-                                                  int ns, int nt, int nv, double *__restrict__ Gscr) {
-	const SlWork w = wm[blockIdx.x];
-	const int n = off[w.s + 1] - off[w.s];
-	const int m = w.n;
-	const bool tside = (m == nt);
-	const int32_t *sl = sl_idx + off[w.s];
-	double *G = Gscr + w.aofs;
-	const int64_t plane = (int64_t)nt * nv;
-	const int K = tside ? ns * n : nt;  // reduction length
-	__shared__ double xs[KT][64 + 1];
-	__shared__ double zs[KT][64 + 1];
-	__shared__ int64_t cofs[kPcaMaxM];  // vertex side: the m column offsets; time side: KT of them
-	const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-	if (!tside)
-		for (int k = threadIdx.x; k < m; k += blockDim.x) cofs[k] = pca_col(sl, n, plane, nt, k);
-	for (int i0 = 0; i0 < m; i0 += 64) {
-		for (int j0 = 0; j0 < m; j0 += 64) {
-			double acc[4][4];
+// Loader of X for the tile products (DgLoader's slices): row i of the operand is time point i (time
+// side: K runs over the columns of X, rows contiguous) or column i of X (vertex side: K runs over
+// time, K contiguous).
+template <bool TSIDE>
+struct PcaLoader {
+	static constexpr bool KC = !TSIDE;
+	const double *D;
+	const int32_t *sl;
+	int64_t plane;
+	int n, nt, rows, i0, m, k;
+	const double *p[TSIDE ? 1 : 8];
+	uint32_t ok;
+	__device__ __forceinline__ void init(const double *D_, const int32_t *sl_, int n_, int64_t plane_, int nt_, int rows_,
+	                                     int i0_) {
+		D = D_; sl = sl_; n = n_; plane = plane_; nt = nt_; rows = rows_; i0 = i0_;
+		ok = 0;
+		if (TSIDE) {
+			m = threadIdx.x & 63;
+			k = threadIdx.x >> 6;
+			ok = i0 + m < rows ? 1u : 0u;
+			p[0] = D + i0 + m;
+		} else {
+			k = threadIdx.x & 15;
+			m = threadIdx.x >> 4;
 #pragma unroll
-			for (int a = 0; a < 4; a++)
-#pragma unroll
-				for (int b = 0; b < 4; b++) acc[a][b] = 0.0;
-			for (int k0 = 0; k0 < K; k0 += KT) {
-				__syncthreads();
-				if (tside) {
-					if (threadIdx.x < KT) {
-						const int k = k0 + threadIdx.x;
-						cofs[threadIdx.x] = k < K ? pca_col(sl, n, plane, nt, k) : -1;
-					}
-					__syncthreads();
-					// xs[kk][r] = X(i0 + r, k0 + kk): consecutive threads read consecutive times
-					for (int e = threadIdx.x; e < KT * 64; e += 256) {
-						const int kk = e >> 6, r = e & 63;
-						const int64_t c = cofs[kk];
-						const int ti = i0 + r, tj = j0 + r;
-						xs[kk][r] = (c >= 0 && ti < m) ? D[c + ti] : 0.0;
-						zs[kk][r] = (c >= 0 && tj < m) ? D[c + tj] : 0.0;
-					}
-				} else {
-					// xs[kk][r] = X(k0 + kk, i0 + r): consecutive threads read consecutive times
-					for (int e = threadIdx.x; e < KT * 64; e += 256) {
-						const int r = e / KT, kk = e - r * KT;
-						const int t = k0 + kk, pi = i0 + r, pj = j0 + r;
-						xs[kk][r] = (t < K && pi < m) ? D[cofs[pi] + t] : 0.0;
-						zs[kk][r] = (t < K && pj < m) ? D[cofs[pj] + t] : 0.0;
-					}
-				}
-				__syncthreads();
-#pragma unroll 4
-				for (int kk = 0; kk < KT; kk++) {
-					double a[4], b[4];
-#pragma unroll
-					for (int q = 0; q < 4; q++) {
-						a[q] = xs[kk][ty + 16 * q];
-						b[q] = zs[kk][tx + 16 * q];
-					}
-#pragma unroll
-					for (int p = 0; p < 4; p++)
-#pragma unroll
-						for (int q = 0; q < 4; q++) acc[p][q] += a[p] * b[q];
-				}
-			}
-#pragma unroll
-			for (int p = 0; p < 4; p++) {
-				const int i = i0 + ty + 16 * p;
-				if (i >= m) continue;
-#pragma unroll
-				for (int q = 0; q < 4; q++) {
-					const int j = j0 + tx + 16 * q;
-					if (j < m) G[(int64_t)j * m + i] = acc[p][q];
-				}
+			for (int j = 0; j < 8; j++) {
+				const int i = i0 + m + 8 * j;
+				const bool in = i < rows;
+				p[j] = D + (in ? pca_col(sl, n, plane, nt, i) : 0) + k;
+				ok |= (in ? 1u : 0u) << j;
 			}
 		}
 	}
+	__device__ __forceinline__ void load(double *s, int k0, int K, const double *safe) const {
+#pragma unroll
+		for (int j = 0; j < 8; j++) {
+			if (TSIDE) {
+				const int kk = k + 2 * j;
+				const bool in = ok && k0 + kk < K;
+				dg_cp8(s + kk * kDgLdM + m, in ? p[0] + pca_col(sl, n, plane, nt, k0 + kk) : safe, in);
+			} else {
+				const bool in = ((ok >> j) & 1u) && k0 + k < K;
+				dg_cp8(s + (m + 8 * j) * kDgLdK + k, in ? p[j] + k0 : safe, in);
+			}
+		}
+	}
+};
+
+// The Gram of every searchlight of a batch into the V scratch at wm.aofs (lower 64 x 64 tiles of
+// m x m, leading dimension m, wm.n = m): X X^T (m = nt, reduction over the ns n columns) or X^T X
+// (m = ns n < nt, reduction over time), one CTA per tile.
+__global__ void __launch_bounds__(kDgThreads) k_pca_gram(const SlWork *__restrict__ wm, const int32_t *__restrict__ sl_idx,
+                                                         const int32_t *__restrict__ off, const double *__restrict__ D,
+                                                         int ns, int nt, int nv, double *__restrict__ Gscr) {
+	extern __shared__ __align__(16) double dg_sm[];
+	const SlWork w = wm[blockIdx.y];
+	const int n = off[w.s + 1] - off[w.s], m = w.n;
+	const int T = (m + kDgTile - 1) / kDgTile;
+	if ((int)blockIdx.x >= T * (T + 1) / 2) return;
+	int ti, tj;
+	dg_lower(blockIdx.x, ti, tj);
+	const int i0 = ti * kDgTile, j0 = tj * kDgTile;
+	const int32_t *sl = sl_idx + off[w.s];
+	const int64_t plane = (int64_t)nt * nv;
+	double acc[2][4][4];
+	dg_zero(acc);
+	if (m == nt) {
+		PcaLoader<true> la, lb;
+		la.init(D, sl, n, plane, nt, m, i0);
+		lb.init(D, sl, n, plane, nt, m, j0);
+		dgemm_core(la, lb, ns * n, D, dg_sm, acc);
+	} else {
+		PcaLoader<false> la, lb;
+		la.init(D, sl, n, plane, nt, m, i0);
+		lb.init(D, sl, n, plane, nt, m, j0);
+		dgemm_core(la, lb, nt, D, dg_sm, acc);
+	}
+	double *G = Gscr + w.aofs;
+	dg_each(acc, [&](int i, int j, double v) {
+		if (i0 + i < m && j0 + j < m) G[(int64_t)(j0 + j) * m + i0 + i] = v;
+	});
 }
 
-// The template of every searchlight of a batch and B = tmpl^T M, the matrix whose polar factor
-// rotates it.  Eigenvectors (V scratch at wm.aofs, column-major, leading dimension m) and
-// eigenvalues (uv + wm.uvofs) from the eigenvector-mode Jacobi; the n largest eigenvalues (ties:
+// The template of every searchlight of a batch and the subjects' sum M.  Eigenvectors (V scratch at wm.aofs, column-major, leading dimension m) and
+// eigenvalues (uv + wm.uvofs) from the eigen decomposition; the n largest eigenvalues (ties:
 // the lower column) are taken in decreasing order.  wm and wn (the polar work items) are in slot
-// order; B (n x n) goes to the polar solve's A region at wn.aofs with the padding columns of its
-// block layout zero.
+// order.
 __global__ void __launch_bounds__(256) k_pca_tmpl(const SlWork *__restrict__ wm, const SlWork *__restrict__ wn,
                                                   const int32_t *__restrict__ sl_idx, const double *__restrict__ D,
                                                   int ns, int nt, int nv, const double *__restrict__ Vscr,
                                                   const double *__restrict__ uv, const int64_t *__restrict__ pofs,
-                                                  double *__restrict__ Pscr, double *__restrict__ Ascr) {
+                                                  double *__restrict__ Pscr) {
 	const SlWork em = wm[blockIdx.x];
 	const SlWork ep = wn[blockIdx.x];
 	const int n = ep.n, m = em.n;
@@ -200,47 +199,64 @@ __global__ void __launch_bounds__(256) k_pca_tmpl(const SlWork *__restrict__ wm,
 		g.C = tmpl; g.ci = 1; g.cj = nt;
 		block_gemm(g, ps, qs);
 	}
-	__syncthreads();
-	// B(r, c) = sum_t tmpl(t, r) M(t, c)
-	GemmArgs<double, double> g;
-	g.M = n; g.N = n; g.K = nt;
-	g.P = tmpl; g.pk = 1; g.pi = nt;
-	g.Q = M; g.qk = 1; g.qj = nt;
-	g.d = nullptr; g.alpha = 1.0;
-	g.E = nullptr; g.ei = 0; g.ej = 0; g.beta = 0.0;
-	double *A = Ascr + ep.aofs;
-	g.C = A; g.ci = 1; g.cj = n;
-	block_gemm(g, ps, qs);
-	const int ncol = ep.nblk * ep.bsz;
-	for (int64_t e = (int64_t)n * n + threadIdx.x; e < (int64_t)n * ncol; e += blockDim.x) A[e] = 0.0;
 }
 
-// C = tmpl R (nt x n, into the work area) from the polar factor R (float, column-major in the T
-// scratch at wn.tofs), R staged as float64 in the M block.  wn in slot order; m of the slot's
-// Gram from wm (slot order).
-__global__ void __launch_bounds__(256) k_pca_contrib(const SlWork *__restrict__ wm, const SlWork *__restrict__ wn,
-                                                     const float *__restrict__ Tscr, int nt,
-                                                     const int64_t *__restrict__ pofs, double *__restrict__ Pscr) {
+// B = tmpl^T M (n x n), the matrix whose polar factor rotates the template, into the polar solve's A
+// region at wn.aofs with the padding columns of its block layout zero.  One CTA per 64 x 64 tile.
+__global__ void __launch_bounds__(kDgThreads) k_pca_b(const SlWork *__restrict__ wm, const SlWork *__restrict__ wn, int nt,
+                                                      const int64_t *__restrict__ pofs, const double *__restrict__ Pscr,
+                                                      double *__restrict__ Ascr) {
+	extern __shared__ __align__(16) double dg_sm[];
+	const SlWork ep = wn[blockIdx.y];
+	const int n = ep.n, m = wm[blockIdx.y].n, T = (n + kDgTile - 1) / kDgTile;
+	if ((int)blockIdx.x >= T * T) return;
+	const PcaLayout L = PcaLayout::make(nt, n, m, m != nt);
+	const double *base = Pscr + pofs[ep.slot];
+	const int i0 = ((int)blockIdx.x % T) * kDgTile, j0 = ((int)blockIdx.x / T) * kDgTile;
+	double acc[2][4][4];
+	dg_zero(acc);
+	dgemm_tile<true, true>(DgOperand{base + L.tmpl, nullptr, nt, n}, i0, DgOperand{base + L.M, nullptr, nt, n}, j0, nt, dg_sm, acc);
+	double *A = Ascr + ep.aofs;
+	dg_each(acc, [&](int i, int j, double v) {
+		if (i0 + i < n && j0 + j < n) A[(int64_t)(j0 + j) * n + i0 + i] = v;
+	});
+	if (blockIdx.x == 0)
+		for (int64_t e = (int64_t)n * n + threadIdx.x; e < (int64_t)n * ep.nblk * ep.bsz; e += blockDim.x) A[e] = 0.0;
+}
+
+// The polar factors R (float, column-major in the T scratch at wn.tofs) as float64 in the M block
+// (M is no longer needed).
+__global__ void __launch_bounds__(256) k_pca_widen(const SlWork *__restrict__ wm, const SlWork *__restrict__ wn,
+                                                   const float *__restrict__ Tscr, int nt,
+                                                   const int64_t *__restrict__ pofs, double *__restrict__ Pscr) {
 	const SlWork ep = wn[blockIdx.x];
 	const int n = ep.n, m = wm[blockIdx.x].n;
+	double *Rd = Pscr + pofs[ep.slot] + PcaLayout::make(nt, n, m, m != nt).M;
+	const float *R = Tscr + ep.tofs;
+	for (int64_t e = threadIdx.x; e < (int64_t)n * n; e += blockDim.x) Rd[e] = (double)R[e];
+}
+
+// C = tmpl R (nt x n, into the work area), one CTA per 64 x 64 tile.  wn in slot order; m of the slot's
+// Gram from wm (slot order).
+__global__ void __launch_bounds__(kDgThreads) k_pca_contrib(const SlWork *__restrict__ wm, const SlWork *__restrict__ wn,
+                                                            int nt, const int64_t *__restrict__ pofs,
+                                                            double *__restrict__ Pscr) {
+	extern __shared__ __align__(16) double dg_sm[];
+	const SlWork ep = wn[blockIdx.y];
+	const int n = ep.n, m = wm[blockIdx.y].n;
+	const int Tt = (nt + kDgTile - 1) / kDgTile, T = (n + kDgTile - 1) / kDgTile;
+	if ((int)blockIdx.x >= Tt * T) return;
 	const PcaLayout L = PcaLayout::make(nt, n, m, m != nt);
 	double *base = Pscr + pofs[ep.slot];
-	const double *tmpl = base + L.tmpl;
-	double *Rd = base + L.M;  // M is no longer needed
-	double *C = base + L.work;
-	const float *R = Tscr + ep.tofs;
-	__shared__ double ps[16][65], qs[16][65];
-	for (int64_t e = threadIdx.x; e < (int64_t)n * n; e += blockDim.x) Rd[e] = (double)R[e];
-	__syncthreads();
+	const int i0 = ((int)blockIdx.x % Tt) * kDgTile, j0 = ((int)blockIdx.x / Tt) * kDgTile;
+	double acc[2][4][4];
+	dg_zero(acc);
 	// C(t, j) = sum_i tmpl(t, i) R(i, j)
-	GemmArgs<double, double> g;
-	g.M = nt; g.N = n; g.K = n;
-	g.P = tmpl; g.pk = nt; g.pi = 1;
-	g.Q = Rd; g.qk = 1; g.qj = n;
-	g.d = nullptr; g.alpha = 1.0;
-	g.E = nullptr; g.ei = 0; g.ej = 0; g.beta = 0.0;
-	g.C = C; g.ci = 1; g.cj = nt;
-	block_gemm(g, ps, qs);
+	dgemm_tile<false, true>(DgOperand{base + L.tmpl, nullptr, nt, nt}, i0, DgOperand{base + L.M, nullptr, n, n}, j0, n, dg_sm, acc);
+	double *C = base + L.work;
+	dg_each(acc, [&](int i, int j, double v) {
+		if (i0 + i < nt && j0 + j < n) C[(int64_t)(j0 + j) * nt + i0 + i] = v;
+	});
 }
 
 // template[:, v] += sum over the searchlights s of [s_lo, s_hi) holding v (member a), in

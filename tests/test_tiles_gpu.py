@@ -58,3 +58,22 @@ def test_ridge_without_penalty_on_singular_data_writes_zeros(gpu):
     assert plan.stats()["n_unconverged"] == 1
     assert not vals.any()
     plan.close()
+
+
+# R is rounded to float32 (6e-8 relative per element); everything else is float64.
+@pytest.mark.parametrize("nt,ns,sizes", [
+    (64, 3, [1, 2, 31, 63, 64]),          # Gram order nt: a whole tile; also ns n < nt (vertex side)
+    (65, 2, [1, 16, 32, 33, 64, 65]),     # one row more than a tile
+    (130, 3, [5, 43, 44, 64, 65, 128]),
+    (400, 1, [63, 129, 257]),             # vertex side only
+])
+def test_pca_template_tile_edges(gpu, nt, ns, sizes):
+    from hyperalignment_b200 import hyperalignment_c as H
+    rng = np.random.default_rng(nt)
+    X, _, idx, off = one_each(sizes, nt, nt)
+    dms = [X @ np.linalg.qr(rng.standard_normal((X.shape[1],) * 2))[0] + 0.1 * rng.standard_normal(X.shape)
+           for _ in range(ns)]
+    sls = [idx[off[s]:off[s + 1]] for s in range(len(sizes))]
+    got = H.searchlight_pca_template(dms, sls, None, 1.0)
+    ref = O.searchlight_pca_template(dms, idx, off, None, 1.0)
+    assert np.linalg.norm(got - ref) / np.linalg.norm(ref) <= 1e-6
