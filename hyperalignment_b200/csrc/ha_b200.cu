@@ -12,6 +12,7 @@
 #include "ha_b200_eig.cuh"
 #include "ha_b200_polar.cuh"
 #include "ha_b200_grid.cuh"
+#include "ha_b200_dgrid.cuh"
 #include "ha_b200_mlp.cuh"
 #include "ha_b200_tc.cuh"
 #include "ha_b200_pca.cuh"
@@ -300,15 +301,15 @@ int launch_eig(const EigWork *d_work, const std::vector<int> &orders, double *A,
 
 struct Chunk {
 	int s0, s1;
-	std::vector<SlWork> w32, w64, weig;  // float32 polar, float64 polar, float64 eigenvector mode
-	std::vector<Bucket> b32, b64, beig;
+	std::vector<SlWork> w32, w64;  // float32 polar, float64 polar
+	std::vector<Bucket> b32, b64;
 	std::vector<SlWork> weig32;  // float32 eigenvector mode (the plain FP32 grid search)
 	std::vector<Bucket> beig32;
 	std::vector<int64_t> tofs;  // per slot
 	int64_t scratch_elems8;     // scratch size in 8-byte units (A and V each)
 	int64_t t_elems;            // T scratch floats
 	int64_t uv_elems;
-	SlWork *d_w32 = nullptr, *d_w64 = nullptr, *d_weig = nullptr, *d_weig32 = nullptr;
+	SlWork *d_w32 = nullptr, *d_w64 = nullptr, *d_weig32 = nullptr;
 	int64_t *d_tofs = nullptr;
 	// tensor-core solve: one work item per searchlight (slot order), 128-row tiles in two size
 	// classes (np <= 256: two CTAs per SM; np > 256), largest searchlights first
@@ -383,6 +384,15 @@ struct HaB200Plan {
 	DevArr<int64_t> gbase;
 	DevArr<int32_t> gnpcs, grows, gtpos, gurows, guntested;
 	DevArr<GridModel> gmdl;
+	// float64 grid search: work lists and the CV description of its kernels; scratch of the eigen solves
+	std::vector<DgModel> dg_models;
+	DevArr<DgItem> dgitem;
+	DevArr<DgSl> dgsl;
+	DevArr<EigWork> dgeig;
+	DevArr<int32_t> dgslot;
+	DevArr<DgModel> dgmdl;
+	DevArr<int32_t> dgint;
+	DevArr<double> dgdbl, eigscr;
 	DevArr<int32_t> gfit;      // fit rows of the learned form / the features
 	DevArr<float> gfeat;       // features of the learned form
 	DevArr<SlWork> gwork;      // fallback work list of the learned form
@@ -466,7 +476,7 @@ size_t scratch_budget_bytes() {
 
 // Sort work items by Jacobi class (resident or blocked, rows per lane), largest first inside a
 // class, and cut them into buckets of one Jacobi kernel instance each.  prec: 0 float32 polar,
-// 1 float64 polar, 2 float64 eigenvector mode, 3 float32 eigenvector mode.
+// 1 float64 polar, 2 float32 eigenvector mode.
 std::vector<Bucket> bucketize(std::vector<SlWork> &items, int prec) {
 	auto key = [](const SlWork &w) { return (w.nblk == 2 ? 0 : 32) + rpl_for(w.n); };
 	std::stable_sort(items.begin(), items.end(), [&](const SlWork &a, const SlWork &b) {
@@ -481,7 +491,7 @@ std::vector<Bucket> bucketize(std::vector<SlWork> &items, int prec) {
 		while (j < (int)items.size() && key(items[j]) == key(items[i])) {
 			int bb, kk;
 			size_t mm;
-			const bool f64 = prec == 1 || prec == 2;
+			const bool f64 = prec == 1;
 			jacobi_layout(items[j].n, f64, bb, kk, mm, f64 ? kSmemMax : fp32_jacobi_budget(), prec < 2);
 			smem = std::max(smem, mm);
 			j++;
@@ -491,7 +501,7 @@ std::vector<Bucket> bucketize(std::vector<SlWork> &items, int prec) {
 		b.count = j - i;
 		b.smem = smem;
 		b.blocked = items[i].nblk != 2;
-		b.threads = jacobi_threads(items[i].bsz, prec == 1 || prec == 2);
+		b.threads = jacobi_threads(items[i].bsz, prec == 1);
 		b.rpl = rpl_for(items[i].n);
 		buckets.push_back(b);
 		i = j;
@@ -509,7 +519,7 @@ int build_chunks(HaB200Plan *P) {
 		int64_t acc8 = 0, tacc = 0, uvacc = 0;
 		std::vector<int64_t> tofs;
 		std::vector<int64_t> aofs8;
-		std::vector<int> bs32, nb32, bs64, nb64, bse, nbe, bse32, nbe32;
+		std::vector<int> bs32, nb32, bs64, nb64, bse32, nbe32;
 		std::vector<size_t> sm32, sm64;
 		while (s < P->count) {
 			int n = P->h_off[s + 1] - P->h_off[s];
@@ -517,16 +527,13 @@ int build_chunks(HaB200Plan *P) {
 			size_t m32, m64;
 			jacobi_layout(n, false, b32, k32, m32, fp32_jacobi_budget());
 			jacobi_layout(n, true, b64, k64, m64);
-			int be, ke;
 			size_t me;
-			jacobi_layout(n, true, be, ke, me, kSmemMax, false);
 			int be32, ke32;
 			jacobi_layout(n, false, be32, ke32, me, fp32_jacobi_budget(), false);
 			int64_t e32 = ((int64_t)n * k32 * b32 * 4 + 7) / 8;
 			int64_t e64 = (int64_t)n * k64 * b64;
-			int64_t eeig = (int64_t)n * ke * be;
 			int64_t eeig32 = ((int64_t)n * ke32 * be32 * 4 + 7) / 8;
-			int64_t region = std::max<int64_t>(std::max(std::max(e32, e64), std::max(eeig, eeig32)), (int64_t)n * n);
+			int64_t region = std::max<int64_t>(std::max(std::max(e32, e64), eeig32), (int64_t)n * n);
 			region = (region + 31) & ~(int64_t)31;
 			size_t bytes_if = (size_t)(acc8 + region) * 8 * 2 + (size_t)(tacc + (int64_t)n * n) * 4;
 			if (!tofs.empty() && bytes_if > budget) break;
@@ -536,7 +543,6 @@ int build_chunks(HaB200Plan *P) {
 			tacc += (int64_t)n * n;
 			bs32.push_back(b32); nb32.push_back(k32); sm32.push_back(m32);
 			bs64.push_back(b64); nb64.push_back(k64); sm64.push_back(m64);
-			bse.push_back(be); nbe.push_back(ke);
 			bse32.push_back(be32); nbe32.push_back(ke32);
 			uvacc += 2 * (int64_t)n;
 			s++;
@@ -548,7 +554,7 @@ int build_chunks(HaB200Plan *P) {
 		ch.tofs = tofs;
 		const int nsl = ch.s1 - ch.s0;
 		// work items, bucketed by (mode, n range), largest first inside a bucket
-		for (int prec = 0; prec < 4; prec++) {  // float32, float64, float64 / float32 eigenvector mode
+		for (int prec = 0; prec < 3; prec++) {  // float32, float64, float32 eigenvector mode
 			std::vector<SlWork> items;
 			int64_t uvo = 0;
 			for (int q = 0; q < nsl; q++) {
@@ -557,9 +563,9 @@ int build_chunks(HaB200Plan *P) {
 				SlWork w;
 				w.s = sidx;
 				w.n = n;
-				w.bsz = prec == 3 ? bse32[q] : prec == 2 ? bse[q] : (prec ? bs64[q] : bs32[q]);
-				w.nblk = prec == 3 ? nbe32[q] : prec == 2 ? nbe[q] : (prec ? nb64[q] : nb32[q]);
-				w.aofs = (prec == 1 || prec == 2) ? aofs8[q] : aofs8[q] * 2;
+				w.bsz = prec == 2 ? bse32[q] : (prec ? bs64[q] : bs32[q]);
+				w.nblk = prec == 2 ? nbe32[q] : (prec ? nb64[q] : nb32[q]);
+				w.aofs = prec == 1 ? aofs8[q] : aofs8[q] * 2;
 				w.tofs = tofs[q];
 				w.sofs = P->h_off[sidx];
 				w.slot = q;
@@ -570,18 +576,15 @@ int build_chunks(HaB200Plan *P) {
 			std::vector<Bucket> buckets = bucketize(items, prec);
 			if (prec == 0) { ch.w32 = items; ch.b32 = buckets; }
 			else if (prec == 1) { ch.w64 = items; ch.b64 = buckets; }
-			else if (prec == 2) { ch.weig = items; ch.beig = buckets; }
 			else { ch.weig32 = items; ch.beig32 = buckets; }
 		}
 		P->chunks.push_back(std::move(ch));
 	}
 	// device copies of the work lists
 	for (auto &ch : P->chunks) {
-		size_t n32 = ch.w32.size(), n64 = ch.w64.size(), ne = ch.weig.size();
+		size_t n32 = ch.w32.size(), n64 = ch.w64.size();
 		if (cudaMalloc(&ch.d_w32, n32 * sizeof(SlWork)) != cudaSuccess) return kHaErrorAlloc;
 		if (cudaMalloc(&ch.d_w64, n64 * sizeof(SlWork)) != cudaSuccess) return kHaErrorAlloc;
-		if (cudaMalloc(&ch.d_weig, ne * sizeof(SlWork)) != cudaSuccess) return kHaErrorAlloc;
-		HA_CUDA(cudaMemcpy(ch.d_weig, ch.weig.data(), ne * sizeof(SlWork), cudaMemcpyHostToDevice));
 		if (cudaMalloc(&ch.d_weig32, ch.weig32.size() * sizeof(SlWork)) != cudaSuccess) return kHaErrorAlloc;
 		HA_CUDA(cudaMemcpy(ch.d_weig32, ch.weig32.data(), ch.weig32.size() * sizeof(SlWork), cudaMemcpyHostToDevice));
 		if (cudaMalloc(&ch.d_tofs, ch.tofs.size() * sizeof(int64_t)) != cudaSuccess) return kHaErrorAlloc;
@@ -640,9 +643,13 @@ int set_smem_attrs() {
 	HA_CUDA(cudaFuncSetAttribute(k_pca_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
 	HA_CUDA(cudaFuncSetAttribute(k_pca_b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
 	HA_CUDA(cudaFuncSetAttribute(k_pca_contrib, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
+	HA_CUDA(cudaFuncSetAttribute(k_dg_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
+	HA_CUDA(cudaFuncSetAttribute(k_dg_q, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
+	HA_CUDA(cudaFuncSetAttribute(k_dg_project, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
+	HA_CUDA(cudaFuncSetAttribute(k_dg_eval, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
+	HA_CUDA(cudaFuncSetAttribute(k_dg_beta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
 	HA_CUDA(cudaFuncSetAttribute(k_ridge_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
 	HA_CUDA(cudaFuncSetAttribute(k_ridge_chol, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRidgeSmem));
-	HA_CUDA(cudaFuncSetAttribute(k_pchol<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kPcholNb * kGridMaxN * 8)));
 	HA_CUDA(cudaFuncSetAttribute(k_pchol<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kPcholNb * kGridMaxN * 4)));
 	done = true;
 	return kHaSuccess;
@@ -1743,7 +1750,7 @@ int grid_prepare(HaB200Plan *P) {
 	return P->scrT64.ensure((size_t)maxT);
 }
 
-size_t pchol_smem(int rpl, size_t esz = sizeof(double)) { return (size_t)kPcholNb * 32 * rpl * esz; }
+size_t pchol_smem(int rpl) { return (size_t)kPcholNb * 32 * rpl * sizeof(float); }
 
 JacobiParams eig_params(bool only_flagged) {
 	JacobiParams jp;
@@ -1783,16 +1790,14 @@ int reduce_chunk64(HaB200Plan *P, Chunk &ch, int out_kind, double *d_vals, cudaS
 // as many as fit the grid scratch budget, and each one's per-slot scratch base offsets.
 struct GridBatch {
 	int i0, i1;
-	int64_t total;  // elements of grid scratch (float64 or float32, by the search's arithmetic)
+	int64_t total;  // float32 elements of grid scratch
 };
 
-void grid_plan_chunk(const Chunk &ch, const GridParams &gp, bool fp32, std::vector<GridBatch> &bt,
-                     std::vector<int64_t> &gbase_all) {
+void grid_plan_chunk(const Chunk &ch, const GridParams &gp, std::vector<GridBatch> &bt, std::vector<int64_t> &gbase_all) {
 	const int nsl = ch.s1 - ch.s0;
 	const int grid = gp.n_alphas * gp.n_npcs;
 	const size_t budget = grid_budget_bytes();
-	const std::vector<SlWork> &items = fp32 ? ch.weig32 : ch.weig;
-	const size_t esz = fp32 ? 4 : 8;
+	const std::vector<SlWork> &items = ch.weig32;
 	const int nitems = (int)items.size();
 	bt.clear();
 	int i0 = 0;
@@ -1804,7 +1809,7 @@ void grid_plan_chunk(const Chunk &ch, const GridParams &gp, bool fp32, std::vect
 		while (i1 < nitems) {
 			const SlWork &wi = items[i1];
 			const GridLayout Lg = GridLayout::make(wi.n, gp.models, gp.mte, gp.ntu, gp.n_alphas, grid);
-			if (i1 > i0 && (size_t)(total + Lg.total) * esz > budget) break;
+			if (i1 > i0 && (size_t)(total + Lg.total) * sizeof(float) > budget) break;
 			gbase_all[g0 + wi.slot] = total;
 			total += Lg.total;
 			i1++;
@@ -1814,21 +1819,18 @@ void grid_plan_chunk(const Chunk &ch, const GridParams &gp, bool fp32, std::vect
 	}
 }
 
-// The launches of one chunk's grid search (no host copies or allocations: capturable); the
-// sub-batches' base offsets are at d_gbase (nsl per sub-batch).  Real is the arithmetic type:
-// double for the float64 grid search, float for the plain FP32 one (the float32 eigenvector-mode
-// work list, the A / V / grid scratch read as float; the winners' betas still go to the float64
-// T scratch for the reduction).
-template <typename Real>
-int grid_chunk_launch_t(HaB200Plan *P, Chunk &ch, const double *d_X, const double *d_Y, const GridSpec &gs,
-                        GridParams gp, const std::vector<GridBatch> &bt, const int64_t *d_gbase, int rowmajor,
-                        int32_t *d_best, double *d_cost, cudaStream_t st) {
-	constexpr bool f32 = sizeof(Real) == 4;
+// The launches of one chunk's plain FP32 grid search (no host copies or allocations: capturable);
+// the sub-batches' base offsets are at d_gbase (nsl per sub-batch).  The A / V / grid scratch are
+// read as float; the winners' betas still go to the float64 T scratch for the reduction.
+int grid_chunk_launch(HaB200Plan *P, Chunk &ch, const double *d_X, const double *d_Y, const GridSpec &gs,
+                      GridParams gp, const std::vector<GridBatch> &bt, const int64_t *d_gbase, int rowmajor,
+                      int32_t *d_best, double *d_cost, cudaStream_t st) {
+	using Real = float;
 	const int nt = P->nt;
 	const int nsl = ch.s1 - ch.s0;
 	const JacobiParams jp = eig_params(false);
-	const std::vector<Bucket> &beig = f32 ? ch.beig32 : ch.beig;
-	SlWork *d_work = f32 ? ch.d_weig32 : ch.d_weig;
+	const std::vector<Bucket> &beig = ch.beig32;
+	SlWork *d_work = ch.d_weig32;
 	Real *A = reinterpret_cast<Real *>(P->scrA.p), *V = reinterpret_cast<Real *>(P->scrV.p);
 	Real *G = reinterpret_cast<Real *>(P->gridscr.p);
 	int rc;
@@ -1846,11 +1848,11 @@ int grid_chunk_launch_t(HaB200Plan *P, Chunk &ch, const double *d_X, const doubl
 				const cudaStream_t bs = g_fan.at((int)bi);
 				const SlWork *wk = d_work + x0;
 				// Gram into the V scratch, its pivoted Cholesky factor into the A scratch
-				{ HA_LAUNCH(f32 ? kHaB200KXcov32 : kHaB200KXcov64, bs); k_xcov_rows<16, Real><<<x1 - x0, kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_X, nt, tr, md.tr_n, V, G, gp, 0); }
-				{ HA_LAUNCH(f32 ? kHaB200KXcov32 : kHaB200KXcov64, bs); k_xcov_rows<16, Real><<<x1 - x0, kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_Y, nt, tr, md.tr_n, A, G, gp, 1); }
-				{ HA_LAUNCH(kHaB200KRidge, bs); k_pchol<Real><<<x1 - x0, kBlock, pchol_smem(b.rpl, sizeof(Real)), bs>>>(wk, V, A, P->stats.p); }
+				{ HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<16, Real><<<x1 - x0, kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_X, nt, tr, md.tr_n, V, G, gp, 0); }
+				{ HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<16, Real><<<x1 - x0, kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_Y, nt, tr, md.tr_n, A, G, gp, 1); }
+				{ HA_LAUNCH(kHaB200KRidge, bs); k_pchol<Real><<<x1 - x0, kBlock, pchol_smem(b.rpl), bs>>>(wk, V, A, P->stats.p); }
 				{
-					HA_LAUNCH(f32 ? kHaB200KJacobi32 : kHaB200KJacobi64, bs);
+					HA_LAUNCH(kHaB200KJacobi32, bs);
 					if ((rc = launch_jacobi<Real>(b.rpl, x1 - x0, b.threads, b.smem, bs, wk, A, V, P->scrT.p, P->stats.p, P->uv.p, jp)) != kHaSuccess)
 						return rc;
 				}
@@ -1865,19 +1867,314 @@ int grid_chunk_launch_t(HaB200Plan *P, Chunk &ch, const double *d_X, const doubl
 	return kHaSuccess;
 }
 
-int grid_chunk_launch(HaB200Plan *P, Chunk &ch, const double *d_X, const double *d_Y, const GridSpec &gs,
-                      GridParams gp, bool fp32, const std::vector<GridBatch> &bt, const int64_t *d_gbase,
-                      int rowmajor, int32_t *d_best, double *d_cost, cudaStream_t st) {
-	return fp32 ? grid_chunk_launch_t<float>(P, ch, d_X, d_Y, gs, gp, bt, d_gbase, rowmajor, d_best, d_cost, st)
-	            : grid_chunk_launch_t<double>(P, ch, d_X, d_Y, gs, gp, bt, d_gbase, rowmajor, d_best, d_cost, st);
+// ---- float64 grid search (ha_b200_dgrid.cuh) ----
+
+// Flag the searchlights as solved in float64 (and unconverged where an eigen solve was).
+__global__ void k_dg_flags(const EigWork *__restrict__ eig, const int32_t *__restrict__ slot, int n, const double *__restrict__ S,
+                           SlStats *__restrict__ stats) {
+	const int q = blockIdx.x * blockDim.x + threadIdx.x;
+	if (q >= n) return;
+	const EigState st = *reinterpret_cast<const EigState *>(S + eig[q].s + EigScratch::make(eig[q].p).state);
+	atomicOr(&stats[slot[q]].flags, kFlagFP64 | (st.bad ? kFlagUnconverged : 0));
 }
 
-// One chunk's grid search enqueued directly (sub-batch plan, scratch and offsets, launches).
-int grid_chunk(HaB200Plan *P, Chunk &ch, const double *d_X, const double *d_Y, const GridSpec &gs,
-               const GridParams &gp, bool fp32, int rowmajor, int32_t *d_best, double *d_cost, cudaStream_t st) {
+// Upload the CV description of the float64 search: distinct training rows with their multiplicities,
+// test rows with those of one model first, and the rows that several models test.
+// The fit rows of the learned form (n_rows > 0) are one model more, without test rows: its parameters
+// go to *fit.
+int dgrid_upload(HaB200Plan *P, const GridSpec &gs, cudaStream_t st, DgParams &dp, const int32_t *rows = nullptr,
+                 int n_rows = 0, DgParams *fit = nullptr) {
+	const int models = (int)gs.mdl.size();
+	std::vector<DgModel> mdl(models + (fit ? 1 : 0));
+	std::vector<int32_t> drow, terow, ovrow, ovptr, ovent;
+	std::vector<double> dsq, tew;
+	std::vector<std::vector<int32_t>> by_row(gs.ntu);  // entries of every tested row
+	std::vector<int32_t> count((size_t)P->nt);
+	int entries = 0;
+	auto distinct = [&](DgModel &d, const int32_t *tr, int n) {
+		d = {};
+		d.tr_n = n;
+		d.d_ofs = (int32_t)drow.size();
+		std::fill(count.begin(), count.end(), 0);
+		for (int i = 0; i < n; i++) count[tr[i]]++;
+		for (int t = 0; t < P->nt; t++)
+			if (count[t]) {
+				drow.push_back(t);
+				dsq.push_back(std::sqrt((double)count[t]));
+			}
+		d.d_n = (int32_t)drow.size() - d.d_ofs;
+	};
+	if (fit) distinct(mdl[models], rows, n_rows);
+	for (int m = 0; m < models; m++) {
+		const GridModel &g = gs.mdl[m];
+		DgModel &d = mdl[m];
+		distinct(d, gs.rows.data() + g.tr_ofs, g.tr_n);
+		d.te_ofs = (int32_t)terow.size();
+		d.te_n = g.te_n;
+		d.entry0 = entries;
+		for (int several = 0; several < 2; several++) {
+			for (int i = 0; i < g.te_n; i++) {
+				const int u = gs.tpos[g.te_ofs + i];
+				if ((gs.winv[u] < 1.0) != (several == 1)) continue;
+				terow.push_back(gs.rows[g.te_ofs + i]);
+				tew.push_back(gs.winv[u]);
+				if (several) by_row[u].push_back(entries++);
+			}
+			if (!several) d.te1 = (int32_t)terow.size() - d.te_ofs;
+		}
+	}
+	ovptr.push_back(0);
+	for (int u = 0; u < gs.ntu; u++)
+		if (!by_row[u].empty()) {
+			ovrow.push_back(gs.urows[u]);
+			ovent.insert(ovent.end(), by_row[u].begin(), by_row[u].end());
+			ovptr.push_back((int32_t)ovent.size());
+		}
+	std::vector<int32_t> ints;
+	size_t at[7];
+	int k = 0;
+	const std::vector<int32_t> *lists[7] = {&drow, &terow, &ovrow, &ovptr, &ovent, &gs.untested, &gs.npcs};
+	for (const std::vector<int32_t> *v : lists) {
+		at[k++] = ints.size();
+		ints.insert(ints.end(), v->begin(), v->end());
+	}
+	std::vector<double> dbl(dsq);
+	dbl.insert(dbl.end(), tew.begin(), tew.end());
+	dbl.insert(dbl.end(), gs.alphas.begin(), gs.alphas.end());
+	int rc;
+	if ((rc = upload_vec(P->dgmdl, mdl, st)) != kHaSuccess || (rc = upload_vec(P->dgint, ints, st)) != kHaSuccess ||
+	    (rc = upload_vec(P->dgdbl, dbl, st)) != kHaSuccess)
+		return rc;
+	dp = {};
+	dp.mdl = P->dgmdl.p;
+	dp.drow = P->dgint.p + at[0];
+	dp.terow = P->dgint.p + at[1];
+	dp.ovrow = P->dgint.p + at[2];
+	dp.ovptr = P->dgint.p + at[3];
+	dp.ovent = P->dgint.p + at[4];
+	dp.untested = P->dgint.p + at[5];
+	dp.npcs = P->dgint.p + at[6];
+	dp.dsq = P->dgdbl.p;
+	dp.tew = P->dgdbl.p + dsq.size();
+	dp.alphas = P->dgdbl.p + dsq.size() + tew.size();
+	dp.models = models;
+	dp.nt = P->nt;
+	dp.n_alphas = (int)gs.alphas.size();
+	dp.n_npcs = (int)gs.npcs.size();
+	dp.nov = (int)ovrow.size();
+	dp.entries = entries;
+	dp.n_untested = (int)gs.untested.size();
+	if (fit) {
+		*fit = dp;
+		fit->mdl = dp.mdl + models;
+		fit->model0 = models;
+		fit->models = 1;
+		fit->nov = fit->entries = fit->n_untested = 0;
+	}
+	P->dg_models = std::move(mdl);
+	return kHaSuccess;
+}
+
+// Sub-batches of searchlights (the widest first) of a float64 search, within the grid scratch budget:
+// work lists with their scratch offsets, uploaded.
+struct DgBatch {
+	size_t sl0, sl1;
+};
+struct DgPlan {
+	std::vector<DgSl> sls;
+	std::vector<int> orders;  // eigen solves' orders, sorted inside a batch
+	std::vector<DgBatch> batches;
+	int na = 1;    // penalties evaluated together
+	int tt = 0;    // 64-row tiles of the longest test list
+	int rows = 0;  // groups of several-model rows
+};
+
+int dg_tiles_of(int n) { return (n + kDgTile - 1) / kDgTile; }
+
+int dgrid_plan(HaB200Plan *P, std::vector<SlWork> work, const DgParams &dp, DgPlan &pl, cudaStream_t st) {
+	std::stable_sort(work.begin(), work.end(), [](const SlWork &a, const SlWork &b) { return a.n > b.n; });
+	const std::vector<DgModel> &mdl = P->dg_models;
+	const int grid = dp.n_alphas * dp.n_npcs;
+	int max_te = 0;
+	for (int m = 0; m < dp.models; m++) max_te = std::max(max_te, mdl[dp.model0 + m].te_n);
+	pl.tt = dg_tiles_of(max_te);
+	pl.rows = (dp.nov + kDgRows - 1) / kDgRows;
+	// two penalties' predictions need about the scratch that the eigen solves had
+	pl.na = std::max(1, std::min({2, dp.n_alphas, 65535 / std::max(1, dp.n_npcs)}));
+	std::vector<DgItem> items;
+	std::vector<EigWork> eig;
+	std::vector<int32_t> slot;
+	const size_t budget = grid_budget_bytes();
+	int64_t o = 0, mx = 1;
+	auto take = [&](int64_t n) {  // 32-byte aligned pieces
+		const int64_t at = o;
+		o = (o + n + 3) & ~(int64_t)3;
+		return at;
+	};
+	for (size_t i = 0; i < work.size();) {
+		const size_t sl0 = pl.sls.size(), first_item = items.size();
+		o = 0;
+		for (; i < work.size(); i++) {
+			const SlWork &w = work[i];
+			const int64_t o0 = o;
+			const size_t items0 = items.size();
+			DgSl sl = {};
+			sl.s = w.s;
+			sl.n = w.n;
+			sl.item0 = (int32_t)(items0 - first_item);
+			sl.sofs = w.sofs;
+			sl.tofs = w.tofs;
+			const int64_t n = w.n;
+			int parts = 0;
+			int64_t eigtot = 0;
+			for (int m = 0; m < dp.models; m++) {
+				const DgModel &md = mdl[dp.model0 + m];
+				DgItem it = {};
+				it.n = w.n;
+				it.dual = md.d_n < w.n ? 1 : 0;
+				it.p = it.dual ? md.d_n : w.n;
+				it.model = m;
+				it.sofs = w.sofs;
+				it.sl = (int32_t)(pl.sls.size() - sl0);
+				it.part0 = parts;
+				parts += dg_tiles_of(md.te_n) * dg_tiles_of(w.n) * 4;
+				it.xd = take(md.d_n * n);
+				it.yd = take(md.d_n * n);
+				it.xte = take(md.te_n * n);
+				it.yte = take(md.te_n * n);
+				it.g = take((int64_t)it.p * it.p);
+				it.c = take((int64_t)(it.dual ? md.te_n : md.d_n) * it.p);
+				it.q = take(it.p * n);
+				it.e = take((int64_t)md.te_n * it.p);
+				it.nv = it.dual ? take(n * it.p) : it.g;
+				it.lam = take(it.p);
+				items.push_back(it);
+				eigtot += EigScratch::make(it.p).total;
+			}
+			sl.nparts = parts + pl.rows;
+			sl.yov = take((int64_t)dp.nov * n);
+			sl.part = take((int64_t)grid * sl.nparts);
+			sl.cost = take(grid);
+			// the eigen solves' scratch is free when the predictions of `na` penalties are written
+			sl.pov = take(std::max(eigtot, (int64_t)pl.na * dp.n_npcs * dp.entries * n));
+			if (pl.sls.size() > sl0 && ((size_t)o * 8 > budget || items.size() - first_item > 65535)) {
+				items.resize(items0);
+				o = o0;
+				break;
+			}
+			int64_t es = sl.pov;
+			for (size_t q = items0; q < items.size(); q++) {
+				eig.push_back({items[q].g, items[q].q, es, items[q].lam, items[q].p, 0});
+				slot.push_back(w.slot);
+				es += EigScratch::make(items[q].p).total;
+			}
+			pl.sls.push_back(sl);
+		}
+		pl.batches.push_back({sl0, pl.sls.size()});
+		mx = std::max(mx, o);
+	}
+	// every batch's eigen solves by order, with their searchlights' slots
+	pl.orders.resize(eig.size());
+	std::vector<EigWork> es(eig.size());
+	std::vector<int32_t> ss(eig.size());
+	for (const DgBatch &b : pl.batches) {
+		const size_t e0 = b.sl0 * dp.models, e1 = b.sl1 * dp.models;
+		std::vector<size_t> idx(e1 - e0);
+		for (size_t q = 0; q < idx.size(); q++) idx[q] = e0 + q;
+		std::stable_sort(idx.begin(), idx.end(), [&](size_t x, size_t y) { return eig[x].p > eig[y].p; });
+		for (size_t q = 0; q < idx.size(); q++) {
+			es[e0 + q] = eig[idx[q]];
+			ss[e0 + q] = slot[idx[q]];
+			pl.orders[e0 + q] = es[e0 + q].p;
+		}
+	}
+	int rc;
+	if ((rc = upload_vec(P->dgeig, es, st)) != kHaSuccess || (rc = upload_vec(P->dgslot, ss, st)) != kHaSuccess ||
+	    (rc = upload_vec(P->dgitem, items, st)) != kHaSuccess || (rc = upload_vec(P->dgsl, pl.sls, st)) != kHaSuccess)
+		return rc;
+	return P->gridscr.ensure((size_t)mx);
+}
+
+// The searchlights [i, i + cnt) of one tile count tn of a batch form a launch class, on a side
+// stream of its own.
+template <typename F>
+int dgrid_classes(const DgPlan &pl, const DgBatch &b, cudaStream_t st, F launch) {
+	int rc = g_fan.begin(st);
+	if (rc != kHaSuccess) return rc;
+	const int ns = (int)(b.sl1 - b.sl0);
+	int c = 0;
+	for (int i = 0; i < ns; c++) {
+		const int tn = dg_tiles_of(pl.sls[b.sl0 + i].n);
+		int j = i;
+		while (j < ns && dg_tiles_of(pl.sls[b.sl0 + j].n) == tn) j++;
+		launch(i, j - i, tn, g_fan.at(c));
+		i = j;
+	}
+	HA_CUDA(cudaGetLastError());
+	return g_fan.end(st);
+}
+
+// Gathered rows, eigen decompositions and factors of every item of a batch.
+int dgrid_factor(HaB200Plan *P, const DgPlan &pl, const DgBatch &b, const double *d_X, const double *d_Y,
+                 const DgParams &dp, cudaStream_t st) {
+	const size_t e0 = b.sl0 * dp.models;
+	const int ne = (int)((b.sl1 - b.sl0) * dp.models);
+	const DgItem *it = P->dgitem.p + e0;
+	double *S = P->gridscr.p;
+	{ HA_LAUNCH(kHaB200KGrid, st); k_dg_gather<<<ne, kBlock, 0, st>>>(it, P->dgsl.p + b.sl0, P->idx.p, d_X, d_Y, S, dp); }
+	int rc = dgrid_classes(pl, b, st, [&](int i, int cnt, int tn, cudaStream_t bs) {
+		HA_LAUNCH(kHaB200KXcov64, bs);
+		k_dg_gram<<<dim3(tn * (tn + 1) / 2 + pl.tt * tn, cnt * dp.models), kDgThreads, kDgSmem, bs>>>(it + (size_t)i * dp.models, S, dp);
+	});
+	if (rc != kHaSuccess) return rc;
+	const std::vector<int> ord(pl.orders.begin() + e0, pl.orders.begin() + e0 + ne);
+	if ((rc = launch_eig(P->dgeig.p + e0, ord, S, S, S, S, st)) != kHaSuccess) return rc;
+	{ HA_LAUNCH(kHaB200KScale, st); k_dg_flags<<<(ne + 127) / 128, 128, 0, st>>>(P->dgeig.p + e0, P->dgslot.p + e0, ne, S, P->stats.p); }
+	int max_d = 0;
+	for (int m = 0; m < dp.models; m++) max_d = std::max(max_d, P->dg_models[dp.model0 + m].d_n);
+	const int td = dg_tiles_of(max_d);
+	return dgrid_classes(pl, b, st, [&](int i, int cnt, int tn, cudaStream_t bs) {
+		const DgItem *ci = it + (size_t)i * dp.models;
+		const int tp = std::min(tn, td);
+		{ HA_LAUNCH(kHaB200KGrid, bs); k_dg_project<<<dim3((std::max(tn, td) + pl.tt) * tp, cnt * dp.models), kDgThreads, kDgSmem, bs>>>(ci, S, dp); }
+		{ HA_LAUNCH(kHaB200KGrid, bs); k_dg_lambda<<<dim3(8 * tp, cnt * dp.models), kBlock, 0, bs>>>(ci, S, dp); }
+		if (d_Y) { HA_LAUNCH(kHaB200KGrid, bs); k_dg_q<<<dim3(tp * tn, cnt * dp.models), kDgThreads, kDgSmem, bs>>>(ci, S, dp); }
+	});
+}
+
+// The float64 grid search of the searchlights `work` (slots of the current chunk): betas to the
+// float64 T scratch, winners and costs to d_best / d_cost.
+int dgrid_run(HaB200Plan *P, const std::vector<SlWork> &work, const double *d_X, const double *d_Y, const DgParams &dp,
+              int rowmajor, int32_t *d_best, double *d_cost, cudaStream_t st) {
+	DgPlan pl;
+	int rc = dgrid_plan(P, work, dp, pl, st);
+	if (rc != kHaSuccess) return rc;
+	double *S = P->gridscr.p;
+	for (const DgBatch &b : pl.batches) {
+		if ((rc = dgrid_factor(P, pl, b, d_X, d_Y, dp, st)) != kHaSuccess) return rc;
+		const DgItem *it = P->dgitem.p + b.sl0 * dp.models;
+		const DgSl *sl = P->dgsl.p + b.sl0;
+		rc = dgrid_classes(pl, b, st, [&](int i, int cnt, int tn, cudaStream_t bs) {
+			const DgItem *ci = it + (size_t)i * dp.models;
+			for (int a0 = 0; a0 < dp.n_alphas; a0 += pl.na) {
+				const int ca = std::min(pl.na, dp.n_alphas - a0);
+				if (pl.tt) { HA_LAUNCH(kHaB200KGrid, bs); k_dg_eval<<<dim3(pl.tt * tn, ca, cnt * dp.models), kDgThreads, kDgSmem, bs>>>(ci, sl, S, dp, a0); }
+				if (pl.rows) { HA_LAUNCH(kHaB200KGrid, bs); k_dg_cost<<<dim3(cnt, ca * dp.n_npcs, pl.rows), kBlock, 0, bs>>>(sl + i, S, dp, a0); }
+			}
+			{ HA_LAUNCH(kHaB200KGrid, bs); k_dg_best<<<cnt, kBlock, 0, bs>>>(sl + i, P->idx.p, d_Y, S, dp, d_best, d_cost); }
+			{ HA_LAUNCH(kHaB200KGrid, bs); k_dg_beta<<<dim3(tn * tn, cnt), kDgThreads, kDgSmem, bs>>>(it, sl + i, S, dp, d_best, nullptr, 0.0f, P->scrT64.p, rowmajor); }
+		});
+		if (rc != kHaSuccess) return rc;
+	}
+	return kHaSuccess;
+}
+
+// One chunk's plain FP32 grid search enqueued directly (sub-batch plan, scratch and offsets, launches).
+int grid_chunk32(HaB200Plan *P, Chunk &ch, const double *d_X, const double *d_Y, const GridSpec &gs,
+                 const GridParams &gp, int rowmajor, int32_t *d_best, double *d_cost, cudaStream_t st) {
 	std::vector<GridBatch> bt;
 	std::vector<int64_t> gbase;
-	grid_plan_chunk(ch, gp, fp32, bt, gbase);
+	grid_plan_chunk(ch, gp, bt, gbase);
 	int64_t mx = 1;
 	for (const auto &b : bt) mx = std::max(mx, b.total);
 	int rc;
@@ -1885,7 +2182,7 @@ int grid_chunk(HaB200Plan *P, Chunk &ch, const double *d_X, const double *d_Y, c
 	if ((rc = P->gbase.ensure(std::max<size_t>(gbase.size(), 1))) != kHaSuccess) return rc;
 	HA_CUDA(cudaMemcpyAsync(P->gbase.p, gbase.data(), gbase.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st));
 	HA_CUDA(cudaStreamSynchronize(st));  // the host vector goes out of scope
-	return grid_chunk_launch(P, ch, d_X, d_Y, gs, gp, fp32, bt, P->gbase.p, rowmajor, d_best, d_cost, st);
+	return grid_chunk_launch(P, ch, d_X, d_Y, gs, gp, bt, P->gbase.p, rowmajor, d_best, d_cost, st);
 }
 
 int run_ridge_grid(HaB200Plan *P, const double *d_X, const double *d_Y, const GridSpec &gs, int out_kind,
@@ -1894,6 +2191,19 @@ int run_ridge_grid(HaB200Plan *P, const double *d_X, const double *d_Y, const Gr
 	const bool fp32 = P->grid_bits == 32;
 	int rc;
 	if ((rc = grid_prepare(P)) != kHaSuccess) return rc;
+	if (!fp32) {
+		DgParams dp;
+		if ((rc = dgrid_upload(P, gs, st, dp)) != kHaSuccess) return rc;
+		HA_CUDA(cudaMemsetAsync(P->counters.p, 0, 5 * sizeof(int32_t), st));
+		for (Chunk &ch : P->chunks) {
+			HA_CUDA(cudaMemsetAsync(P->stats.p, 0, (size_t)(ch.s1 - ch.s0) * sizeof(SlStats), st));
+			if ((rc = dgrid_run(P, ch.w64, d_X, d_Y, dp, rowmajor, d_best, d_cost, st)) != kHaSuccess) return rc;
+			if ((rc = reduce_chunk64(P, ch, out_kind, d_vals, st)) != kHaSuccess) return rc;
+		}
+		P->last_chunk = (int)P->chunks.size() - 1;
+		P->last_rowmajor = rowmajor;
+		return kHaSuccess;
+	}
 	GridParams gp;
 	if ((rc = grid_upload(P, gs, st, gp)) != kHaSuccess) return rc;
 	// sub-batches of every chunk, their scratch offsets uploaded once, the scratch sized once: what
@@ -1905,7 +2215,7 @@ int run_ridge_grid(HaB200Plan *P, const double *d_X, const double *d_Y, const Gr
 	int64_t mx = 1;
 	for (size_t c = 0; c < P->chunks.size(); c++) {
 		gofs[c] = gbase.size();
-		grid_plan_chunk(P->chunks[c], gp, fp32, bts[c], gbase);
+		grid_plan_chunk(P->chunks[c], gp, bts[c], gbase);
 		for (const auto &b : bts[c]) mx = std::max(mx, b.total);
 	}
 	if ((rc = P->gridscr.ensure((size_t)mx)) != kHaSuccess) return rc;
@@ -1917,7 +2227,7 @@ int run_ridge_grid(HaB200Plan *P, const double *d_X, const double *d_Y, const Gr
 		for (size_t c = 0; c < P->chunks.size(); c++) {
 			Chunk &ch = P->chunks[c];
 			HA_CUDA(cudaMemsetAsync(P->stats.p, 0, (size_t)(ch.s1 - ch.s0) * sizeof(SlStats), ls));
-			int r = grid_chunk_launch(P, ch, d_X, d_Y, gs, gp, fp32, bts[c], P->gbase.p + gofs[c], rowmajor, d_best, d_cost, ls);
+			int r = grid_chunk_launch(P, ch, d_X, d_Y, gs, gp, bts[c], P->gbase.p + gofs[c], rowmajor, d_best, d_cost, ls);
 			if (r != kHaSuccess) return r;
 			if ((r = reduce_chunk64(P, ch, out_kind, d_vals, ls)) != kHaSuccess) return r;
 		}
@@ -1975,47 +2285,34 @@ int run_ridge_grid(HaB200Plan *P, const double *d_X, const double *d_Y, const Gr
 	return kHaSuccess;
 }
 
-// Eigen decomposition of every searchlight's Gram over the given rows (device list, n_rows
+// Plain FP32 eigen decomposition of every searchlight's Gram over the given rows (device list, n_rows
 // entries): the pivoted Cholesky factor and the eigenvector-mode Jacobi leave the eigenvectors in
 // the V scratch and the eigenvalues in the u/v buffer; with d_Y, C = X^T Y over the same rows goes
-// to the T scratch of the arithmetic type (float64 T scratch for double, float32 T scratch for
-// float).  Then the features of the chunk's searchlights.
-template <typename Real>
-int eigen_chunk(HaB200Plan *P, Chunk &ch, const double *d_X, const double *d_Y, const int32_t *d_rows, int n_rows,
-                float *d_feat, cudaStream_t st) {
-	constexpr bool f32 = sizeof(Real) == 4;
+// to the float32 T scratch.  Then the features of the chunk's searchlights.
+int eigen_chunk32(HaB200Plan *P, Chunk &ch, const double *d_X, const double *d_Y, const int32_t *d_rows, int n_rows,
+                  float *d_feat, cudaStream_t st) {
 	GridParams gp = {};
 	const JacobiParams jp = eig_params(false);
-	Real *A = reinterpret_cast<Real *>(P->scrA.p), *V = reinterpret_cast<Real *>(P->scrV.p);
-	Real *Cout = f32 ? reinterpret_cast<Real *>(P->scrT.p) : reinterpret_cast<Real *>(P->scrT64.p);
-	const std::vector<Bucket> &beig = f32 ? ch.beig32 : ch.beig;
-	const std::vector<SlWork> &items = f32 ? ch.weig32 : ch.weig;
-	SlWork *d_work = f32 ? ch.d_weig32 : ch.d_weig;
+	float *A = reinterpret_cast<float *>(P->scrA.p), *V = reinterpret_cast<float *>(P->scrV.p);
 	int rc;
 	if ((rc = g_fan.begin(st)) != kHaSuccess) return rc;
-	for (size_t bi = 0; bi < beig.size(); bi++) {
-		const Bucket &b = beig[bi];
+	for (size_t bi = 0; bi < ch.beig32.size(); bi++) {
+		const Bucket &b = ch.beig32[bi];
 		const cudaStream_t bs = g_fan.at((int)bi);
-		const SlWork *wk = d_work + b.first;
-		{ HA_LAUNCH(f32 ? kHaB200KXcov32 : kHaB200KXcov64, bs); k_xcov_rows<16, Real><<<b.count, kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_X, P->nt, d_rows, n_rows, V, nullptr, gp, 0); }
-		if (d_Y) { HA_LAUNCH(f32 ? kHaB200KXcov32 : kHaB200KXcov64, bs); k_xcov_rows<16, Real><<<b.count, kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_Y, P->nt, d_rows, n_rows, Cout, nullptr, gp, 2); }
-		{ HA_LAUNCH(kHaB200KRidge, bs); k_pchol<Real><<<b.count, kBlock, pchol_smem(b.rpl, sizeof(Real)), bs>>>(wk, V, A, P->stats.p); }
+		const SlWork *wk = ch.d_weig32 + b.first;
+		{ HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<16, float><<<b.count, kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_X, P->nt, d_rows, n_rows, V, nullptr, gp, 0); }
+		if (d_Y) { HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<16, float><<<b.count, kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_Y, P->nt, d_rows, n_rows, P->scrT.p, nullptr, gp, 2); }
+		{ HA_LAUNCH(kHaB200KRidge, bs); k_pchol<float><<<b.count, kBlock, pchol_smem(b.rpl), bs>>>(wk, V, A, P->stats.p); }
 		{
-			HA_LAUNCH(f32 ? kHaB200KJacobi32 : kHaB200KJacobi64, bs);
-			if ((rc = launch_jacobi<Real>(b.rpl, b.count, b.threads, b.smem, bs, wk, A, V, P->scrT.p, P->stats.p, P->uv.p, jp)) != kHaSuccess)
+			HA_LAUNCH(kHaB200KJacobi32, bs);
+			if ((rc = launch_jacobi<float>(b.rpl, b.count, b.threads, b.smem, bs, wk, A, V, P->scrT.p, P->stats.p, P->uv.p, jp)) != kHaSuccess)
 				return rc;
 		}
 	}
 	if ((rc = g_fan.end(st)) != kHaSuccess) return rc;
-	{ HA_LAUNCH(kHaB200KGrid, st); k_features<<<(int)items.size(), kBlock, 0, st>>>(d_work, P->uv.p, d_feat); }
+	{ HA_LAUNCH(kHaB200KGrid, st); k_features<<<(int)ch.weig32.size(), kBlock, 0, st>>>(ch.d_weig32, P->uv.p, d_feat); }
 	HA_CUDA(cudaGetLastError());
 	return kHaSuccess;
-}
-
-int eigen_chunk_any(HaB200Plan *P, Chunk &ch, const double *d_X, const double *d_Y, const int32_t *d_rows, int n_rows,
-                    float *d_feat, cudaStream_t st) {
-	return P->grid_bits == 32 ? eigen_chunk<float>(P, ch, d_X, d_Y, d_rows, n_rows, d_feat, st)
-	                          : eigen_chunk<double>(P, ch, d_X, d_Y, d_rows, n_rows, d_feat, st);
 }
 
 int upload_rows(HaB200Plan *P, const int32_t *rows, int n_rows, cudaStream_t st) {
@@ -2035,10 +2332,23 @@ int run_ridge_features(HaB200Plan *P, const double *d_X, const int32_t *rows, in
 	int rc;
 	if ((rc = grid_prepare(P)) != kHaSuccess) return rc;
 	if ((rc = upload_rows(P, rows, n_rows, st)) != kHaSuccess) return rc;
+	DgParams dp, fit;
+	if (P->grid_bits != 32 && (rc = dgrid_upload(P, GridSpec(), st, dp, rows, n_rows, &fit)) != kHaSuccess) return rc;
 	for (size_t c = 0; c < P->chunks.size(); c++) {
 		Chunk &ch = P->chunks[c];
 		HA_CUDA(cudaMemsetAsync(P->stats.p, 0, (size_t)(ch.s1 - ch.s0) * sizeof(SlStats), st));
-		if ((rc = eigen_chunk_any(P, ch, d_X, nullptr, P->gfit.p, n_rows, d_feat, st)) != kHaSuccess) return rc;
+		if (P->grid_bits == 32) {
+			if ((rc = eigen_chunk32(P, ch, d_X, nullptr, P->gfit.p, n_rows, d_feat, st)) != kHaSuccess) return rc;
+			continue;
+		}
+		DgPlan pl;
+		if ((rc = dgrid_plan(P, ch.w64, fit, pl, st)) != kHaSuccess) return rc;
+		for (const DgBatch &b : pl.batches) {
+			if ((rc = dgrid_factor(P, pl, b, d_X, nullptr, fit, st)) != kHaSuccess) return rc;
+			HA_LAUNCH(kHaB200KGrid, st);
+			k_dg_features<<<(int)(b.sl1 - b.sl0), kFeatSv, 0, st>>>(P->dgitem.p + b.sl0, P->dgsl.p + b.sl0, P->gridscr.p, d_feat);
+		}
+		HA_CUDA(cudaGetLastError());
 	}
 	return kHaSuccess;
 }
@@ -2057,51 +2367,75 @@ int run_ridge_learned(HaB200Plan *P, const double *d_X, const double *d_Y, const
 	if ((rc = grid_prepare(P)) != kHaSuccess) return rc;
 	if ((rc = upload_rows(P, rows, n_rows, st)) != kHaSuccess) return rc;
 	GridParams gp;
-	if ((rc = grid_upload(P, gs, st, gp)) != kHaSuccess) return rc;
-	if ((rc = P->gfeat.ensure((size_t)P->count * (kFeatSv + 1))) != kHaSuccess) return rc;
+	DgParams dp, fit;
+	if (fp32 && (rc = grid_upload(P, gs, st, gp)) != kHaSuccess) return rc;
+	if (!fp32 && (rc = dgrid_upload(P, gs, st, dp, rows, n_rows, &fit)) != kHaSuccess) return rc;
+	const size_t nfeat = (size_t)P->count * (kFeatSv + 1);
+	if ((rc = P->gfeat.ensure(nfeat)) != kHaSuccess) return rc;
+	HA_CUDA(cudaMemsetAsync(P->gfeat.p, 0, nfeat * sizeof(float), st));
 	HA_CUDA(cudaMemsetAsync(P->counters.p, 0, 5 * sizeof(int32_t), st));
 	std::vector<float> hprob;
 	for (size_t c = 0; c < P->chunks.size(); c++) {
 		Chunk &ch = P->chunks[c];
 		const int nsl = ch.s1 - ch.s0;
 		HA_CUDA(cudaMemsetAsync(P->stats.p, 0, (size_t)nsl * sizeof(SlStats), st));
-		if ((rc = eigen_chunk_any(P, ch, d_X, d_Y, P->gfit.p, n_rows, P->gfeat.p, st)) != kHaSuccess) return rc;
-		if ((rc = ha_b200_mlp_infer(d_params, C, P->gfeat.p + (size_t)ch.s0 * (kFeatSv + 1), nsl, d_choice + ch.s0,
-		                            d_prob + ch.s0, st)) != kHaSuccess)
-			return rc;
+		auto propose = [&]() {
+			return ha_b200_mlp_infer(d_params, C, P->gfeat.p + (size_t)ch.s0 * (kFeatSv + 1), nsl, d_choice + ch.s0,
+			                         d_prob + ch.s0, st);
+		};
 		if (fp32) {
+			if ((rc = eigen_chunk32(P, ch, d_X, d_Y, P->gfit.p, n_rows, P->gfeat.p, st)) != kHaSuccess) return rc;
+			if ((rc = propose()) != kHaSuccess) return rc;
 			HA_LAUNCH(kHaB200KGrid, st);
 			k_proposed_fit<float><<<(int)ch.weig32.size(), kBlock, 0, st>>>(ch.d_weig32, reinterpret_cast<const float *>(P->scrV.p), P->uv.p, reinterpret_cast<float *>(P->scrA.p), P->scrT.p, P->scrT64.p, d_choice, d_prob, min_prob, gp.alphas, gp.npcs, gp.n_npcs, n_rows, rowmajor);
 		} else {
-			HA_LAUNCH(kHaB200KGrid, st);
-			k_proposed_fit<double><<<(int)ch.weig.size(), kBlock, 0, st>>>(ch.d_weig, P->scrV.p, P->uv.p, P->scrA.p, P->scrT64.p, P->scrT64.p, d_choice, d_prob, min_prob, gp.alphas, gp.npcs, gp.n_npcs, n_rows, rowmajor);
+			// a batch's factors are at hand only until the next one's: the proposals are taken after every
+			// batch (those of searchlights without features yet are overwritten later)
+			DgPlan pl;
+			if ((rc = dgrid_plan(P, ch.w64, fit, pl, st)) != kHaSuccess) return rc;
+			for (const DgBatch &b : pl.batches) {
+				if ((rc = dgrid_factor(P, pl, b, d_X, d_Y, fit, st)) != kHaSuccess) return rc;
+				const DgItem *it = P->dgitem.p + b.sl0;
+				const DgSl *sl = P->dgsl.p + b.sl0;
+				{ HA_LAUNCH(kHaB200KGrid, st); k_dg_features<<<(int)(b.sl1 - b.sl0), kFeatSv, 0, st>>>(it, sl, P->gridscr.p, P->gfeat.p); }
+				if ((rc = propose()) != kHaSuccess) return rc;
+				rc = dgrid_classes(pl, b, st, [&](int i, int cnt, int tn, cudaStream_t bs) {
+					HA_LAUNCH(kHaB200KGrid, bs);
+					k_dg_beta<<<dim3(tn * tn, cnt), kDgThreads, kDgSmem, bs>>>(it, sl + i, P->gridscr.p, fit, d_choice, d_prob, min_prob, P->scrT64.p, rowmajor);
+				});
+				if (rc != kHaSuccess) return rc;
+			}
 		}
 		HA_CUDA(cudaGetLastError());
 		// searchlights below the threshold: the full grid search
 		hprob.resize((size_t)nsl);
 		HA_CUDA(cudaMemcpyAsync(hprob.data(), d_prob + ch.s0, (size_t)nsl * 4, cudaMemcpyDeviceToHost, st));
 		HA_CUDA(cudaStreamSynchronize(st));
-		// the fallback searchlights as a work list of their own (same buckets, same scratch slots)
-		Chunk fb;
-		fb.s0 = ch.s0;
-		fb.s1 = ch.s1;
-		const std::vector<Bucket> &cb = fp32 ? ch.beig32 : ch.beig;
-		const std::vector<SlWork> &cw = fp32 ? ch.weig32 : ch.weig;
-		std::vector<SlWork> &fw = fp32 ? fb.weig32 : fb.weig;
-		std::vector<Bucket> &fbk = fp32 ? fb.beig32 : fb.beig;
-		for (const Bucket &b : cb) {
-			Bucket nb = b;
-			nb.first = (int)fw.size();
-			for (int i = b.first; i < b.first + b.count; i++)
-				if (hprob[(size_t)(cw[i].s - ch.s0)] < min_prob) fw.push_back(cw[i]);
-			nb.count = (int)fw.size() - nb.first;
-			if (nb.count > 0) fbk.push_back(nb);
-		}
-		if (!fw.empty()) {
-			if ((rc = P->gwork.ensure(fw.size())) != kHaSuccess) return rc;
-			HA_CUDA(cudaMemcpyAsync(P->gwork.p, fw.data(), fw.size() * sizeof(SlWork), cudaMemcpyHostToDevice, st));
-			(fp32 ? fb.d_weig32 : fb.d_weig) = P->gwork.p;
-			if ((rc = grid_chunk(P, fb, d_X, d_Y, gs, gp, fp32, rowmajor, d_choice, nullptr, st)) != kHaSuccess) return rc;
+		// the fallback searchlights as a work list of their own (same scratch slots)
+		auto below = [&](const SlWork &w) { return hprob[(size_t)(w.s - ch.s0)] < min_prob; };
+		if (fp32) {
+			Chunk fb;  // same buckets
+			fb.s0 = ch.s0;
+			fb.s1 = ch.s1;
+			for (const Bucket &b : ch.beig32) {
+				Bucket nb = b;
+				nb.first = (int)fb.weig32.size();
+				for (int i = b.first; i < b.first + b.count; i++)
+					if (below(ch.weig32[i])) fb.weig32.push_back(ch.weig32[i]);
+				nb.count = (int)fb.weig32.size() - nb.first;
+				if (nb.count > 0) fb.beig32.push_back(nb);
+			}
+			if (!fb.weig32.empty()) {
+				if ((rc = P->gwork.ensure(fb.weig32.size())) != kHaSuccess) return rc;
+				HA_CUDA(cudaMemcpyAsync(P->gwork.p, fb.weig32.data(), fb.weig32.size() * sizeof(SlWork), cudaMemcpyHostToDevice, st));
+				fb.d_weig32 = P->gwork.p;
+				if ((rc = grid_chunk32(P, fb, d_X, d_Y, gs, gp, rowmajor, d_choice, nullptr, st)) != kHaSuccess) return rc;
+			}
+		} else {
+			std::vector<SlWork> fw;
+			for (const SlWork &w : ch.w64)
+				if (below(w)) fw.push_back(w);
+			if (!fw.empty() && (rc = dgrid_run(P, fw, d_X, d_Y, dp, rowmajor, d_choice, nullptr, st)) != kHaSuccess) return rc;
 		}
 		if ((rc = reduce_chunk64(P, ch, out_kind, d_vals, st)) != kHaSuccess) return rc;
 	}
@@ -2911,7 +3245,6 @@ void ha_b200_plan_destroy(HaB200Plan *P) {
 	for (auto &ch : P->chunks) {
 		if (ch.d_w32) cudaFree(ch.d_w32);
 		if (ch.d_w64) cudaFree(ch.d_w64);
-		if (ch.d_weig) cudaFree(ch.d_weig);
 		if (ch.d_weig32) cudaFree(ch.d_weig32);
 		if (ch.d_tofs) cudaFree(ch.d_tofs);
 		if (ch.d_tcw) cudaFree(ch.d_tcw);
@@ -2928,6 +3261,8 @@ void ha_b200_plan_destroy(HaB200Plan *P) {
 	P->gridscr.release(); P->galpha.release(); P->gwinv.release(); P->gbase.release(); P->gnpcs.release();
 	P->grows.release(); P->gtpos.release(); P->gurows.release(); P->guntested.release(); P->gmdl.release();
 	P->gfit.release(); P->gfeat.release(); P->gwork.release();
+	P->dgitem.release(); P->dgsl.release(); P->dgeig.release(); P->dgslot.release(); P->dgmdl.release();
+	P->dgint.release(); P->dgdbl.release(); P->eigscr.release();
 	P->tcXb.release(); P->tcYb.release(); P->tcXp.release(); P->tcXq.release(); P->tcPp.release(); P->tcA.release(); P->tcRes.release();
 	P->tcSt.release(); P->tcSched.release(); P->tcPlain.release(); P->tcQueue.release();
 	if (P->grid_graph) cudaGraphExecDestroy(P->grid_graph);

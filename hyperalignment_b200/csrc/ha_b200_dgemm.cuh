@@ -106,10 +106,12 @@ __device__ __forceinline__ void dg_mma(double (&c)[4], const double (&a)[4], con
 // 16 u + g + 8 (e >> 1), column 8 v + 2 t + (e & 1) of that 32 x 32 block (g = lane / 4, t = lane % 4).
 // Ends with a barrier, so the stages may be reused at once.  la and lb load the operands' K slices
 // (their rows already placed at m0 and n0); `safe` is any readable address, the source of the
-// zero-size copies of elements outside an operand.
+// zero-size copies of elements outside an operand.  cv (shared memory, may be null) scales slice k
+// of the product by cv[k].  A warp whose 32 x 32 block lies outside the product (active false) only helps
+// to load it.
 template <typename LA, typename LB>
 __device__ __forceinline__ void dgemm_core(const LA &la, const LB &lb, int K, const double *safe, double *sm,
-                                           double (&acc)[2][4][4]) {
+                                           double (&acc)[2][4][4], bool active = true, const double *cv = nullptr) {
 	constexpr bool AKC = LA::KC, BKC = LB::KC;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int g = lane >> 2, t = lane & 3, wm = 32 * (warp & 1), wn = 32 * (warp >> 1);
@@ -128,14 +130,24 @@ __device__ __forceinline__ void dgemm_core(const LA &la, const LB &lb, int K, co
 		asm volatile("cp.async.wait_group %0;" ::"n"(kDgStages - 2) : "memory");
 		__syncthreads();
 		fill(s + kDgStages - 1);
+		if (!active) continue;
 		const double *as = sm + (s % kDgStages) * 2 * kDgOperand, *bs = as + kDgOperand;
 #pragma unroll
 		for (int kk = 0; kk < kDgK; kk += 8) {
 			double a[2][4], b[4][2];
+			double c0 = 1.0, c1 = 1.0;
+			if (cv) {
+				const int k = s * kDgK + kk + t;
+				c0 = k < K ? cv[k] : 0.0;
+				c1 = k + 4 < K ? cv[k + 4] : 0.0;
+			}
 #pragma unroll
 			for (int u = 0; u < 2; u++)
 #pragma unroll
-				for (int e = 0; e < 4; e++) a[u][e] = dg_frag<AKC>(as, wm + 16 * u + g + 8 * (e & 1), kk + t + 4 * (e >> 1));
+				for (int e = 0; e < 4; e++) {
+					a[u][e] = dg_frag<AKC>(as, wm + 16 * u + g + 8 * (e & 1), kk + t + 4 * (e >> 1));
+					if (cv) a[u][e] *= e >> 1 ? c1 : c0;
+				}
 #pragma unroll
 			for (int v = 0; v < 4; v++)
 #pragma unroll
@@ -150,6 +162,12 @@ __device__ __forceinline__ void dgemm_core(const LA &la, const LB &lb, int K, co
 	__syncthreads();
 }
 
+// Whether the warp's 32 x 32 block of the tile at (m0, n0) holds any element of a rows x cols product.
+__device__ __forceinline__ bool dg_active(int m0, int rows, int n0, int cols) {
+	const int warp = threadIdx.x >> 5;
+	return m0 + 32 * (warp & 1) < rows && n0 + 32 * (warp >> 1) < cols;
+}
+
 template <bool AKC, bool BKC>
 __device__ __forceinline__ void dgemm_tile(const DgOperand &A, int m0, const DgOperand &B, int n0, int K, double *sm,
                                            double (&acc)[2][4][4]) {
@@ -157,7 +175,7 @@ __device__ __forceinline__ void dgemm_tile(const DgOperand &A, int m0, const DgO
 	DgLoader<BKC> lb;
 	la.init(A, m0, threadIdx.x);
 	lb.init(B, n0, threadIdx.x);
-	dgemm_core(la, lb, K, A.base, sm, acc);
+	dgemm_core(la, lb, K, A.base, sm, acc, dg_active(m0, A.rows, n0, B.rows));
 }
 
 // Lower tile b of a T x T grid: row ti holds ti + 1 tiles.

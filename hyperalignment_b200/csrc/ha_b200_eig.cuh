@@ -58,7 +58,7 @@ struct EigState {
 	int32_t next;    // first eigenvalue not yet found
 	int32_t sweeps;  // sweeps recorded in the last round
 	int32_t done;    // round (1, 2) in which the iteration finished, 0: not yet
-	int32_t pad_;
+	int32_t bad;     // ended without converging
 	double scale;    // the tridiagonal matrix holds T / scale
 };
 
@@ -486,6 +486,7 @@ __global__ void __launch_bounds__(32) k_eig_ql(const EigWork *__restrict__ work,
 		st->sweeps = ns;
 		st->scale = scale;
 		st->done = last ? round : 0;
+		st->bad = last && full ? 1 : 0;
 	}
 }
 

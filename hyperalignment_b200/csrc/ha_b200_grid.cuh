@@ -1,6 +1,6 @@
-// ha_b200_grid.cuh -- per-searchlight ridge grid search with cross-validated ensembles.  The grid
-// kernels are templated on the arithmetic type Real: double for the float64 search, float for the
-// plain FP32 form (inputs, alphas and the output betas stay float64).
+// ha_b200_grid.cuh -- per-searchlight ridge grid search with cross-validated ensembles, the plain FP32
+// form: the kernels are templated on the arithmetic type Real and instantiated with float (inputs,
+// alphas and the output betas stay float64).  The float64 search is ha_b200_dgrid.cuh.
 //
 // Composition of the reference's ha_ridge_grid (csrc/ha_ridge.c:97-227) and ha_ensemble_ridge
 // (csrc/ha_ridge.c:229-345) applied to every searchlight: X = X[:, sl] and the searchlight's n

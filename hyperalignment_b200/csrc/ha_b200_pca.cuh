@@ -119,12 +119,12 @@ __global__ void __launch_bounds__(kDgThreads) k_pca_gram(const SlWork *__restric
 		PcaLoader<true> la, lb;
 		la.init(D, sl, n, plane, nt, m, i0);
 		lb.init(D, sl, n, plane, nt, m, j0);
-		dgemm_core(la, lb, ns * n, D, dg_sm, acc);
+		dgemm_core(la, lb, ns * n, D, dg_sm, acc, dg_active(i0, m, j0, m));
 	} else {
 		PcaLoader<false> la, lb;
 		la.init(D, sl, n, plane, nt, m, i0);
 		lb.init(D, sl, n, plane, nt, m, j0);
-		dgemm_core(la, lb, nt, D, dg_sm, acc);
+		dgemm_core(la, lb, nt, D, dg_sm, acc, dg_active(i0, m, j0, m));
 	}
 	double *G = Gscr + w.aofs;
 	dg_each(acc, [&](int i, int j, double v) {

@@ -77,3 +77,45 @@ def test_pca_template_tile_edges(gpu, nt, ns, sizes):
     got = H.searchlight_pca_template(dms, sls, None, 1.0)
     ref = O.searchlight_pca_template(dms, idx, off, None, 1.0)
     assert np.linalg.norm(got - ref) / np.linalg.norm(ref) <= 1e-6
+
+
+# Costs are sums of squares whose predictions carry the conditioning of G + alpha I (here < 1e4 for
+# alpha >= 1e-1) times n eps; the repository's own bound for this search is 1e-8.
+@pytest.mark.parametrize("nt,sizes,folds", [
+    (150, [1, 2, 15, 16, 17, 63, 64, 65], 3),      # Gram and kernel forms of every model
+    (300, [40, 127, 128, 129, 191, 193, 300], 4),  # both sides of the distinct-row count
+])
+def test_ridge_grid_tile_edges(gpu, nt, sizes, folds):
+    from hyperalignment_b200 import hyperalignment_c as H
+    rng = np.random.default_rng(nt)
+    X, Y, idx, off = one_each(sizes, nt, nt)
+    Y = 0.3 * X + Y
+    tr = [rng.integers(0, nt, nt).astype(np.int32) for _ in range(folds)]
+    te = [np.setdiff1d(np.arange(nt), t).astype(np.int32)[:65 + 3 * k] for k, t in enumerate(tr)]
+    te[0] = te[0][:0]  # a model that tests nothing
+    sls = [idx[off[s]:off[s + 1]] for s in range(len(sizes))]
+    indptr, indices = H.sparse_pattern(sls, X.shape[1])
+    data = np.zeros(indices.size)
+    alphas, npcs = np.array([0.1, 3.0, 100.0]), [7, 16, 3, 33, 600]
+    best, costs = H.searchlight_ridge_grid(X, Y, sls, indptr, indices, data, alphas, npcs, tr, te, return_costs=True)
+    ref, rbest, rcosts = O.searchlight_ridge_grid_csc(X, Y, idx, off, indptr, indices, np.zeros(indices.size), alphas,
+                                                      npcs, tr, te, None)
+    np.testing.assert_allclose(costs, rcosts, rtol=1e-8, atol=0)
+    np.testing.assert_array_equal(best, rbest)
+    assert np.linalg.norm(data - ref) <= 1e-8 * np.linalg.norm(ref)
+
+
+# lambda is accurate to n eps lambda_max: a singular value at relative s to 512 * 2.2e-16 / (2 s), and a
+# Gaussian X of 700 rows keeps s > 0.1; the features are float32 (6e-8).
+def test_features_at_eigen_solver_orders(gpu):
+    import torch
+    sizes = [1, 2, 3, 15, 16, 17, 18, 63, 64, 65, 128, 129, 192, 193, 256, 257, 384, 385, 511, 512]
+    X, _, idx, off = one_each(sizes, 700, 9)
+    plan = Plan(700, X.shape[1], idx, off, weights=np.ones(idx.size))
+    f = torch.zeros((len(sizes), 65), dtype=torch.float32, device="cuda")
+    dX = upload(X)
+    plan.ridge_features_device(dX.data_ptr(), np.arange(700), f.data_ptr())
+    got = f.cpu().numpy()
+    plan.close()
+    ref = O.ridge_features(X, idx, off, np.arange(700))
+    np.testing.assert_allclose(got, ref, rtol=0, atol=2.5e-7)
