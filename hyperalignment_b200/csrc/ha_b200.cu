@@ -15,6 +15,7 @@
 #include "ha_b200_dgrid.cuh"
 #include "ha_b200_mlp.cuh"
 #include "ha_b200_tc.cuh"
+#include "ha_b200_tcres.cuh"
 #include "ha_b200_pca.cuh"
 
 #include <cuda_runtime.h>
@@ -319,6 +320,13 @@ struct Chunk {
 	TcTile *d_tct[2] = {nullptr, nullptr};
 	std::vector<int32_t> tco[2];  // persistent solve: work indices per size class, largest first
 	int32_t *d_tco[2] = {nullptr, nullptr};
+	// the resident iteration's searchlights, largest first: np > 128 (CTA pairs), 65-128, <= 64; the tiles of
+	// the searchlights that are left to the per-phase iteration follow `tct`'s classes
+	std::vector<int32_t> tcr[3];
+	int32_t *d_tcr[3] = {nullptr, nullptr, nullptr};
+	std::vector<TcTile> tcl[2];
+	TcTile *d_tcl[2] = {nullptr, nullptr};
+	unsigned char *d_tclists = nullptr;  // what the lists above lie in
 	// the tensor-core iteration loop of this chunk captured as a CUDA graph, and what it was
 	// captured for (output order, layouts); replayed while those are unchanged
 	cudaGraphExec_t tc_graph = nullptr;
@@ -970,9 +978,30 @@ int tc_small_ctas_per_sm() {
 	return v;
 }
 
+// The resident iteration for searchlights of np <= 256 (HA_B200_TC_RESIDENT=0: the per-phase kernels for
+// all; both give the same bits).
+bool tc_resident() {
+	static int v = -1;
+	if (v < 0) {
+		const char *e = getenv("HA_B200_TC_RESIDENT");
+		v = (e && e[0] == '0') ? 0 : 1;
+	}
+	return v == 1;
+}
+
+// Shared memory of a resident launch whose largest searchlight is np: a CTA pair holds all of tensor
+// memory, so it asks for more than half of the SM's shared memory and no second pair waits beside it.
+size_t tc_resident_smem(int np, int cl) {
+	const size_t s = tcres_smem(np, cl);
+	return cl == 2 ? std::max<size_t>(s, 116 * 1024) : s;
+}
+
 int set_tc_attrs() {
 	static bool done = false;
 	if (done) return kHaSuccess;
+	HA_CUDA(cudaFuncSetAttribute((k_tc_resident<1, 3>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_resident_smem(128, 1)));
+	HA_CUDA(cudaFuncSetAttribute((k_tc_resident<1, 2>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_resident_smem(64, 1)));
+	HA_CUDA(cudaFuncSetAttribute((k_tc_resident<2, 4>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_resident_smem(kTcResMaxNp, 2)));
 	HA_CUDA(cudaFuncSetAttribute(k_tc_gemm<kTcPhaseXcov>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemLarge));
 	HA_CUDA(cudaFuncSetAttribute(k_tc_gemm<kTcPhaseGram>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemLarge));
 	HA_CUDA(cudaFuncSetAttribute(k_tc_gemm<kTcPhaseUpdate>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemLarge));
@@ -1024,7 +1053,9 @@ int build_tc(HaB200Plan *P) {
 		for (int c = 0; c < 2; c++) {
 			ch.tct[c].clear();
 			ch.tco[c].clear();
+			ch.tcl[c].clear();
 		}
+		for (auto &r : ch.tcr) r.clear();
 		for (int q : order) {
 			const int np = ch.tcw[q].np;
 			const int c = np > 256 ? 1 : 0;
@@ -1036,19 +1067,34 @@ int build_tc(HaB200Plan *P) {
 				if (h0 < np) ch.tct[np - h0 <= 128 ? 0 : 1].push_back({q, t, h0, np - h0});
 			}
 			ch.tco[c].push_back(q);
+			if (tc_resident() && np <= kTcResMaxNp) {
+				ch.tcr[np > 128 ? 0 : np > 64 ? 1 : 2].push_back(q);
+			} else {
+				for (int t = 0; t * 128 < np; t++) {
+					ch.tcl[h0 <= 128 ? 0 : 1].push_back({q, t, 0, h0});
+					if (h0 < np) ch.tcl[np - h0 <= 128 ? 0 : 1].push_back({q, t, h0, np - h0});
+				}
+			}
 		}
-		if (cudaMalloc(&ch.d_tcw, (size_t)nsl * sizeof(TcWork)) != cudaSuccess) return kHaErrorAlloc;
-		HA_CUDA(cudaMemcpy(ch.d_tcw, ch.tcw.data(), (size_t)nsl * sizeof(TcWork), cudaMemcpyHostToDevice));
+		// the lists in one allocation and one copy
+		std::vector<unsigned char> blob;
+		std::vector<std::pair<void **, size_t>> at;
+		auto add = [&](auto &v, auto **d) {
+			at.push_back({(void **)d, blob.size()});
+			const unsigned char *b = (const unsigned char *)v.data();
+			blob.insert(blob.end(), b, b + v.size() * sizeof(v[0]));
+			blob.resize((blob.size() + 255) & ~(size_t)255);
+		};
+		add(ch.tcw, &ch.d_tcw);
 		for (int c = 0; c < 2; c++) {
-			const size_t cnt = std::max<size_t>(ch.tct[c].size(), 1);
-			if (cudaMalloc(&ch.d_tct[c], cnt * sizeof(TcTile)) != cudaSuccess) return kHaErrorAlloc;
-			if (!ch.tct[c].empty())
-				HA_CUDA(cudaMemcpy(ch.d_tct[c], ch.tct[c].data(), ch.tct[c].size() * sizeof(TcTile), cudaMemcpyHostToDevice));
-			const size_t co = std::max<size_t>(ch.tco[c].size(), 1);
-			if (cudaMalloc(&ch.d_tco[c], co * sizeof(int32_t)) != cudaSuccess) return kHaErrorAlloc;
-			if (!ch.tco[c].empty())
-				HA_CUDA(cudaMemcpy(ch.d_tco[c], ch.tco[c].data(), ch.tco[c].size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+			add(ch.tct[c], &ch.d_tct[c]);
+			add(ch.tco[c], &ch.d_tco[c]);
+			add(ch.tcl[c], &ch.d_tcl[c]);
 		}
+		for (int r = 0; r < 3; r++) add(ch.tcr[r], &ch.d_tcr[r]);
+		if (cudaMalloc(&ch.d_tclists, blob.size()) != cudaSuccess) return kHaErrorAlloc;
+		for (auto &x : at) *x.first = ch.d_tclists + x.second;
+		HA_CUDA(cudaMemcpy(ch.d_tclists, blob.data(), blob.size(), cudaMemcpyHostToDevice));
 	}
 	if ((rc = P->tcXp.ensure((size_t)maxX)) != kHaSuccess) return rc;
 	if ((rc = P->tcXq.ensure((size_t)maxX)) != kHaSuccess) return rc;
@@ -1129,14 +1175,15 @@ void launch_tc_tiles(int ntiles, TcArgs a, cudaStream_t st, int nmax, bool persi
 }
 
 // Launch one phase of the tile product over the size classes of a chunk (only class `only` when
-// it is 0 or 1), each with its layout's shared memory.
+// it is 0 or 1), each with its layout's shared memory; left: only the searchlights that the resident
+// iteration leaves.
 template <int PHASE>
 int launch_tc(const Chunk &ch, TcArgs a, cudaStream_t st, int kind, const int *smem, int only = -1,
-              bool persist = false) {
+              bool persist = false, bool left = false) {
 	for (int c = 0; c < 2; c++) {
-		const int ntiles = (int)ch.tct[c].size();
+		const int ntiles = (int)(left ? ch.tcl[c] : ch.tct[c]).size();
 		if (!ntiles || (only >= 0 && c != only)) continue;
-		a.tiles = ch.d_tct[c];
+		a.tiles = left ? ch.d_tcl[c] : ch.d_tct[c];
 		a.smem_bytes = smem[c];
 		HA_LAUNCH(kind, st);
 		launch_tc_tiles<PHASE>(ntiles, a, st, c ? 256 : 128, persist);
@@ -1307,14 +1354,53 @@ int run_procrustes_tc(HaB200Plan *P, const double *d_X, const double *d_Y, bool 
 				a.plain = sched[k].plain;
 				a.last = (k == maxit - 1) ? 1 : 0;
 				const bool persist = k >= tc_iter_from();
-				int r = launch_tc<kTcPhaseGram>(ch, a, ls, kHaB200KTcNs, P->tc_smem, -1, persist);
+				int r = launch_tc<kTcPhaseGram>(ch, a, ls, kHaB200KTcNs, P->tc_smem, -1, persist, true);
 				if (r != kHaSuccess) return r;
-				if ((r = launch_tc<kTcPhaseUpdate>(ch, a, ls, kHaB200KTcNs, P->tc_smem, -1, persist)) != kHaSuccess)
+				if ((r = launch_tc<kTcPhaseUpdate>(ch, a, ls, kHaB200KTcNs, P->tc_smem, -1, persist, true)) != kHaSuccess)
 					return r;
 			}
 			return kHaSuccess;
 		};
-		if (!graphs_enabled() || g_timing) {
+		// the resident iteration of the other searchlights beside it
+		if ((rc = g_fan.begin(st)) != kHaSuccess) return rc;
+		for (int r = 0; r < 3; r++) {
+			const int cnt = (int)ch.tcr[r].size();
+			if (!cnt) continue;
+			TcResArgs ra = {};
+			ra.work = ch.d_tcw;
+			ra.order = ch.d_tcr[r];
+			ra.X0 = P->tcXp.p;
+			ra.T = T;
+			ra.t_rowmajor = rowmajor;
+			ra.st_in = P->tcSt.p;
+			ra.st_out = P->tcSt.p + (size_t)(maxit & 1) * P->max_slots;
+			ra.c1 = P->tcSched.p;
+			ra.c3 = P->tcSched.p + maxit;
+			ra.plain = P->tcPlain.p;
+			ra.maxit = maxit;
+			ra.tol_stop = (float)ns_tol();
+			ra.err = P->counters.p + 4;
+			const int np = ch.tcw[ch.tcr[r][0]].np, cl = r == 0 ? 2 : 1;
+			cudaLaunchConfig_t cfg = {};
+			cfg.gridDim = dim3((unsigned)(cnt * cl));
+			cfg.blockDim = dim3(r == 0 ? 512 : r == 1 ? 384 : 256);
+			cfg.dynamicSmemBytes = tc_resident_smem(np, cl);
+			cfg.stream = g_fan.at(r);
+			cudaLaunchAttribute at[1];
+			at[0].id = cudaLaunchAttributeClusterDimension;
+			at[0].val.clusterDim.x = cl;
+			at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+			cfg.attrs = at;
+			cfg.numAttrs = 1;
+			HA_LAUNCH(kHaB200KTcNs, cfg.stream);
+			const cudaError_t le = r == 0 ? cudaLaunchKernelEx(&cfg, k_tc_resident<2, 4>, ra)
+			                     : r == 1 ? cudaLaunchKernelEx(&cfg, k_tc_resident<1, 3>, ra)
+			                              : cudaLaunchKernelEx(&cfg, k_tc_resident<1, 2>, ra);
+			HA_CUDA(le);
+		}
+		if (ch.tcl[0].empty() && ch.tcl[1].empty()) {
+			// nothing is left to the per-phase iteration
+		} else if (!graphs_enabled() || g_timing) {
 			if ((rc = enqueue_loop(st)) != kHaSuccess) return rc;
 		} else {
 			const int key[3] = {rowmajor, P->tc_smem[0], P->tc_smem[1]};
@@ -1351,6 +1437,7 @@ int run_procrustes_tc(HaB200Plan *P, const double *d_X, const double *d_Y, bool 
 			g_launches += ch.tc_graph_kernels;
 			g_kernel_n[kHaB200KTcNs] += ch.tc_graph_kernels;
 		}
+		if ((rc = g_fan.end(st)) != kHaSuccess) return rc;
 		{ HA_LAUNCH(kHaB200KTcNs, st); k_tc_ns_finish<<<nsl, 256, 0, st>>>(ch.d_tcw, P->tcA.p, T, P->tcSt.p + (size_t)(maxit & 1) * P->max_slots,
 		                                                              P->stats.p, rowmajor); }
 		}
@@ -3247,12 +3334,8 @@ void ha_b200_plan_destroy(HaB200Plan *P) {
 		if (ch.d_w64) cudaFree(ch.d_w64);
 		if (ch.d_weig32) cudaFree(ch.d_weig32);
 		if (ch.d_tofs) cudaFree(ch.d_tofs);
-		if (ch.d_tcw) cudaFree(ch.d_tcw);
+		if (ch.d_tclists) cudaFree(ch.d_tclists);
 		if (ch.tc_graph) cudaGraphExecDestroy(ch.tc_graph);
-		for (int c = 0; c < 2; c++) {
-			if (ch.d_tct[c]) cudaFree(ch.d_tct[c]);
-			if (ch.d_tco[c]) cudaFree(ch.d_tco[c]);
-		}
 	}
 	P->idx.release(); P->off.release(); P->lo.release(); P->hi.release(); P->w.release();
 	P->vlptr.release(); P->vlent.release(); P->patptr.release(); P->patcol.release();

@@ -119,3 +119,55 @@ def test_features_at_eigen_solver_orders(gpu):
     plan.close()
     ref = O.ridge_features(X, idx, off, np.arange(700))
     np.testing.assert_allclose(got, ref, rtol=0, atol=2.5e-7)
+
+
+_RESIDENT_SCRIPT = r"""
+import sys
+import numpy as np
+import torch
+sys.path.insert(0, sys.argv[1])
+from hyperalignment_b200 import _lib as L
+from hyperalignment_b200.plan import Plan
+rng = np.random.default_rng(5)
+sizes = [1, 15, 16, 17, 32, 33, 63, 64, 65, 80, 112, 127, 128, 129, 144, 145, 160, 176, 200, 208, 240, 241, 255, 256, 257, 300]
+nv, nt = 300, 400
+X = rng.standard_normal((nt, nv))
+Y = X @ np.linalg.qr(rng.standard_normal((nv, nv)))[0] + 0.1 * rng.standard_normal((nt, nv))
+X[:, 7] = X[:, 3]  # exactly singular searchlights among them
+idx = np.concatenate([np.arange(n) for n in sizes]).astype(np.int32)
+off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+plan = Plan(nt, nv, idx, off, weights=np.ones(idx.size))
+dX = torch.from_numpy(np.asfortranarray(X).ravel(order="F")).cuda()
+dY = torch.from_numpy(np.asfortranarray(Y).ravel(order="F")).cuda()
+out = {}
+for kind in (L.OUT_CSR, L.OUT_CSC):
+    v = torch.zeros(plan.nnz, dtype=torch.float64, device="cuda")
+    for _ in range(2):
+        v.zero_()
+        plan.procrustes_device(dX.data_ptr(), dY.data_ptr(), v.data_ptr(), True, True, L.SOLVER_TC, kind)
+    torch.cuda.synchronize()
+    out[f"v{kind}"] = v.cpu().numpy()
+    st = plan.searchlight_stats(0, len(sizes))
+    out[f"s{kind}"], out[f"f{kind}"], out[f"u{kind}"] = st["sweeps"], st["flags"], st["s_max"]
+    for s, T in enumerate(plan.local_transforms(0, len(sizes))):
+        out[f"T{kind}_{s}"] = T
+np.savez(sys.argv[2], **out)
+"""
+
+
+def test_resident_iteration_bitwise_equal(gpu, tmp_path):
+    """The iteration on resident planes (one CTA up to 128, a pair up to 256) and the per-phase kernels
+    (HA_B200_TC_RESIDENT=0) take the same products in the same order: transforms, values, iteration
+    counts and flags are identical bit for bit, at and around every tile size."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    res = []
+    for v in "01":
+        path = tmp_path / f"r{v}.npz"
+        subprocess.run([sys.executable, "-c", _RESIDENT_SCRIPT, root, str(path)],
+                       env=dict(os.environ, HA_B200_TC_RESIDENT=v), check=True, timeout=300)
+        res.append(np.load(path))
+    for k in res[0].files:
+        assert res[0][k].tobytes() == res[1][k].tobytes(), k
