@@ -620,6 +620,20 @@ int build_chunks(HaB200Plan *P) {
 	return kHaSuccess;
 }
 
+// The weighted sum of a chunk's local results into the pattern's values.
+template <typename TT>
+void launch_reduce(HaB200Plan *P, const Chunk &ch, const TT *T, int out_kind, double *d_vals, cudaStream_t st) {
+	const int cap = std::min(P->max_row, 16384);
+	const size_t with_map = (size_t)cap * sizeof(double) + (size_t)P->nv * sizeof(uint16_t);
+	const bool map = P->nv <= kReduceMapNv && cap == P->max_row && with_map <= kSmemMax;
+	const size_t smem = map ? with_map : (size_t)cap * 12;
+	HA_LAUNCH(kHaB200KReduce, st);
+	auto *k = map ? &k_reduce<TT, true> : &k_reduce<TT, false>;
+	(*k)<<<P->nv, kBlock, smem, st>>>(P->vlptr.p, P->vlent.p, P->off.p, P->idx.p, P->has_weights ? P->w.p : nullptr,
+	                                  P->patptr.p, P->patcol.p, T, ch.d_tofs, P->scale.p, ch.s0, ch.s1,
+	                                  out_kind == kHaB200OutCSC ? 1 : 0, cap, P->nv, d_vals);
+}
+
 __global__ void k_count_flags(const SlStats *__restrict__ st, int n, int32_t *__restrict__ counters) {
 	int q = blockIdx.x * blockDim.x + threadIdx.x;
 	if (q >= n) return;
@@ -637,8 +651,10 @@ int set_smem_attrs() {
 		fprintf(stderr, "ha_b200: cudaFuncSetAttribute on the Jacobi kernels failed\n");
 		return kHaErrorInternal;
 	}
-	HA_CUDA(cudaFuncSetAttribute(k_reduce<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
-	HA_CUDA(cudaFuncSetAttribute(k_reduce<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
+	HA_CUDA(cudaFuncSetAttribute((k_reduce<float, false>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
+	HA_CUDA(cudaFuncSetAttribute((k_reduce<double, false>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
+	HA_CUDA(cudaFuncSetAttribute((k_reduce<float, true>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
+	HA_CUDA(cudaFuncSetAttribute((k_reduce<double, true>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
 	HA_CUDA(cudaFuncSetAttribute(k_pattern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
 	HA_CUDA(cudaFuncSetAttribute(k_eig_tridiag<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)eig_tridiag_smem(512)));
 	HA_CUDA(cudaFuncSetAttribute(k_eig_tridiag<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)eig_tridiag_smem(384)));
@@ -1288,8 +1304,6 @@ int run_procrustes_tc(HaB200Plan *P, const double *d_X, const double *d_Y, bool 
 	static const std::vector<NsStep> sched = ns_schedule();
 	const int maxit = (int)sched.size();
 	float *T = P->scrT.p;
-	const int smem_cap = std::min(P->max_row, 16384);
-	const size_t red_smem = (size_t)smem_cap * 12;
 	for (size_t c = 0; c < P->chunks.size(); c++) {
 		Chunk &ch = P->chunks[c];
 		const int nsl = ch.s1 - ch.s0;
@@ -1473,10 +1487,7 @@ int run_procrustes_tc(HaB200Plan *P, const double *d_X, const double *d_Y, bool 
 		{ HA_LAUNCH(kHaB200KScale, st); k_scale<<<(nsl + 127) / 128, 128, 0, st>>>(ch.d_w64, nsl, P->idx.p, P->var.p, P->stats.p, nt, scal ? 1 : 0,
 		                                          P->scale.p); }
 		{ HA_LAUNCH(kHaB200KScale, st); k_count_flags<<<(nsl + 127) / 128, 128, 0, st>>>(P->stats.p, nsl, P->counters.p); }
-		{ HA_LAUNCH(kHaB200KReduce, st); k_reduce<float><<<nv, kBlock, red_smem, st>>>(P->vlptr.p, P->vlent.p, P->off.p, P->idx.p,
-		                                       P->has_weights ? P->w.p : nullptr, P->patptr.p, P->patcol.p, T,
-		                                       ch.d_tofs, P->scale.p, ch.s0, ch.s1, out_kind == kHaB200OutCSC ? 1 : 0,
-		                                       smem_cap, d_vals); }
+		launch_reduce<float>(P, ch, T, out_kind, d_vals, st);
 		HA_CUDA(cudaGetLastError());
 	}
 	P->last_chunk = (int)P->chunks.size() - 1;
@@ -1517,8 +1528,6 @@ int run_procrustes(HaB200Plan *P, const double *d_X, const double *d_Y, bool ref
 	}
 	HA_CUDA(cudaMemsetAsync(P->counters.p, 0, 5 * sizeof(int32_t), st));
 	float *T = P->scrT.p;
-	int smem_cap = std::min(P->max_row, 16384);
-	size_t red_smem = (size_t)smem_cap * 12;
 	for (size_t c = 0; c < P->chunks.size(); c++) {
 		Chunk &ch = P->chunks[c];
 		const int nsl = ch.s1 - ch.s0;
@@ -1583,10 +1592,7 @@ int run_procrustes(HaB200Plan *P, const double *d_X, const double *d_Y, bool ref
 		{ HA_LAUNCH(kHaB200KScale, st); k_scale<<<(nsl + 127) / 128, 128, 0, st>>>(ch.d_w64, nsl, P->idx.p, P->var.p, P->stats.p, nt, scal ? 1 : 0,
 		                                          P->scale.p); }
 		{ HA_LAUNCH(kHaB200KScale, st); k_count_flags<<<(nsl + 127) / 128, 128, 0, st>>>(P->stats.p, nsl, P->counters.p); }
-		{ HA_LAUNCH(kHaB200KReduce, st); k_reduce<float><<<nv, kBlock, red_smem, st>>>(P->vlptr.p, P->vlent.p, P->off.p, P->idx.p,
-		                                       P->has_weights ? P->w.p : nullptr, P->patptr.p, P->patcol.p, T,
-		                                       ch.d_tofs, P->scale.p, ch.s0, ch.s1, out_kind == kHaB200OutCSC ? 1 : 0,
-		                                       smem_cap, d_vals); }
+		launch_reduce<float>(P, ch, T, out_kind, d_vals, st);
 		HA_CUDA(cudaGetLastError());
 	}
 	P->last_chunk = (int)P->chunks.size() - 1;
@@ -1597,7 +1603,7 @@ int run_procrustes(HaB200Plan *P, const double *d_X, const double *d_Y, bool ref
 // Enqueue the searchlight ridge solve + reduction over all chunks (float64 throughout).
 int run_ridge(HaB200Plan *P, const double *d_X, const double *d_Y, double alpha, int out_kind, double *d_vals,
               cudaStream_t st) {
-	const int nt = P->nt, nv = P->nv;
+	const int nt = P->nt;
 	const int rowmajor = out_kind == kHaB200OutCSR ? 1 : 0;
 	int rc;
 	if (P->chunks.empty() && (rc = build_chunks(P)) != kHaSuccess) return rc;
@@ -1605,8 +1611,6 @@ int run_ridge(HaB200Plan *P, const double *d_X, const double *d_Y, double alpha,
 	for (auto &ch : P->chunks) maxT = std::max(maxT, ch.t_elems);
 	if ((rc = P->scrT64.ensure((size_t)maxT)) != kHaSuccess) return rc;
 	HA_CUDA(cudaMemsetAsync(P->counters.p, 0, 5 * sizeof(int32_t), st));
-	const int smem_cap = std::min(P->max_row, 16384);
-	const size_t red_smem = (size_t)smem_cap * 12;
 	for (size_t c = 0; c < P->chunks.size(); c++) {
 		Chunk &ch = P->chunks[c];
 		const int nsl = ch.s1 - ch.s0;
@@ -1628,10 +1632,7 @@ int run_ridge(HaB200Plan *P, const double *d_X, const double *d_Y, double alpha,
 		if ((rc = g_fan.end(st)) != kHaSuccess) return rc;
 		{ HA_LAUNCH(kHaB200KScale, st); k_scale<<<(nsl + 127) / 128, 128, 0, st>>>(ch.d_w64, nsl, P->idx.p, nullptr, P->stats.p, nt, 0, P->scale.p); }
 		{ HA_LAUNCH(kHaB200KScale, st); k_count_flags<<<(nsl + 127) / 128, 128, 0, st>>>(P->stats.p, nsl, P->counters.p); }
-		{ HA_LAUNCH(kHaB200KReduce, st); k_reduce<double><<<nv, kBlock, red_smem, st>>>(P->vlptr.p, P->vlent.p, P->off.p, P->idx.p,
-		                                       P->has_weights ? P->w.p : nullptr, P->patptr.p, P->patcol.p, P->scrT64.p,
-		                                       ch.d_tofs, P->scale.p, ch.s0, ch.s1, out_kind == kHaB200OutCSC ? 1 : 0,
-		                                       smem_cap, d_vals); }
+		launch_reduce<double>(P, ch, P->scrT64.p, out_kind, d_vals, st);
 		HA_CUDA(cudaGetLastError());
 	}
 	P->last_chunk = (int)P->chunks.size() - 1;
@@ -1856,14 +1857,9 @@ JacobiParams eig_params(bool only_flagged) {
 // Scale (1), flag counts and the deterministic reduction of one chunk's float64 betas.
 int reduce_chunk64(HaB200Plan *P, Chunk &ch, int out_kind, double *d_vals, cudaStream_t st) {
 	const int nsl = ch.s1 - ch.s0;
-	const int smem_cap = std::min(P->max_row, 16384);
-	const size_t red_smem = (size_t)smem_cap * 12;
 	{ HA_LAUNCH(kHaB200KScale, st); k_scale<<<(nsl + 127) / 128, 128, 0, st>>>(ch.d_w64, nsl, P->idx.p, nullptr, P->stats.p, P->nt, 0, P->scale.p); }
 	{ HA_LAUNCH(kHaB200KScale, st); k_count_flags<<<(nsl + 127) / 128, 128, 0, st>>>(P->stats.p, nsl, P->counters.p); }
-	{ HA_LAUNCH(kHaB200KReduce, st); k_reduce<double><<<P->nv, kBlock, red_smem, st>>>(P->vlptr.p, P->vlent.p, P->off.p, P->idx.p,
-	                                       P->has_weights ? P->w.p : nullptr, P->patptr.p, P->patcol.p, P->scrT64.p,
-	                                       ch.d_tofs, P->scale.p, ch.s0, ch.s1, out_kind == kHaB200OutCSC ? 1 : 0,
-	                                       smem_cap, d_vals); }
+	launch_reduce<double>(P, ch, P->scrT64.p, out_kind, d_vals, st);
 	HA_CUDA(cudaGetLastError());
 	return kHaSuccess;
 }

@@ -1260,70 +1260,126 @@ __global__ void k_pattern(const int64_t *__restrict__ vl_ptr, const int2 *__rest
 // One CTA per vertex v.  Its entries (s, a) (v is member a of searchlight s) are sorted by s;
 // those of the current chunk [s_lo, s_hi) are visited in that order, and for each one the
 // whole row a of the searchlight's M_s (M_s = T_s for CSR output, T_s^T for CSC output) is
-// added at the slots of its columns, found by binary search in v's sorted pattern row.
+// added at the slots of its columns in v's sorted pattern row.
 // Within one searchlight the columns are distinct, so threads never collide; a barrier
 // separates searchlights, so every sum runs in ascending searchlight order on every run.
 //   CSR (row v = dense row v):   val(v, u_b) += w_s[a] * scale_s * T_s[a][b]
 //   CSC (column v):              val(u_b, v) += w_s[b] * scale_s * T_s[b][a]
-template <typename TT>
+// A barrier per searchlight makes the chain of one entry the bound (measured 4.0 ms for 10,242 vertices
+// with about 200 entries each, when every entry followed its list entry, offsets, columns and a binary
+// search of each slot in turn).  So the entries' addresses and factors are gathered 64 at a time, the
+// next entry's columns and row are on their way while the current one is added, and with MAP the
+// slots come from a table over the vertices in shared memory (two bytes each, nv <= kReduceMapNv;
+// above that the binary search stays).
+constexpr int kReduceBatch = 64;
+constexpr int kReducePer = 2;          // columns per thread and entry (n <= 512)
+constexpr int kReduceMapNv = 49152;    // 96 KB of table: two CTAs an SM
+
+template <typename TT, bool MAP>
 __global__ void __launch_bounds__(256) k_reduce(const int64_t *__restrict__ vl_ptr, const int2 *__restrict__ vl_ent,
                                                 const int32_t *__restrict__ sl_off, const int32_t *__restrict__ sl_idx,
                                                 const double *__restrict__ wts, const int64_t *__restrict__ pat_ptr,
                                                 const int32_t *__restrict__ pat_col, const TT *__restrict__ Tscr,
                                                 const int64_t *__restrict__ tofs_by_slot,
                                                 const double *__restrict__ scale_by_slot, int s_lo, int s_hi,
-                                                int csc, int smem_cap, double *__restrict__ values) {
+                                                int csc, int smem_cap, int nv, double *__restrict__ values) {
 	extern __shared__ __align__(16) unsigned char smem_raw[];
+	__shared__ int64_t s_row[kReduceBatch];  // element offset of row a of M_s
+	__shared__ double s_sc[kReduceBatch];    // scale_s (CSC) or w_s[a] * scale_s
+	__shared__ int2 s_sl[kReduceBatch];      // flat offset and size of searchlight s
 	const int v = blockIdx.x;
 	const int64_t e0 = vl_ptr[v], e1 = vl_ptr[v + 1];
-	// first entry with s >= s_lo (entries sorted by s)
-	int64_t lo = e0, hi = e1;
-	while (lo < hi) {
-		int64_t mid = (lo + hi) >> 1;
-		if (vl_ent[mid].x < s_lo) lo = mid + 1; else hi = mid;
-	}
-	const int64_t eb = lo;
-	if (eb >= e1 || vl_ent[eb].x >= s_hi) return;
+	// the entries with s_lo <= s < s_hi (sorted by s)
+	auto first_at = [&](int s) {
+		int64_t lo = e0, hi = e1;
+		while (lo < hi) {
+			const int64_t mid = (lo + hi) >> 1;
+			if (vl_ent[mid].x < s) lo = mid + 1; else hi = mid;
+		}
+		return lo;
+	};
+	const int64_t eb = first_at(s_lo), ee = first_at(s_hi);
+	if (eb >= ee) return;
 	const int64_t p0 = pat_ptr[v];
 	const int L = (int)(pat_ptr[v + 1] - p0);
 	const bool in_smem = L <= smem_cap;
 	double *acc;
 	const int32_t *cols;
+	uint16_t *map = nullptr;
+	if (MAP) map = reinterpret_cast<uint16_t *>(smem_raw + (size_t)smem_cap * sizeof(double));
 	if (in_smem) {
 		acc = reinterpret_cast<double *>(smem_raw);
-		int32_t *cs = reinterpret_cast<int32_t *>(acc + L);
+		int32_t *cs = MAP ? nullptr : reinterpret_cast<int32_t *>(acc + L);
 		for (int k = threadIdx.x; k < L; k += blockDim.x) {
 			acc[k] = values[p0 + k];
-			cs[k] = pat_col[p0 + k];
+			if (MAP) map[pat_col[p0 + k]] = (uint16_t)k;
+			else cs[k] = pat_col[p0 + k];
 		}
 		cols = cs;
-		__syncthreads();
 	} else {
 		acc = values + p0;
 		cols = pat_col + p0;
 	}
-	for (int64_t e = eb; e < e1; e++) {
-		const int2 ent = vl_ent[e];
-		const int s = ent.x;
-		if (s >= s_hi) break;
-		const int a = ent.y;
-		const int o0 = sl_off[s];
-		const int n = sl_off[s + 1] - o0;
-		const int slot = s - s_lo;
-		const TT *M = Tscr + tofs_by_slot[slot] + (int64_t)a * n;
-		const double sc = scale_by_slot[slot];
-		const double wa = wts ? wts[o0 + a] : 1.0;
-		for (int b = threadIdx.x; b < n; b += blockDim.x) {
-			const int u = sl_idx[o0 + b];
-			int l = 0, h = L;
-			while (l < h) {
-				int mid = (l + h) >> 1;
-				if (cols[mid] < u) l = mid + 1; else h = mid;
-			}
-			double wgt = csc ? (wts ? wts[o0 + b] : 1.0) : wa;
-			acc[l] += (double)M[b] * (wgt * sc);
+	for (int64_t eq = eb; eq < ee; eq += kReduceBatch) {
+		const int ne = (int)min((int64_t)kReduceBatch, ee - eq);
+		__syncthreads();
+		if ((int)threadIdx.x < ne) {
+			const int2 ent = vl_ent[eq + threadIdx.x];
+			const int o0 = sl_off[ent.x], n = sl_off[ent.x + 1] - o0, slot = ent.x - s_lo;
+			const double sc = scale_by_slot[slot];
+			s_row[threadIdx.x] = tofs_by_slot[slot] + (int64_t)ent.y * n;
+			s_sl[threadIdx.x] = make_int2(o0, n);
+			s_sc[threadIdx.x] = csc ? sc : (wts ? wts[o0 + ent.y] : 1.0) * sc;
 		}
 		__syncthreads();
+		int u[kReducePer];
+		TT m[kReducePer];
+		double wb[kReducePer];
+		auto fetch = [&](int e) {
+			const int2 sl = s_sl[e];
+			const TT *M = Tscr + s_row[e];
+#pragma unroll
+			for (int q = 0; q < kReducePer; q++) {
+				const int b = threadIdx.x + 256 * q;
+				u[q] = -1;
+				if (b < sl.y) {
+					u[q] = sl_idx[sl.x + b];
+					m[q] = M[b];
+					wb[q] = csc && wts ? wts[sl.x + b] : 1.0;
+				}
+			}
+		};
+		fetch(0);
+		for (int e = 0; e < ne; e++) {
+			const double sc = s_sc[e];
+			int cu[kReducePer];
+			TT cm[kReducePer];
+			double cw[kReducePer];
+#pragma unroll
+			for (int q = 0; q < kReducePer; q++) {
+				cu[q] = u[q];
+				cm[q] = m[q];
+				cw[q] = wb[q];
+			}
+			if (e + 1 < ne) fetch(e + 1);
+#pragma unroll
+			for (int q = 0; q < kReducePer; q++) {
+				if (cu[q] < 0) continue;
+				int l = 0;
+				if (MAP && in_smem) {
+					l = map[cu[q]];
+				} else {
+					const int32_t *cl = MAP ? pat_col + p0 : cols;
+					int h = L;
+					while (l < h) {
+						const int mid = (l + h) >> 1;
+						if (cl[mid] < cu[q]) l = mid + 1; else h = mid;
+					}
+				}
+				acc[l] += (double)cm[q] * (csc ? cw[q] * sc : sc);
+			}
+			__syncthreads();
+		}
 	}
 	if (in_smem) {
 		for (int k = threadIdx.x; k < L; k += blockDim.x) values[p0 + k] = acc[k];
