@@ -16,6 +16,7 @@
 #include "ha_b200_mlp.cuh"
 #include "ha_b200_tc.cuh"
 #include "ha_b200_tcres.cuh"
+#include "ha_b200_tcxcov.cuh"
 #include "ha_b200_pca.cuh"
 
 #include <cuda_runtime.h>
@@ -318,6 +319,8 @@ struct Chunk {
 	std::vector<TcTile> tct[2];
 	TcWork *d_tcw = nullptr;
 	TcTile *d_tct[2] = {nullptr, nullptr};
+	std::vector<TcTile> tcx[2];  // the cross-covariance's tiles (tcx_tiles)
+	TcTile *d_tcx[2] = {nullptr, nullptr};
 	std::vector<int32_t> tco[2];  // persistent solve: work indices per size class, largest first
 	int32_t *d_tco[2] = {nullptr, nullptr};
 	// the resident iteration's searchlights, largest first: np > 128 (CTA pairs), 65-128, <= 64; the tiles of
@@ -1018,7 +1021,7 @@ int set_tc_attrs() {
 	HA_CUDA(cudaFuncSetAttribute((k_tc_resident<1, 3>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_resident_smem(128, 1)));
 	HA_CUDA(cudaFuncSetAttribute((k_tc_resident<1, 2>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_resident_smem(64, 1)));
 	HA_CUDA(cudaFuncSetAttribute((k_tc_resident<2, 4>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_resident_smem(kTcResMaxNp, 2)));
-	HA_CUDA(cudaFuncSetAttribute(k_tc_gemm<kTcPhaseXcov>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemLarge));
+	HA_CUDA(cudaFuncSetAttribute(k_tc_xcov, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcXSmem[1]));
 	HA_CUDA(cudaFuncSetAttribute(k_tc_gemm<kTcPhaseGram>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemLarge));
 	HA_CUDA(cudaFuncSetAttribute(k_tc_gemm<kTcPhaseUpdate>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemLarge));
 	HA_CUDA(cudaFuncSetAttribute(k_tc_gemm<kTcPhaseGram, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemLarge));
@@ -1070,6 +1073,7 @@ int build_tc(HaB200Plan *P) {
 			ch.tct[c].clear();
 			ch.tco[c].clear();
 			ch.tcl[c].clear();
+			ch.tcx[c].clear();
 		}
 		for (auto &r : ch.tcr) r.clear();
 		for (int q : order) {
@@ -1082,6 +1086,7 @@ int build_tc(HaB200Plan *P) {
 				ch.tct[h0 <= 128 ? 0 : 1].push_back({q, t, 0, h0});
 				if (h0 < np) ch.tct[np - h0 <= 128 ? 0 : 1].push_back({q, t, h0, np - h0});
 			}
+			tcx_tiles(q, np, [&](int cls, const TcTile &tl) { ch.tcx[cls].push_back(tl); });
 			ch.tco[c].push_back(q);
 			if (tc_resident() && np <= kTcResMaxNp) {
 				ch.tcr[np > 128 ? 0 : np > 64 ? 1 : 2].push_back(q);
@@ -1106,6 +1111,7 @@ int build_tc(HaB200Plan *P) {
 			add(ch.tct[c], &ch.d_tct[c]);
 			add(ch.tco[c], &ch.d_tco[c]);
 			add(ch.tcl[c], &ch.d_tcl[c]);
+			add(ch.tcx[c], &ch.d_tcx[c]);
 		}
 		for (int r = 0; r < 3; r++) add(ch.tcr[r], &ch.d_tcr[r]);
 		if (cudaMalloc(&ch.d_tclists, blob.size()) != cudaSuccess) return kHaErrorAlloc;
@@ -1172,22 +1178,28 @@ int tc_iter_from() {
 // persistent kernel when `persist`.
 template <int PHASE>
 void launch_tc_tiles(int ntiles, TcArgs a, cudaStream_t st, int nmax, bool persist) {
-	if constexpr (PHASE != kTcPhaseXcov) {
-		if (persist) {
-			// stages for the tiles' widest B, then the CTA's tile list; enough CTAs that none holds
-			// more than kTcIterMaxTiles tiles (beyond one per SM they run in later waves)
-			const int stage = 2 * 4096 + 64 * nmax;
-			const int list = kTcIterMaxTiles * (int)sizeof(TcIterTile);
-			a.smem_bytes = std::min(kTcMaxStages, (int)(kSmemMax - list) / stage) * stage + list;
-			const int grid = std::min(ntiles, std::max(g_num_sms, (ntiles + kTcIterMaxTiles - 1) / kTcIterMaxTiles));
-			k_tc_iter<PHASE><<<grid, kTcIterThreads, a.smem_bytes, st>>>(a, ntiles, nmax);
-			return;
-		}
+	if (persist) {
+		// stages for the tiles' widest B, then the CTA's tile list; enough CTAs that none holds
+		// more than kTcIterMaxTiles tiles (beyond one per SM they run in later waves)
+		const int stage = 2 * 4096 + 64 * nmax;
+		const int list = kTcIterMaxTiles * (int)sizeof(TcIterTile);
+		a.smem_bytes = std::min(kTcMaxStages, (int)(kSmemMax - list) / stage) * stage + list;
+		const int grid = std::min(ntiles, std::max(g_num_sms, (ntiles + kTcIterMaxTiles - 1) / kTcIterMaxTiles));
+		k_tc_iter<PHASE><<<grid, kTcIterThreads, a.smem_bytes, st>>>(a, ntiles, nmax);
+		return;
 	}
-	if (PHASE != kTcPhaseXcov && (tc_bulk_mask() >> (PHASE > 0 ? PHASE - 1 : 0) & 1))
-		k_tc_gemm<PHASE, PHASE != kTcPhaseXcov><<<ntiles, kTcThreads, a.smem_bytes, st>>>(a);
+	if (tc_bulk_mask() >> (PHASE - 1) & 1)
+		k_tc_gemm<PHASE, true><<<ntiles, kTcThreads, a.smem_bytes, st>>>(a);
 	else
 		k_tc_gemm<PHASE><<<ntiles, kTcThreads, a.smem_bytes, st>>>(a);
+}
+
+void launch_tc_xcov(const TcTile *tiles, int ntiles, int cls, TcXArgs x, cudaStream_t st) {
+	if (!ntiles) return;
+	x.tiles = tiles;
+	x.smem_bytes = kTcXSmem[cls];
+	HA_LAUNCH(kHaB200KTcXcov, st);
+	k_tc_xcov<<<ntiles, kTcXThreads, x.smem_bytes, st>>>(x);
 }
 
 // Launch one phase of the tile product over the size classes of a chunk (only class `only` when
@@ -1286,7 +1298,7 @@ int autotune_tc(HaB200Plan *P, const Chunk &ch, TcArgs a, cudaStream_t st) {
 int run_procrustes_tc(HaB200Plan *P, const double *d_X, const double *d_Y, bool scal, int out_kind, double *d_vals,
                       cudaStream_t st) {
 	const int nt = P->nt, nv = P->nv;
-	const int ntp = (nt + 15) & ~15;
+	const int ntp = (nt + kTcXK - 1) / kTcXK * kTcXK;
 	const int rowmajor = out_kind == kHaB200OutCSR ? 1 : 0;
 	int rc;
 	if (P->chunks.empty() && (rc = build_chunks(P)) != kHaSuccess) return rc;
@@ -1310,15 +1322,9 @@ int run_procrustes_tc(HaB200Plan *P, const double *d_X, const double *d_Y, bool 
 		HA_CUDA(cudaMemsetAsync(P->stats.p, 0, (size_t)nsl * sizeof(SlStats), st));
 		TcArgs a = {};
 		a.work = ch.d_tcw;
-		a.Xb = P->tcXb.p;
-		a.Yb = P->tcYb.p;
-		a.vplane = vplane;
-		a.ntp = ntp;
-		a.sl_idx = P->idx.p;
 		a.Xp = P->tcXp.p;
 		a.Xw = P->tcXq.p;
 		a.Pp = P->tcPp.p;
-		a.A32 = P->tcA.p;
 		a.T = T;
 		a.t_rowmajor = rowmajor;
 		a.res_part = P->tcRes.p;
@@ -1347,7 +1353,10 @@ int run_procrustes_tc(HaB200Plan *P, const double *d_X, const double *d_Y, bool 
 			}
 			HA_CUDA(cudaGetLastError());
 		} else {
-		if ((rc = launch_tc<kTcPhaseXcov>(ch, a, st, kHaB200KTcXcov, P->tc_smem)) != kHaSuccess) return rc;
+		// the wider tiles (one CTA per SM) first
+		for (int x = 1; x >= 0; x--)
+			launch_tc_xcov(ch.d_tcx[x], (int)ch.tcx[x].size(), x,
+			               TcXArgs{ch.d_tcw, nullptr, P->tcXb.p, P->tcYb.p, vplane, ntp, P->idx.p, P->tcA.p, 0, P->counters.p + 4}, st);
 		{ HA_LAUNCH(kHaB200KTcNs, st); k_tc_ns_init<<<nsl, 256, 0, st>>>(ch.d_tcw, P->tcA.p, P->tcXp.p, P->tcSt.p, P->tcRes.p); }
 		if (!P->tc_tuned && autotune_enabled()) {
 			a.st_in = P->tcSt.p;
@@ -3705,7 +3714,7 @@ int ha_b200_tc_selftest(int32_t which, int32_t n, int32_t nt, const float *h_a, 
 	if (rc != kHaSuccess) return rc;
 	if ((rc = set_tc_attrs()) != kHaSuccess) return rc;
 	const int np = (n + 15) & ~15;
-	const int ntp = (nt + 15) & ~15;
+	const int ntp = (nt + kTcXK - 1) / kTcXK * kTcXK;
 	const int64_t pe3 = 3 * (int64_t)np * np;
 	DevArr<__nv_bfloat16> Xp, Pp, Xb, Yb;
 	DevArr<float> A32, T, R, in0, in1;
@@ -3734,6 +3743,12 @@ int ha_b200_tc_selftest(int32_t which, int32_t n, int32_t nt, const float *h_a, 
 		tiles.push_back({0, t, 0, h0});
 		if (h0 < np) tiles.push_back({0, t, h0, np - h0});
 	}
+	std::vector<TcTile> xt[2];
+	if (which == 2) {
+		tcx_tiles(0, np, [&](int cls, const TcTile &tl) { xt[cls].push_back(tl); });
+		tiles = xt[0];
+		tiles.insert(tiles.end(), xt[1].begin(), xt[1].end());
+	}
 	std::vector<int32_t> hs((size_t)n);
 	for (int i = 0; i < n; i++) hs[i] = i;
 	cudaStream_t st = 0;
@@ -3754,7 +3769,6 @@ int ha_b200_tc_selftest(int32_t which, int32_t n, int32_t nt, const float *h_a, 
 		a.Xp = Xp.p;
 		a.Xw = Xp.p;
 		a.Pp = Pp.p;
-		a.A32 = A32.p;
 		a.T = T.p;
 		a.t_rowmajor = 1;
 		a.st_in = dst.p;
@@ -3778,8 +3792,9 @@ int ha_b200_tc_selftest(int32_t which, int32_t n, int32_t nt, const float *h_a, 
 			}
 			k_split3_vertex_major<<<64, kBlock, 0, st>>>(d0.p, nt, n, ntp, Xb.p);
 			k_split3_vertex_major<<<64, kBlock, 0, st>>>(d1.p, nt, n, ntp, Yb.p);
-			a.Xb = Xb.p; a.Yb = Yb.p; a.vplane = vplane; a.ntp = ntp; a.sl_idx = sl.p;
-			{ HA_LAUNCH(kHaB200KTcXcov, st); k_tc_gemm<kTcPhaseXcov><<<grid, kTcThreads, a.smem_bytes, st>>>(a); }
+			const TcXArgs x = {dw.p, nullptr, Xb.p, Yb.p, vplane, ntp, sl.p, A32.p, 0, err.p};
+			launch_tc_xcov(dt.p, (int)xt[0].size(), 0, x, st);
+			launch_tc_xcov(dt.p + xt[0].size(), (int)xt[1].size(), 1, x, st);
 			std::vector<float> full((size_t)np * np);
 			if (cudaGetLastError() != cudaSuccess ||
 			    cudaMemcpy(full.data(), A32.p, full.size() * 4, cudaMemcpyDeviceToHost) != cudaSuccess) {

@@ -96,18 +96,10 @@ struct TcState {
 struct TcArgs {
 	const TcWork *work;
 	const TcTile *tiles;
-	// cross-covariance: vertex-major bf16 planes [plane][nv][ntp], ntp = nt rounded up to 16
-	const __nv_bfloat16 *Xb;
-	const __nv_bfloat16 *Yb;
-	int64_t vplane;  // elements per vertex-major plane (nv * ntp)
-	int ntp;
-	const int32_t *sl_idx;
-	// Newton-Schulz
 	__nv_bfloat16 *Xp;  // iterate planes (offsets from TcWork::xofs), read
 	__nv_bfloat16 *Xw;  // where the update writes the next iterate: the other of two buffers, since the
 	                    // two column halves of a row tile both read the whole row tile of X
 	__nv_bfloat16 *Pp;  // P planes (TcWork::pofs)
-	float *A32;         // cross-covariance (TcWork::aofs)
 	float *T;           // T scratch (TcWork::tofs)
 	int t_rowmajor;
 	const TcState *st_in;
@@ -463,21 +455,19 @@ __device__ __forceinline__ void tc_issue_products(uint32_t tmem, uint32_t st, in
 // ---------------------------------------------------------------------------------------------
 // the tile-product kernel
 // ---------------------------------------------------------------------------------------------
-// PHASE kTcPhaseXcov:   A32 = X_sl^T Y_sl                       (K = time, padded to 16)
 // PHASE kTcPhaseGram:   P = c1 I + c3 X^T X, residual partials   (skips searchlights already done)
 // PHASE kTcPhaseUpdate: X <- X P, or T = X P for the final update (decided from the residual)
 // BULK (Gram and update only): warp-specialised stages filled by bulk copies instead of the
 // per-thread loads (see the main loop).
 template <int PHASE, bool BULK = false>
 __global__ void __launch_bounds__(kTcThreads) k_tc_gemm(const TcArgs a) {
-	static_assert(!(BULK && PHASE == kTcPhaseXcov), "the gathered cross-covariance has no bulk form");
+	static_assert(PHASE != kTcPhaseXcov, "the cross-covariance has its own kernel");
 	extern __shared__ __align__(128) unsigned char tc_smem[];
 	__shared__ uint64_t s_bar[kTcMaxStages];   // stage consumed: the stage's products completed
 	__shared__ uint64_t s_full[kTcMaxStages];  // stage filled (bulk form): its copies landed
 	__shared__ uint64_t s_acc;
 	__shared__ uint32_t s_tmem;
 	__shared__ int s_fail;
-	__shared__ int32_t s_sl[PHASE == kTcPhaseXcov ? kTcMaxNp : 1];
 
 	const TcTile tl = a.tiles[blockIdx.x];
 	const TcWork w = a.work[tl.w];
@@ -491,7 +481,7 @@ __global__ void __launch_bounds__(kTcThreads) k_tc_gemm(const TcArgs a) {
 
 	const float c1 = a.c1, c3 = a.c3;
 	bool final_update = false;
-	if (PHASE != kTcPhaseXcov) {
+	{
 		const TcState st = a.st_in[w.slot];
 		if (st.done) {
 			if (PHASE == kTcPhaseUpdate && t == 0 && tid == 0) a.st_out[w.slot] = st;
@@ -528,7 +518,7 @@ __global__ void __launch_bounds__(kTcThreads) k_tc_gemm(const TcArgs a) {
 	const int stage_bytes = tc_stage_bytes(N, NPL);
 	int S = a.smem_bytes / stage_bytes;
 	if (S > kTcMaxStages) S = kTcMaxStages;
-	const int nk = (PHASE == kTcPhaseXcov) ? (a.ntp >> 4) : (np >> 4);
+	const int nk = np >> 4;
 	const uint32_t ncols = tc_tmem_cols(N);
 	const uint32_t smem0 = smem_u32(tc_smem);
 
@@ -543,8 +533,6 @@ __global__ void __launch_bounds__(kTcThreads) k_tc_gemm(const TcArgs a) {
 		s_fail = (S < 2) ? 1 : 0;
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
-	if (PHASE == kTcPhaseXcov)
-		for (int i = tid; i < n; i += kTcThreads) s_sl[i] = a.sl_idx[w.sofs + i];
 	if (BULK && gA < 16 && S <= kTcMaxStages) {
 		// the copies fill only the A rows inside the searchlight: zero every stage's A planes once
 		for (int st = 0; st < S; st++)
@@ -562,21 +550,17 @@ __global__ void __launch_bounds__(kTcThreads) k_tc_gemm(const TcArgs a) {
 	const __nv_bfloat16 *Xs = a.Xp + w.xofs;
 	const __nv_bfloat16 *Bs = (PHASE == kTcPhaseGram) ? Xs : (const __nv_bfloat16 *)(a.Pp + w.pofs);
 	TcLoadPlan lp;
-	tc_plan_tile<PHASE>(lp, s_sl, n, np, a.ntp, t, n0, N);
-	const __nv_bfloat16 *srcA = (PHASE == kTcPhaseXcov) ? a.Xb : Xs;
-	const __nv_bfloat16 *srcB = (PHASE == kTcPhaseXcov) ? a.Yb : Bs;
-	const int64_t pstride = (PHASE == kTcPhaseXcov) ? a.vplane : (int64_t)np * np;
+	tc_plan_tile<PHASE>(lp, nullptr, n, np, 0, t, n0, N);
+	const int64_t pstride = (int64_t)np * np;
 	auto load = [&](int ks, int s) {
-		tc_load_slice<NPL>(lp, srcA, pstride, srcB, pstride, N, ks, smem0 + s * stage_bytes);
+		tc_load_slice<NPL>(lp, Xs, pstride, Bs, pstride, N, ks, smem0 + s * stage_bytes);
 	};
 
-	// operand majors: cross-covariance K/K, Gram MN/MN, update K/MN
+	// operand majors: Gram MN/MN, update K/MN
 	const int a_mn = (PHASE == kTcPhaseGram) ? 1 : 0;
-	const int b_mn = (PHASE == kTcPhaseXcov) ? 0 : 1;
 	const int N0 = N > 256 ? 256 : N;
-	const bool f16 = PHASE != kTcPhaseXcov;
-	const uint32_t id0 = mma_idesc(128, N0, a_mn, b_mn, f16);
-	const uint32_t id1 = N > 256 ? mma_idesc(128, N - 256, a_mn, b_mn, f16) : 0u;
+	const uint32_t id0 = mma_idesc(128, N0, a_mn, 1, true);
+	const uint32_t id1 = N > 256 ? mma_idesc(128, N - 256, a_mn, 1, true) : 0u;
 
 	if (BULK && !failed) {
 		// Warp 0 fills stage ks % S with bulk copies (their bytes complete the stage's full barrier)
@@ -606,7 +590,7 @@ __global__ void __launch_bounds__(kTcThreads) k_tc_gemm(const TcArgs a) {
 				if (!__shfl_sync(0xffffffffu, ok, 0)) break;
 				const uint32_t st = smem0 + s * stage_bytes;
 				const int p = lane >> 4, q = lane & 15;  // A part: plane p, core group q (update) or K half q (Gram)
-				const __nv_bfloat16 *Ap = srcA + p * pe;
+				const __nv_bfloat16 *Ap = Xs + p * pe;
 				const uint32_t sa = st + p * 4096;
 				if (PHASE == kTcPhaseGram) {
 					if (q < 2)
@@ -617,7 +601,7 @@ __global__ void __launch_bounds__(kTcThreads) k_tc_gemm(const TcArgs a) {
 				if (lane < 4) {  // B part: plane lane >> 1, K half lane & 1
 					const int pb = lane >> 1, k = lane & 1;
 					bulk_g2s(st + 2 * 4096 + pb * 32 * N + k * 16 * N,
-					         srcB + pb * pe + ((int64_t)(2 * ks + k) * npg + g0) * 64, 16u * N, &s_full[s]);
+					         Bs + pb * pe + ((int64_t)(2 * ks + k) * npg + g0) * 64, 16u * N, &s_full[s]);
 				}
 				issued = ks + 1;
 			}
@@ -694,17 +678,9 @@ __global__ void __launch_bounds__(kTcThreads) k_tc_gemm(const TcArgs a) {
 			float v[16];
 			tmem_ld16(trow + (uint32_t)c0, v);
 			if (row >= np) continue;
-			if (PHASE != kTcPhaseXcov) {
 #pragma unroll
-				for (int q = 0; q < 16; q++) v[q] *= kTcAccUnscale;
-			}
-			if (PHASE == kTcPhaseXcov) {
-				if (row < n) {
-					float4 *dst = reinterpret_cast<float4 *>(a.A32 + w.aofs + (int64_t)row * np + n0 + c0);
-#pragma unroll
-					for (int q = 0; q < 4; q++) dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-				}
-			} else if (PHASE == kTcPhaseGram) {
+			for (int q = 0; q < 16; q++) v[q] *= kTcAccUnscale;
+			if (PHASE == kTcPhaseGram) {
 #pragma unroll
 				for (int q = 0; q < 16; q++) {
 					const int col = n0 + c0 + q;

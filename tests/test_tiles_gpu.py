@@ -171,3 +171,21 @@ def test_resident_iteration_bitwise_equal(gpu, tmp_path):
         res.append(np.load(path))
     for k in res[0].files:
         assert res[0][k].tobytes() == res[1][k].tobytes(), k
+
+
+# The three-part split is exact to 2^-24 and the FP32 accumulator takes 6 nt / 16 additions: for nt <= 260
+# a relative error of 2^-24 sqrt(6 * 260 / 16) * O(1) in the 2-norm, 5e-6 with a factor of eight to spare.
+@pytest.mark.parametrize("nt", [1, 31, 32, 33, 65, 260])
+def test_cross_covariance_tile_edges(gpu, hlib, nt):
+    """Both size classes, one and two row tiles per block, one and two row blocks, short last stages."""
+    rng = np.random.default_rng(nt)
+    fp = L.c_float_p
+    for n in [1, 2, 16, 17, 63, 80, 96, 97, 127, 128, 129, 144, 192, 193, 255, 256, 257, 288, 384, 385, 496, 512]:
+        A = rng.standard_normal((n, nt)).astype(np.float32)
+        B = rng.standard_normal((n, nt)).astype(np.float32)
+        out = np.zeros((n, n), dtype=np.float32)
+        assert hlib.ha_b200_tc_selftest(2, n, nt, A.ctypes.data_as(fp), B.ctypes.data_as(fp), out.ctypes.data_as(fp)) == 0
+        ref = A.astype(np.float64) @ B.astype(np.float64).T
+        # a product of few samples can cancel: bounded against the factors instead of the result
+        scale = np.linalg.norm(A, axis=1)[:, None] * np.linalg.norm(B, axis=1)[None, :]
+        assert (np.abs(out - ref) <= 5e-6 * scale).all(), n
