@@ -2647,11 +2647,10 @@ int host_threads() {
 	return std::max(1, t);
 }
 
-// Cached plan for the host entry points (geometry + weights identify it). The hash only
-// screens; a hit is confirmed against the full key, so a collision rebuilds instead of reusing.
+// Cached plan for the host entry points: the geometry and weights identify it, compared in full (a
+// comparison of a plan's few megabytes takes 0.1 ms where a byte-wise hash of them took 3).
 HaB200Plan *g_cached_plan = nullptr;
 int g_cached_dev = -1;  // device the cached plan and the host-call buffers live on
-uint64_t g_cached_key = 0;
 int g_cached_mode = 0;
 double g_cached_radius = 0.0;
 std::vector<double> g_cached_aux;  // the dists or weights the cached plan was built from
@@ -2673,16 +2672,7 @@ int get_plan(int32_t nt, int32_t nv, const int32_t *idx, const int32_t *off, con
              double radius, const double *weights, bool unweighted, HaB200Plan **out) {
 	if (!idx || !off || count <= 0) return kHaErrorArg;
 	if (off[count] < 0) return kHaErrorArg;
-	uint64_t h = 1469598103934665603ULL;
-	int32_t hdr[3] = {nt, nv, count};
-	h = fnv1a(hdr, sizeof(hdr), h);
-	h = fnv1a(&radius, sizeof(radius), h);
-	h = fnv1a(off, ((size_t)count + 1) * 4, h);
-	h = fnv1a(idx, (size_t)off[count] * 4, h);
-	int mode = dists ? 1 : weights ? 2 : unweighted ? 3 : 0;
-	h = fnv1a(&mode, sizeof(mode), h);
-	if (dists) h = fnv1a(dists, (size_t)off[count] * 8, h);
-	if (weights) h = fnv1a(weights, (size_t)off[count] * 8, h);
+	const int mode = dists ? 1 : weights ? 2 : unweighted ? 3 : 0;
 	const double *aux = weights ? weights : dists;  // weights override dists in plan_create_impl
 	int dev = 0;
 	if (cudaGetDevice(&dev) != cudaSuccess) return kHaErrorInternal;
@@ -2696,8 +2686,7 @@ int get_plan(int32_t nt, int32_t nv, const int32_t *idx, const int32_t *off, con
 		g_cached_plan = nullptr;
 		if (cudaSetDevice(dev) != cudaSuccess) return kHaErrorInternal;
 	}
-	if (g_cached_plan && g_cached_key == h &&
-	    cached_plan_matches(nt, nv, idx, off, count, radius, mode, aux)) {
+	if (g_cached_plan && cached_plan_matches(nt, nv, idx, off, count, radius, mode, aux)) {
 		*out = g_cached_plan;
 		return kHaSuccess;
 	}
@@ -2709,7 +2698,6 @@ int get_plan(int32_t nt, int32_t nv, const int32_t *idx, const int32_t *off, con
 	if (rc != kHaSuccess) return rc;
 	g_cached_plan = *out;
 	g_cached_dev = dev;
-	g_cached_key = h;
 	g_cached_mode = mode;
 	g_cached_radius = radius;
 	if (aux) g_cached_aux.assign(aux, aux + off[count]);

@@ -28,8 +28,8 @@ def _flatten(sls, dists):
     sizes = np.array([len(s) for s in sls], dtype=np.int32)
     offsets = np.zeros(len(sls) + 1, dtype=np.int32)
     np.cumsum(sizes, out=offsets[1:])
-    idx = np.ascontiguousarray(np.concatenate(sls).astype(np.int32))
-    d = None if dists is None else np.ascontiguousarray(np.concatenate(dists).astype(np.float64))
+    idx = np.ascontiguousarray(np.concatenate(sls).astype(np.int32, copy=False))
+    d = None if dists is None else np.ascontiguousarray(np.concatenate(dists).astype(np.float64, copy=False))
     if d is not None and d.size != idx.size:
         raise ValueError("dists must hold one distance per searchlight member")
     return idx, offsets, d
