@@ -17,6 +17,7 @@
 #include "ha_b200_tc.cuh"
 #include "ha_b200_tcres.cuh"
 #include "ha_b200_tcxcov.cuh"
+#include "ha_b200_tcwide.cuh"
 #include "ha_b200_pca.cuh"
 
 #include <cuda_runtime.h>
@@ -319,6 +320,8 @@ struct Chunk {
 	std::vector<TcTile> tct[2];
 	TcWork *d_tcw = nullptr;
 	TcTile *d_tct[2] = {nullptr, nullptr};
+	std::vector<TcTile> tcw_t;  // the wide iteration's tiles (tcw_tiles)
+	TcTile *d_tcw_t = nullptr;
 	std::vector<TcTile> tcx[2];  // the cross-covariance's tiles (tcx_tiles)
 	TcTile *d_tcx[2] = {nullptr, nullptr};
 	std::vector<int32_t> tco[2];  // persistent solve: work indices per size class, largest first
@@ -1021,6 +1024,8 @@ int set_tc_attrs() {
 	HA_CUDA(cudaFuncSetAttribute((k_tc_resident<1, 3>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_resident_smem(128, 1)));
 	HA_CUDA(cudaFuncSetAttribute((k_tc_resident<1, 2>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_resident_smem(64, 1)));
 	HA_CUDA(cudaFuncSetAttribute((k_tc_resident<2, 4>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_resident_smem(kTcResMaxNp, 2)));
+	HA_CUDA(cudaFuncSetAttribute(k_tc_wide<kTcPhaseGram>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcWSmem));
+	HA_CUDA(cudaFuncSetAttribute(k_tc_wide<kTcPhaseUpdate>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcWSmem));
 	HA_CUDA(cudaFuncSetAttribute(k_tc_xcov, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcXSmem[1]));
 	HA_CUDA(cudaFuncSetAttribute(k_tc_gemm<kTcPhaseGram>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemLarge));
 	HA_CUDA(cudaFuncSetAttribute(k_tc_gemm<kTcPhaseUpdate>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemLarge));
@@ -1076,6 +1081,7 @@ int build_tc(HaB200Plan *P) {
 			ch.tcx[c].clear();
 		}
 		for (auto &r : ch.tcr) r.clear();
+		ch.tcw_t.clear();
 		for (int q : order) {
 			const int np = ch.tcw[q].np;
 			const int c = np > 256 ? 1 : 0;
@@ -1090,6 +1096,8 @@ int build_tc(HaB200Plan *P) {
 			ch.tco[c].push_back(q);
 			if (tc_resident() && np <= kTcResMaxNp) {
 				ch.tcr[np > 128 ? 0 : np > 64 ? 1 : 2].push_back(q);
+			} else if (tc_resident()) {
+				tcw_tiles(q, np, [&](const TcTile &tl) { ch.tcw_t.push_back(tl); });
 			} else {
 				for (int t = 0; t * 128 < np; t++) {
 					ch.tcl[h0 <= 128 ? 0 : 1].push_back({q, t, 0, h0});
@@ -1114,6 +1122,7 @@ int build_tc(HaB200Plan *P) {
 			add(ch.tcx[c], &ch.d_tcx[c]);
 		}
 		for (int r = 0; r < 3; r++) add(ch.tcr[r], &ch.d_tcr[r]);
+		add(ch.tcw_t, &ch.d_tcw_t);
 		if (cudaMalloc(&ch.d_tclists, blob.size()) != cudaSuccess) return kHaErrorAlloc;
 		for (auto &x : at) *x.first = ch.d_tclists + x.second;
 		HA_CUDA(cudaMemcpy(ch.d_tclists, blob.data(), blob.size(), cudaMemcpyHostToDevice));
@@ -1192,6 +1201,16 @@ void launch_tc_tiles(int ntiles, TcArgs a, cudaStream_t st, int nmax, bool persi
 		k_tc_gemm<PHASE, true><<<ntiles, kTcThreads, a.smem_bytes, st>>>(a);
 	else
 		k_tc_gemm<PHASE><<<ntiles, kTcThreads, a.smem_bytes, st>>>(a);
+}
+
+template <int PHASE>
+void launch_tc_wide(const Chunk &ch, TcArgs a, cudaStream_t st) {
+	const int n = (int)ch.tcw_t.size();
+	if (!n) return;
+	a.tiles = ch.d_tcw_t;
+	const int grid = std::min(n, std::max(g_num_sms, (n + kTcWMaxTiles - 1) / kTcWMaxTiles));
+	HA_LAUNCH(kHaB200KTcNs, st);
+	k_tc_wide<PHASE><<<grid, kTcWThreads<PHASE>, kTcWSmem, st>>>(a, n);
 }
 
 void launch_tc_xcov(const TcTile *tiles, int ntiles, int cls, TcXArgs x, cudaStream_t st) {
@@ -1376,6 +1395,8 @@ int run_procrustes_tc(HaB200Plan *P, const double *d_X, const double *d_Y, bool 
 				a.c3 = sched[k].c3;
 				a.plain = sched[k].plain;
 				a.last = (k == maxit - 1) ? 1 : 0;
+				launch_tc_wide<kTcPhaseGram>(ch, a, ls);
+				launch_tc_wide<kTcPhaseUpdate>(ch, a, ls);
 				const bool persist = k >= tc_iter_from();
 				int r = launch_tc<kTcPhaseGram>(ch, a, ls, kHaB200KTcNs, P->tc_smem, -1, persist, true);
 				if (r != kHaSuccess) return r;
@@ -1421,7 +1442,7 @@ int run_procrustes_tc(HaB200Plan *P, const double *d_X, const double *d_Y, bool 
 			                              : cudaLaunchKernelEx(&cfg, k_tc_resident<1, 2>, ra);
 			HA_CUDA(le);
 		}
-		if (ch.tcl[0].empty() && ch.tcl[1].empty()) {
+		if (ch.tcw_t.empty() && ch.tcl[0].empty() && ch.tcl[1].empty()) {
 			// nothing is left to the per-phase iteration
 		} else if (!graphs_enabled() || g_timing) {
 			if ((rc = enqueue_loop(st)) != kHaSuccess) return rc;

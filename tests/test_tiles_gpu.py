@@ -189,3 +189,23 @@ def test_cross_covariance_tile_edges(gpu, hlib, nt):
         # a product of few samples can cancel: bounded against the factors instead of the result
         scale = np.linalg.norm(A, axis=1)[:, None] * np.linalg.norm(B, axis=1)[None, :]
         assert (np.abs(out - ref) <= 5e-6 * scale).all(), n
+
+
+def test_wide_iteration_bitwise_equal(gpu, tmp_path):
+    """The 256-row tiles of the iteration past 256 vertices against the 128-row kernels: identical bits where
+    the second row block and the column halves are one step wide, odd, or full, and K ends in half a stage."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    script = _RESIDENT_SCRIPT.replace(
+        _RESIDENT_SCRIPT[_RESIDENT_SCRIPT.index("sizes = "):_RESIDENT_SCRIPT.index("X = rng")],
+        "sizes = [200, 257, 271, 272, 273, 288, 320, 351, 384, 385, 400, 449, 496, 511, 512]\nnv, nt = 512, 600\n")
+    res = []
+    for v in "01":
+        path = tmp_path / f"w{v}.npz"
+        subprocess.run([sys.executable, "-c", script, root, str(path)],
+                       env=dict(os.environ, HA_B200_TC_RESIDENT=v), check=True, timeout=300)
+        res.append(np.load(path))
+    for k in res[0].files:
+        assert res[0][k].tobytes() == res[1][k].tobytes(), k
