@@ -1398,7 +1398,8 @@ __global__ void k_split3_vertex_major(const double *__restrict__ X, int nt, int 
 
 // X_0 = A / u with u = min(||A||_F, sqrt(||A||_1 ||A||_inf)) >= sigma_max(A), written as the two
 // core-tiled FP16 planes of the iteration (np x np, padding zero); iteration state and residual
-// slots cleared.
+// slots cleared.  Bound by memory: A is read once for the norms (rows and columns together, in the
+// order of two separate passes) and once for the planes.
 __global__ void __launch_bounds__(256) k_tc_ns_init(const TcWork *__restrict__ work, const float *__restrict__ A32,
                                                     __nv_bfloat16 *__restrict__ Xp, TcState *__restrict__ st,
                                                     float *__restrict__ res_part) {
@@ -1408,23 +1409,48 @@ __global__ void __launch_bounds__(256) k_tc_ns_init(const TcWork *__restrict__ w
 	__shared__ double s_red[2][8];
 	__shared__ float s_colsum[kTcMaxNp];
 	__shared__ float s_u;
+	__shared__ __align__(16) float s_rows[2][8][kTcMaxNp];
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	// eight rows at a time: a warp sums its row while every thread adds its columns in row order
 	double fro = 0.0, rowmax = 0.0;
-	for (int r = warp; r < n; r += 8) {
-		double rs = 0.0;
-		for (int c = lane; c < n; c += 32) {
-			const double x = A[(int64_t)r * np + c];
-			fro += x * x;
-			rs += fabs(x);
+	float cs[kTcMaxNp / 256] = {};
+	const int q4 = np >> 2;
+	auto fetch = [&](int r0, int buf) {
+		for (int e = threadIdx.x; e < 8 * q4; e += 256) {
+			const int r = e / q4, c = 4 * (e - r * q4);
+			if (r0 + r < n) cp_async16(smem_u32(&s_rows[buf][r][c]), A + (int64_t)(r0 + r) * np + c, 16u);
 		}
-		rs = warp_sum(rs);
-		rowmax = fmax(rowmax, rs);
+		cp_async_commit();
+	};
+	fetch(0, 0);
+	for (int r0 = 0, buf = 0; r0 < n; r0 += 8, buf ^= 1) {
+		if (r0 + 8 < n) {
+			fetch(r0 + 8, buf ^ 1);
+			cp_async_wait_keep(1);
+		} else {
+			cp_async_wait_keep(0);
+		}
+		__syncthreads();
+		if (r0 + warp < n) {
+			double rs = 0.0;
+			for (int c = lane; c < n; c += 32) {
+				const double x = s_rows[buf][warp][c];
+				fro += x * x;
+				rs += fabs(x);
+			}
+			rowmax = fmax(rowmax, warp_sum(rs));
+		}
+#pragma unroll
+		for (int k = 0; k < kTcMaxNp / 256; k++) {
+			const int c = threadIdx.x + 256 * k;
+			if (c < n)
+				for (int i = 0; i < 8 && r0 + i < n; i++) cs[k] += fabsf(s_rows[buf][i][c]);
+		}
+		__syncthreads();
 	}
-	for (int c = threadIdx.x; c < n; c += blockDim.x) {
-		float cs = 0.f;
-		for (int r = 0; r < n; r++) cs += fabsf(A[(int64_t)r * np + c]);
-		s_colsum[c] = cs;
-	}
+#pragma unroll
+	for (int k = 0; k < kTcMaxNp / 256; k++)
+		if ((int)threadIdx.x + 256 * k < n) s_colsum[threadIdx.x + 256 * k] = cs[k];
 	fro = warp_sum(fro);
 	if (lane == 0) { s_red[0][warp] = fro; s_red[1][warp] = rowmax; }
 	__syncthreads();
@@ -1444,17 +1470,18 @@ __global__ void __launch_bounds__(256) k_tc_ns_init(const TcWork *__restrict__ w
 	const float inv = 1.f / s_u;
 	const int64_t pe = (int64_t)np * np;
 	__nv_bfloat16 *X0 = Xp + w.xofs;
-	// one thread per core-matrix row (8 elements)
-	const int64_t chunks = (int64_t)np * npg;
-	for (int64_t e = threadIdx.x; e < chunks; e += blockDim.x) {
-		const int row = (int)(e / npg), cg = (int)(e - (int64_t)row * npg);
-		float v[8];
+	// one thread per core-matrix row (8 elements), the eight rows of a core side by side: 128 bytes stored
+	for (int e = threadIdx.x; e < np * npg; e += 256) {
+		const int core = e >> 3, rg = core / npg, cg = core - rg * npg, row = 8 * rg + (e & 7);
+		float v[8] = {};
+		if (row < n) {
+			const float4 *src = reinterpret_cast<const float4 *>(A + (int64_t)row * np + 8 * cg);
+			const float4 x = src[0], y = src[1];
+			const float f[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
 #pragma unroll
-		for (int q = 0; q < 8; q++) {
-			const int col = 8 * cg + q;
-			v[q] = (row < n && col < n) ? A[(int64_t)row * np + col] * inv : 0.f;
+			for (int q = 0; q < 8; q++) v[q] = 8 * cg + q < n ? f[q] * inv : 0.f;
 		}
-		const int64_t o = ((int64_t)(row >> 3) * npg + cg) * 64 + (row & 7) * 8;
+		const int64_t o = (int64_t)core * 64 + (row & 7) * 8;
 		store_split8h(v, X0 + o, X0 + pe + o);
 	}
 }
@@ -1470,11 +1497,22 @@ __global__ void __launch_bounds__(256) k_tc_ns_finish(const TcWork *__restrict__
 	const int n = w.n, np = w.np;
 	const float *A = A32 + w.aofs;
 	const float *T = Tscr + w.tofs;
+	// the products of elements tid, tid + 256, ... in that order, their loads eight at a time
 	double s = 0.0;
-	for (int64_t e = threadIdx.x; e < (int64_t)n * n; e += blockDim.x) {
-		const int r = (int)(e / n), c = (int)(e - (int64_t)r * n);
-		const float tv = t_rowmajor ? T[(int64_t)r * n + c] : T[(int64_t)c * n + r];
-		s += (double)tv * (double)A[(int64_t)r * np + c];
+	int r = (int)threadIdx.x / n, c = (int)threadIdx.x - r * n;
+	while (r < n) {
+		float tv[8], av[8];
+#pragma unroll
+		for (int k = 0; k < 8; k++) {
+			tv[k] = av[k] = 0.f;
+			if (r < n) {
+				tv[k] = t_rowmajor ? T[(int64_t)r * n + c] : T[(int64_t)c * n + r];
+				av[k] = A[(int64_t)r * np + c];
+				for (c += 256; c >= n; c -= n) r++;
+			}
+		}
+#pragma unroll
+		for (int k = 0; k < 8; k++) s += (double)tv[k] * (double)av[k];
 	}
 	s = warp_sum(s);
 	__shared__ double red[8];
