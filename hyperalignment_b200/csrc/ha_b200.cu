@@ -1329,7 +1329,7 @@ int run_procrustes_tc(HaB200Plan *P, const double *d_X, const double *d_Y, bool 
 	{ HA_LAUNCH(kHaB200KConvert, st); k_split3_vertex_major<<<148 * 8, kBlock, 0, st>>>(d_Y, nt, nv, ntp, P->tcYb.p); }
 	if (scal) {
 		if ((rc = P->var.ensure((size_t)nv)) != kHaSuccess) return rc;
-		{ HA_LAUNCH(kHaB200KColVar, st); k_col_var_over_nt<<<(nv + 127) / 128, 128, 0, st>>>(d_X, nt, nv, P->var.p); }
+		{ HA_LAUNCH(kHaB200KColVar, st); k_col_var_over_nt<<<(nv + kScanCols - 1) / kScanCols, 256, 0, st>>>(d_X, nt, nv, P->var.p); }
 	}
 	HA_CUDA(cudaMemsetAsync(P->counters.p, 0, 5 * sizeof(int32_t), st));
 	static const std::vector<NsStep> sched = ns_schedule();
@@ -1554,7 +1554,7 @@ int run_procrustes(HaB200Plan *P, const double *d_X, const double *d_Y, bool ref
 	}
 	if (scal) {
 		if ((rc = P->var.ensure((size_t)nv)) != kHaSuccess) return rc;
-		{ HA_LAUNCH(kHaB200KColVar, st); k_col_var_over_nt<<<(nv + 127) / 128, 128, 0, st>>>(d_X, nt, nv, P->var.p); }
+		{ HA_LAUNCH(kHaB200KColVar, st); k_col_var_over_nt<<<(nv + kScanCols - 1) / kScanCols, 256, 0, st>>>(d_X, nt, nv, P->var.p); }
 	}
 	HA_CUDA(cudaMemsetAsync(P->counters.p, 0, 5 * sizeof(int32_t), st));
 	float *T = P->scrT.p;
@@ -2910,7 +2910,7 @@ int template_impl(const double *dms, int ns, int nt, int nv, const int32_t *idx,
 	cudaStream_t st = 0;
 	if (cudaMemcpyAsync(D.p, dms, m * ns * 8, cudaMemcpyHostToDevice, st) != cudaSuccess) return done(kHaErrorInternal);
 	const int eg = 148 * 8;
-	const int zg = (nv + 127) / 128;
+	const int zg = (nv + kScanCols - 1) / kScanCols;
 	// aligned_s = X_s @ SL(X_s -> target)
 	auto align = [&](int s, const double *target) -> int {
 		if (cudaMemsetAsync(vals.p, 0, (size_t)P->nnz * 8, st) != cudaSuccess) return kHaErrorInternal;
@@ -2924,9 +2924,9 @@ int template_impl(const double *dms, int ns, int nt, int nv, const int32_t *idx,
 		return done(kHaErrorInternal);
 	for (int s = 1; s < ns; s++) {
 		if ((rc = align(s, common.p)) != kHaSuccess) return done(rc);
-		if (zs) k_zscore_cols<<<zg, 128, 0, st>>>(A.p + m * s, nt, nv);
+		if (zs) k_zscore_cols<<<zg, 256, 0, st>>>(A.p + m * s, nt, nv);
 		k_axpbz<<<eg, 256, 0, st>>>(common.p, common.p, A.p + m * s, 0.5, 1.0, (int64_t)m);
-		if (zs) k_zscore_cols<<<zg, 128, 0, st>>>(common.p, nt, nv);
+		if (zs) k_zscore_cols<<<zg, 256, 0, st>>>(common.p, nt, nv);
 	}
 	for (int it = 0; it < level2; it++) {
 		// common = sum over subjects (in subject order)
@@ -2934,14 +2934,14 @@ int template_impl(const double *dms, int ns, int nt, int nv, const int32_t *idx,
 		for (int s = 1; s < ns; s++) k_axpbz<<<eg, 256, 0, st>>>(common.p, common.p, A.p + m * s, 1.0, 1.0, (int64_t)m);
 		for (int s = 0; s < ns; s++) {
 			k_axpbz<<<eg, 256, 0, st>>>(ref.p, common.p, A.p + m * s, 1.0 / (ns - 1), -1.0, (int64_t)m);
-			if (zs) k_zscore_cols<<<zg, 128, 0, st>>>(ref.p, nt, nv);
+			if (zs) k_zscore_cols<<<zg, 256, 0, st>>>(ref.p, nt, nv);
 			if ((rc = align(s, ref.p)) != kHaSuccess) return done(rc);
 		}
 	}
 	k_axpbz<<<eg, 256, 0, st>>>(common.p, A.p, nullptr, 1.0, 0.0, (int64_t)m);
 	for (int s = 1; s < ns; s++) k_axpbz<<<eg, 256, 0, st>>>(common.p, common.p, A.p + m * s, 1.0, 1.0, (int64_t)m);
 	if (zs)
-		k_zscore_cols<<<zg, 128, 0, st>>>(common.p, nt, nv);
+		k_zscore_cols<<<zg, 256, 0, st>>>(common.p, nt, nv);
 	else
 		k_axpbz<<<eg, 256, 0, st>>>(common.p, common.p, nullptr, 1.0 / ns, 0.0, (int64_t)m);
 	if (cudaGetLastError() != cudaSuccess ||

@@ -209,3 +209,21 @@ def test_wide_iteration_bitwise_equal(gpu, tmp_path):
         res.append(np.load(path))
     for k in res[0].files:
         assert res[0][k].tobytes() == res[1][k].tobytes(), k
+
+
+@pytest.mark.parametrize("nv,nt", [(1, 2), (15, 127), (16, 128), (17, 129), (33, 257), (162, 40)])
+def test_template_column_edges(gpu, nv, nt):
+    """Column statistics and the product with the transform at the edges of their tiles (16 columns, 128
+    samples; four entries, 384 samples): the template against the oracle, which sums in the same order.  The
+    transforms come from FP32 products of well-conditioned Gaussian series: 1e-5 of the template's norm."""
+    from hyperalignment_b200 import hyperalignment_c as H
+    rng = np.random.default_rng(100 * nv + nt)
+    base = rng.standard_normal((nt, nv))
+    dms = [base + 0.5 * rng.standard_normal((nt, nv)) for _ in range(2)]
+    n = min(nv, max(1, nt // 4), 12)
+    sls = [np.sort((c + np.arange(n)) % nv).astype(np.int32) for c in range(nv)]
+    dists = [np.linspace(0.0, 0.5, n) for _ in range(nv)]
+    idx, off = np.concatenate(sls), np.concatenate([[0], np.cumsum([n] * nv)]).astype(np.int32)
+    out = H.searchlight_template(dms, sls, dists, 1.0, True, True, True, 1)
+    ref = O.searchlight_template(dms, idx, off, np.concatenate(dists), 1.0, True, True, True, 1)
+    assert np.linalg.norm(out - ref) <= 1e-5 * np.linalg.norm(ref)
