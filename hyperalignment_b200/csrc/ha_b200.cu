@@ -1961,8 +1961,8 @@ int grid_chunk_launch(HaB200Plan *P, Chunk &ch, const double *d_X, const double 
 				const cudaStream_t bs = g_fan.at((int)bi);
 				const SlWork *wk = d_work + x0;
 				// Gram into the V scratch, its pivoted Cholesky factor into the A scratch
-				{ HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<16, Real><<<x1 - x0, kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_X, nt, tr, md.tr_n, V, G, gp, 0); }
-				{ HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<16, Real><<<x1 - x0, kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_Y, nt, tr, md.tr_n, A, G, gp, 1); }
+				{ HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<Real><<<dim3(x1 - x0, xrows_tiles(32 * b.rpl, 0)), kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_X, nt, tr, md.tr_n, V, G, gp, 0); }
+				{ HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<Real><<<dim3(x1 - x0, xrows_tiles(32 * b.rpl, 1)), kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_Y, nt, tr, md.tr_n, A, G, gp, 1); }
 				{ HA_LAUNCH(kHaB200KRidge, bs); k_pchol<Real><<<x1 - x0, kBlock, pchol_smem(b.rpl), bs>>>(wk, V, A, P->stats.p); }
 				{
 					HA_LAUNCH(kHaB200KJacobi32, bs);
@@ -2413,8 +2413,8 @@ int eigen_chunk32(HaB200Plan *P, Chunk &ch, const double *d_X, const double *d_Y
 		const Bucket &b = ch.beig32[bi];
 		const cudaStream_t bs = g_fan.at((int)bi);
 		const SlWork *wk = ch.d_weig32 + b.first;
-		{ HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<16, float><<<b.count, kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_X, P->nt, d_rows, n_rows, V, nullptr, gp, 0); }
-		if (d_Y) { HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<16, float><<<b.count, kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_Y, P->nt, d_rows, n_rows, P->scrT.p, nullptr, gp, 2); }
+		{ HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<float><<<dim3(b.count, xrows_tiles(32 * b.rpl, 0)), kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_X, P->nt, d_rows, n_rows, V, nullptr, gp, 0); }
+		if (d_Y) { HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<float><<<dim3(b.count, xrows_tiles(32 * b.rpl, 2)), kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_Y, P->nt, d_rows, n_rows, P->scrT.p, nullptr, gp, 2); }
 		{ HA_LAUNCH(kHaB200KRidge, bs); k_pchol<float><<<b.count, kBlock, pchol_smem(b.rpl), bs>>>(wk, V, A, P->stats.p); }
 		{
 			HA_LAUNCH(kHaB200KJacobi32, bs);

@@ -82,10 +82,19 @@ __device__ __forceinline__ GridLayout grid_layout(const GridParams &gp, int n) {
 }
 
 // A_s = X[rows, sl]^T Z[rows, sl] (Z = X for the Gram, Y for the cross-covariance) over one row
-// list with duplicates, in Real, the k_xcov tiling with gathered rows.  Output column-major:
-// mode 0 at Ascr + w.aofs with ncol columns (padding columns zero), mode 1 into the searchlight's
-// grid C block, mode 2 at Ascr + w.tofs (n x n).
-template <int KT, typename Real>
+// list with duplicates, in Real, summed in row order.  Output column-major: mode 0 (the Gram; Z is X) at
+// Ascr + w.aofs with ncol columns (padding columns zero), mode 1 into the searchlight's grid C block,
+// mode 2 at Ascr + w.tofs (n x n).
+// One CTA per searchlight and 64 x 64 tile, 4 x 4 elements a thread (with one CTA per searchlight walking the
+// tiles, 512 searchlights of 50-500 vertices and five models of 400 rows took 29.9 ms in all); of the
+// Gram the lower tiles, each stored twice.  A warp brings in four rows by eight samples at a time, which
+// its stores into the sample-major tiles leave free of bank conflicts.
+constexpr int kXrT = 32, kXrPitch = 68;
+__host__ __device__ __forceinline__ int xrows_tiles(int nmax, int mode) {
+	const int nb = (nmax + 63) / 64;
+	return mode == 0 ? nb * (nb + 1) / 2 : nb * nb;
+}
+template <typename Real>
 __global__ void __launch_bounds__(256) k_xcov_rows(const SlWork *__restrict__ work, const int32_t *__restrict__ sl_idx,
                                                    const double *__restrict__ X, const double *__restrict__ Z, int nt,
                                                    const int32_t *__restrict__ rows, int nrows, Real *__restrict__ Ascr,
@@ -95,66 +104,68 @@ __global__ void __launch_bounds__(256) k_xcov_rows(const SlWork *__restrict__ wo
 	const int ncol = w.nblk * w.bsz;
 	const int32_t *sl = sl_idx + w.sofs;
 	Real *A = mode == 1 ? Gscr + gp.gbase[w.slot] + grid_layout(gp, n).C : Ascr + (mode == 2 ? w.tofs : w.aofs);
-	__shared__ Real xs[KT][64 + 1];
-	__shared__ Real zs[KT][64 + 1];
+	if (mode == 0 && blockIdx.y == 0)
+		for (int64_t e = (int64_t)n * n + threadIdx.x; e < (int64_t)n * ncol; e += 256) A[e] = Real(0);
+	int bi, bj;
+	if (mode == 0) {
+		bi = 0;
+		for (bj = (int)blockIdx.y; bj > bi; bi++) bj -= bi + 1;  // tile y of the lower triangle by rows
+	} else {
+		const int nb = (n + 63) / 64;
+		bi = (int)blockIdx.y / nb;
+		bj = (int)blockIdx.y - bi * nb;
+	}
+	const int i0 = 64 * bi, j0 = 64 * bj;
+	if (i0 >= n) return;
+	__shared__ __align__(16) Real xs[kXrT][kXrPitch];
+	__shared__ __align__(16) Real zs[kXrT][kXrPitch];
 	__shared__ int32_t vi[64], vj[64];
-	__shared__ int32_t rt[KT];
-	const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-	for (int i0 = 0; i0 < n; i0 += 64) {
-		for (int j0 = 0; j0 < n; j0 += 64) {
-			__syncthreads();
-			if (threadIdx.x < 64) {
-				const int i = i0 + threadIdx.x;
-				vi[threadIdx.x] = (i < n) ? sl[i] : -1;
-			} else if (threadIdx.x < 128) {
-				const int j = j0 + threadIdx.x - 64;
-				vj[threadIdx.x - 64] = (j < n) ? sl[j] : -1;
-			}
-			Real acc[4][4];
+	const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, warp = tid >> 5, lane = tid & 31;
+	if (tid < 64) vi[tid] = (i0 + tid < n) ? sl[i0 + tid] : -1;
+	else if (tid < 128) vj[tid - 64] = (j0 + tid - 64 < n) ? sl[j0 + tid - 64] : -1;
+	Real acc[4][4];
 #pragma unroll
-			for (int a = 0; a < 4; a++)
+	for (int p = 0; p < 4; p++)
 #pragma unroll
-				for (int b = 0; b < 4; b++) acc[a][b] = Real(0);
-			for (int t0 = 0; t0 < nrows; t0 += KT) {
-				__syncthreads();
-				if (threadIdx.x < KT) rt[threadIdx.x] = (t0 + threadIdx.x < nrows) ? rows[t0 + threadIdx.x] : -1;
-				__syncthreads();
-				for (int e = threadIdx.x; e < 64 * KT; e += 256) {
-					const int r = e / KT, t = e - r * KT;
-					const int tt = rt[t];
-					const int v = vi[r], u = vj[r];
-					xs[t][r] = (v >= 0 && tt >= 0) ? (Real)X[(int64_t)v * nt + tt] : Real(0);
-					zs[t][r] = (u >= 0 && tt >= 0) ? (Real)Z[(int64_t)u * nt + tt] : Real(0);
-				}
-				__syncthreads();
-#pragma unroll 4
-				for (int t = 0; t < KT; t++) {
-					Real a[4], b[4];
+		for (int q = 0; q < 4; q++) acc[p][q] = Real(0);
+	for (int t0 = 0; t0 < nrows; t0 += kXrT) {
+		__syncthreads();
+		// warp: samples 8 (warp % 4) .., rows 4 (warp / 4) .. and every eighth from there
+		const int t = 8 * (warp & 3) + (lane & 7), tt = t0 + t < nrows ? rows[t0 + t] : -1;
 #pragma unroll
-					for (int q = 0; q < 4; q++) {
-						a[q] = xs[t][ty + 16 * q];
-						b[q] = zs[t][tx + 16 * q];
-					}
+		for (int k = 0; k < 8; k++) {
+			const int r = 8 * k + 4 * (warp >> 2) + (lane >> 3);
+			const int v = vi[r], u = vj[r];
+			xs[t][r] = (v >= 0 && tt >= 0) ? (Real)X[(int64_t)v * nt + tt] : Real(0);
+			zs[t][r] = (u >= 0 && tt >= 0) ? (Real)Z[(int64_t)u * nt + tt] : Real(0);
+		}
+		__syncthreads();
+#pragma unroll 8
+		for (int s = 0; s < kXrT; s++) {
+			Real a[4], b[4];
 #pragma unroll
-					for (int p = 0; p < 4; p++)
-#pragma unroll
-						for (int q = 0; q < 4; q++) acc[p][q] += a[p] * b[q];
-				}
+			for (int q = 0; q < 4; q++) {
+				a[q] = xs[s][4 * ty + q];
+				b[q] = zs[s][4 * tx + q];
 			}
 #pragma unroll
-			for (int p = 0; p < 4; p++) {
-				const int i = i0 + ty + 16 * p;
-				if (i >= n) continue;
+			for (int p = 0; p < 4; p++)
 #pragma unroll
-				for (int q = 0; q < 4; q++) {
-					const int j = j0 + tx + 16 * q;
-					if (j < n) A[(int64_t)j * n + i] = acc[p][q];
-				}
-			}
+				for (int q = 0; q < 4; q++) acc[p][q] += a[p] * b[q];
 		}
 	}
-	if (mode == 0)
-		for (int64_t e = (int64_t)n * n + threadIdx.x; e < (int64_t)n * ncol; e += 256) A[e] = Real(0);
+#pragma unroll
+	for (int p = 0; p < 4; p++) {
+		const int i = i0 + 4 * ty + p;
+		if (i >= n) continue;
+#pragma unroll
+		for (int q = 0; q < 4; q++) {
+			const int j = j0 + 4 * tx + q;
+			if (j >= n) continue;
+			A[(int64_t)j * n + i] = acc[p][q];
+			if (mode == 0 && bi != bj) A[(int64_t)i * n + j] = acc[p][q];
+		}
+	}
 }
 
 // Pivoted Cholesky G = sum_k r_k r_k^T (pivot = largest remaining diagonal, ties to the smaller
