@@ -2499,8 +2499,11 @@ int run_ridge_learned(HaB200Plan *P, const double *d_X, const double *d_Y, const
 		if (fp32) {
 			if ((rc = eigen_chunk32(P, ch, d_X, d_Y, P->gfit.p, n_rows, P->gfeat.p, st)) != kHaSuccess) return rc;
 			if ((rc = propose()) != kHaSuccess) return rc;
-			HA_LAUNCH(kHaB200KGrid, st);
-			k_proposed_fit<float><<<(int)ch.weig32.size(), kBlock, 0, st>>>(ch.d_weig32, reinterpret_cast<const float *>(P->scrV.p), P->uv.p, reinterpret_cast<float *>(P->scrA.p), P->scrT.p, P->scrT64.p, d_choice, d_prob, min_prob, gp.alphas, gp.npcs, gp.n_npcs, n_rows, rowmajor);
+			const float *V = reinterpret_cast<const float *>(P->scrV.p);
+			float *Q = reinterpret_cast<float *>(P->scrA.p);
+			const dim3 grid((unsigned)ch.weig32.size(), kProposedParts);
+			{ HA_LAUNCH(kHaB200KGrid, st); k_proposed_q<float><<<grid, kBlock, 0, st>>>(ch.d_weig32, V, Q, P->scrT.p, d_prob, min_prob); }
+			{ HA_LAUNCH(kHaB200KGrid, st); k_proposed_beta<float><<<grid, kBlock, 0, st>>>(ch.d_weig32, V, P->uv.p, Q, P->scrT64.p, d_choice, d_prob, min_prob, gp.alphas, gp.npcs, gp.n_npcs, n_rows, rowmajor); }
 		} else {
 			// a batch's factors are at hand only until the next one's: the proposals are taken after every
 			// batch (those of searchlights without features yet are overwritten later)

@@ -566,26 +566,45 @@ __global__ void __launch_bounds__(256) k_features(const SlWork *__restrict__ wor
 // (csrc/ha_ridge.c:97-227) restricted to one (alpha, PC count), with mult_k the number of PC
 // chunks up to p that contain component k's rank (clipped at K = min(rows, n)).  V (eigenvectors,
 // column-major ld n) and lambda come from the eigenvector-mode Jacobi, C = X_fit^T Y_fit is at
-// Cin + w.tofs; beta goes to Bout + w.tofs (float64, T layout; Cin may be Bout: C is read first);
-// Q = V^T C goes to the A scratch.  Real is the arithmetic type of the products.
+// Cin + w.tofs; beta goes to Bout + w.tofs (float64, T layout); Q = V^T C goes to the A scratch by
+// k_proposed_q, beta from it by k_proposed_beta.  Real is the arithmetic type of the products.  Both spread
+// a searchlight's tiles over gridDim.y CTAs: with one CTA per searchlight doing both products the largest
+// searchlights (n = 500) set the time, 12.7 ms for 512 searchlights.
+constexpr int kProposedParts = 16;
+
 template <typename Real>
-__global__ void __launch_bounds__(256) k_proposed_fit(const SlWork *__restrict__ work, const Real *__restrict__ Vscr,
-                                                      const double *__restrict__ uvbuf, Real *__restrict__ Ascr,
-                                                      const Real *Cin, double *Bout, const int32_t *__restrict__ cls,
-                                                      const float *__restrict__ prob, float min_prob,
-                                                      const double *__restrict__ alphas, const int32_t *__restrict__ npcs,
-                                                      int n_npcs, int rows, int t_rowmajor) {
+__global__ void __launch_bounds__(256) k_proposed_q(const SlWork *__restrict__ work, const Real *__restrict__ Vscr,
+                                                    Real *__restrict__ Ascr, const Real *__restrict__ Cin,
+                                                    const float *__restrict__ prob, float min_prob) {
+	__shared__ Real ps[16][65], qs[16][65];
+	const SlWork w = work[blockIdx.x];
+	if (prob[w.s] < min_prob) return;
+	const int n = w.n;
+	// Q(k, j) = sum_i V(i, k) C(i, j)
+	GemmArgs<Real, Real> g;
+	g.d = nullptr; g.alpha = Real(1); g.E = nullptr; g.ei = 0; g.ej = 0; g.beta = Real(0);
+	g.M = n; g.N = n; g.K = n;
+	g.P = Vscr + w.aofs; g.pk = 1; g.pi = n;
+	g.Q = Cin + w.tofs; g.qk = 1; g.qj = n;
+	g.C = Ascr + w.aofs; g.ci = 1; g.cj = n;
+	block_gemm(g, ps, qs, (int)blockIdx.y, (int)gridDim.y);
+}
+
+template <typename Real>
+__global__ void __launch_bounds__(256) k_proposed_beta(const SlWork *__restrict__ work, const Real *__restrict__ Vscr,
+                                                       const double *__restrict__ uvbuf, const Real *__restrict__ Ascr,
+                                                       double *__restrict__ Bout, const int32_t *__restrict__ cls,
+                                                       const float *__restrict__ prob, float min_prob,
+                                                       const double *__restrict__ alphas, const int32_t *__restrict__ npcs,
+                                                       int n_npcs, int rows, int t_rowmajor) {
 	__shared__ Real ps[16][65], qs[16][65];
 	__shared__ int order[kGridMaxN];
 	__shared__ Real cval[kGridMaxN];
 	const SlWork w = work[blockIdx.x];
 	if (prob[w.s] < min_prob) return;
-	const int n = w.n;
-	const Real *V = Vscr + w.aofs;
+	const int n = w.n, nb = (n + 63) / 64;
+	if ((int)blockIdx.y >= nb * nb) return;
 	const double *lam = uvbuf + w.uvofs;
-	Real *Q = Ascr + w.aofs;
-	const Real *Cs = Cin + w.tofs;
-	double *B = Bout + w.tofs;
 	const int g = cls[w.s];
 	const int a = g / n_npcs, p = g - a * n_npcs;
 	const Real al = (Real)alphas[a];
@@ -602,24 +621,15 @@ __global__ void __launch_bounds__(256) k_proposed_fit(const SlWork *__restrict__
 		const int k = order[r];
 		cval[k] = mult ? (Real)mult / (al + (Real)lam[k]) : Real(0);
 	}
-	GemmArgs<Real, Real> gm;
-	gm.d = nullptr; gm.alpha = Real(1); gm.E = nullptr; gm.ei = 0; gm.ej = 0; gm.beta = Real(0);
-	// Q(k, j) = sum_i V(i, k) C(i, j)
-	gm.M = n; gm.N = n; gm.K = n;
-	gm.P = V; gm.pk = 1; gm.pi = n;
-	gm.Q = Cs; gm.qk = 1; gm.qj = n;
-	gm.C = Q; gm.ci = 1; gm.cj = n;
-	block_gemm(gm, ps, qs);
-	__syncthreads();  // every read of C (which may share memory with beta) is done
+	__syncthreads();
 	// beta(i, j) = sum_k V(i, k) c_k Q(k, j), in the T layout
-	gm.P = V; gm.pk = n; gm.pi = 1;
-	gm.Q = Q; gm.qk = 1; gm.qj = n;
-	gm.d = cval;
 	GemmArgs<Real, double> gb;
-	gb.M = gm.M; gb.N = gm.N; gb.K = gm.K; gb.P = gm.P; gb.pk = gm.pk; gb.pi = gm.pi; gb.Q = gm.Q; gb.qk = gm.qk;
-	gb.qj = gm.qj; gb.d = gm.d; gb.alpha = Real(1); gb.E = nullptr; gb.ei = 0; gb.ej = 0; gb.beta = Real(0);
-	gb.C = B; gb.ci = t_rowmajor ? n : 1; gb.cj = t_rowmajor ? 1 : n;
-	block_gemm(gb, ps, qs);
+	gb.M = n; gb.N = n; gb.K = n;
+	gb.P = Vscr + w.aofs; gb.pk = n; gb.pi = 1;
+	gb.Q = Ascr + w.aofs; gb.qk = 1; gb.qj = n;
+	gb.d = cval; gb.alpha = Real(1); gb.E = nullptr; gb.ei = 0; gb.ej = 0; gb.beta = Real(0);
+	gb.C = Bout + w.tofs; gb.ci = t_rowmajor ? n : 1; gb.cj = t_rowmajor ? 1 : n;
+	block_gemm(gb, ps, qs, (int)blockIdx.y, (int)gridDim.y);
 }
 
 }  // namespace hab200

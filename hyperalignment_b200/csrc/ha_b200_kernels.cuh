@@ -542,7 +542,8 @@ __device__ Real block_max_nonneg(Real v, Real *scratch32) {
 // generic small GEMM:  C(i, j) = alpha * sum_k P(k, i) d(k) Q(k, j) + beta * E(i, j)
 // ---------------------------------------------------------------------------------------------
 // Operands are addressed through strides, P(k, i) = P[k*pk + i*pi] etc., so the same routine
-// serves every layout used here; tiles of 64x64 outputs per pass, K staged in chunks of 16.
+// serves every layout used here; tiles of 64x64 outputs per pass, K staged in chunks of 16.  Of the tiles,
+// those with index part modulo parts.
 template <typename Real, typename OutT = Real>
 struct GemmArgs {
 	int M, N, K;
@@ -560,12 +561,14 @@ struct GemmArgs {
 };
 
 template <typename Real, typename OutT>
-__device__ void block_gemm(const GemmArgs<Real, OutT> &g, Real (*ps)[65], Real (*qs)[65]) {
+__device__ void block_gemm(const GemmArgs<Real, OutT> &g, Real (*ps)[65], Real (*qs)[65], int part = 0, int parts = 1) {
 	constexpr int KC = 16;
 	const int tx = threadIdx.x & 15, ty = (threadIdx.x >> 4) & 15;
 	const int nthr = blockDim.x;  // 256 assumed for the compute mapping
+	int tile = 0;
 	for (int i0 = 0; i0 < g.M; i0 += 64) {
 		for (int j0 = 0; j0 < g.N; j0 += 64) {
+			if (tile++ % parts != part) continue;
 			Real acc[4][4];
 #pragma unroll
 			for (int a = 0; a < 4; a++)
