@@ -180,7 +180,8 @@ int ha_searchlight_ridge_csc_b200(
  * model-averaged beta (n_s x n_s) is scattered like ha_searchlight_ridge_csc_b200.  PC chunks
  * follow the reference: [npcs[p-1], npcs[p]) clipped at min(train rows, n_s), summed over p.
  * cost_out (count x n_alphas x n_npcs float64, may be NULL) receives every grid cost.
- * Computed in float64 (eigen decomposition of X_tr^T X_tr by Jacobi rotations).  kHaErrorArg for
+ * Computed in float64 (eigen decomposition of the smaller side's Gram of the distinct training rows by
+ * tridiagonalisation and implicit QL).  kHaErrorArg for
  * negative PC counts, non-finite alphas, empty training lists, rows outside [0, nt), a row
  * repeated within one test list, or a searchlight of more than 512 vertices.
  */
@@ -237,7 +238,7 @@ int ha_searchlight_template_b200(
  * tmpl = U_n S_n / sqrt(n_subj) from the top n singular pairs of X; R = polar(tmpl^T sum_s
  * dms_s[:, sl]) (reflection allowed, no scaling); tpl_out[:, sl] += (tmpl R) diag(w) with the
  * searchlight weights of sl_dists and radius (ha_compute_weights).  The singular pairs are exact
- * (float64 Gram of the smaller side, eigen decomposition by Jacobi rotations): they agree with the
+ * (float64 Gram of the smaller side, eigen decomposition by tridiagonalisation and implicit QL): they agree with the
  * reference's randomized SVD where the top-n singular subspace is separated from the rest.
  * dms: n_subj consecutive nt x nv float64 column-major matrices (host); tpl_out: nt x nv float64
  * column-major (host, overwritten).  kHaErrorArg when a searchlight holds more than nt vertices
@@ -290,7 +291,8 @@ int ha_b200_plan_pattern(const HaB200Plan *plan, int64_t *indptr, int32_t *indic
 int ha_b200_plan_device_pattern(const HaB200Plan *plan, const int64_t **d_indptr, const int32_t **d_indices);
 /* Searchlights of the last run that were solved in FP64, and that hit the sweep limit. */
 int ha_b200_plan_stats(const HaB200Plan *plan, int32_t *n_fp64, int32_t *n_jacobi_unconverged);
-/* Jacobi sweeps of the last run: sum over searchlights (final solve of each) and maximum. */
+/* Jacobi sweeps of the last run: sum over searchlights (final solve of each) and maximum (0 after a
+ * float64 grid search, which has none). */
 int ha_b200_plan_sweep_stats(const HaB200Plan *plan, int64_t *sweeps_sum, int32_t *sweeps_max);
 /*
  * Per-searchlight solve record of the last run, searchlights [first, first + n) of its last
@@ -489,8 +491,8 @@ int ha_b200_kernel_times(double *ms, int64_t *launches);
 int64_t ha_b200_launch_count(void);
 
 /*
- * Tile layout of the tensor-core solver's per-phase launches, per size class (tiles of at most 128
- * columns; of 129-256): shared memory per CTA in KB, which sets the CTAs per SM and the pipeline
+ * Tile layout of the tensor-core solver's 128-row per-phase launches (HA_B200_TC_RESIDENT=0; by default
+ * the iteration runs in kernels of fixed layout), per size class (tiles of at most 128 columns; of 129-256): shared memory per CTA in KB, which sets the CTAs per SM and the pipeline
  * depth.  Class 0 candidates: 110, 72, 53 KB (2, 3, 4 CTAs per SM); class 1: 110, 200 KB (2, 1).
  * The plan's first tensor-core run times one Gram launch per candidate with CUDA events and keeps
  * the fastest (environment HA_B200_AUTOTUNE=0 keeps 110 / 110 instead); every layout gives the same
@@ -500,8 +502,8 @@ int64_t ha_b200_launch_count(void);
 int ha_b200_plan_tc_layout(const HaB200Plan *plan, int32_t *smem_kb, int32_t *tuned, double *cand_ms);
 
 /*
- * Repeated launch sequences (the tensor-core iteration of a plan chunk, the ridge grid search of a
- * plan) are captured once into CUDA graphs and replayed; off, they are launched one by one.  On by
+ * Repeated launch sequences (the tensor-core iteration of a plan chunk for its searchlights of more than 256
+ * vertices, the FP32 ridge grid search of a plan) are captured once into CUDA graphs and replayed; off, they are launched one by one.  On by
  * default (environment HA_B200_GRAPHS=0 turns it off); the results are the same bit for bit.
  */
 void ha_b200_set_graphs(bool on);
