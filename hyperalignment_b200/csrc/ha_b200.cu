@@ -490,7 +490,7 @@ size_t scratch_budget_bytes() {
 
 // Sort work items by Jacobi class (resident or blocked, rows per lane), largest first inside a
 // class, and cut them into buckets of one Jacobi kernel instance each.  prec: 0 float32 polar,
-// 1 float64 polar, 2 float32 eigenvector mode.
+// 1 float64 polar, 2 float32 eigenvector mode, 3 float64 eigenvector mode.
 std::vector<Bucket> bucketize(std::vector<SlWork> &items, int prec) {
 	auto key = [](const SlWork &w) { return (w.nblk == 2 ? 0 : 32) + rpl_for(w.n); };
 	std::stable_sort(items.begin(), items.end(), [&](const SlWork &a, const SlWork &b) {
@@ -505,7 +505,7 @@ std::vector<Bucket> bucketize(std::vector<SlWork> &items, int prec) {
 		while (j < (int)items.size() && key(items[j]) == key(items[i])) {
 			int bb, kk;
 			size_t mm;
-			const bool f64 = prec == 1;
+			const bool f64 = prec == 1 || prec == 3;
 			jacobi_layout(items[j].n, f64, bb, kk, mm, f64 ? kSmemMax : fp32_jacobi_budget(), prec < 2);
 			smem = std::max(smem, mm);
 			j++;
@@ -515,7 +515,7 @@ std::vector<Bucket> bucketize(std::vector<SlWork> &items, int prec) {
 		b.count = j - i;
 		b.smem = smem;
 		b.blocked = items[i].nblk != 2;
-		b.threads = jacobi_threads(items[i].bsz, prec == 1);
+		b.threads = jacobi_threads(items[i].bsz, prec == 1 || prec == 3);
 		b.rpl = rpl_for(items[i].n);
 		buckets.push_back(b);
 		i = j;
@@ -680,6 +680,7 @@ int set_smem_attrs() {
 	HA_CUDA(cudaFuncSetAttribute(k_dg_beta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
 	HA_CUDA(cudaFuncSetAttribute(k_ridge_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgSmem));
 	HA_CUDA(cudaFuncSetAttribute(k_ridge_chol, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRidgeSmem));
+	HA_CUDA(cudaFuncSetAttribute(k_pchol<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kPcholNb * kGridMaxN * 8)));
 	HA_CUDA(cudaFuncSetAttribute(k_pchol<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kPcholNb * kGridMaxN * 4)));
 	done = true;
 	return kHaSuccess;
@@ -1868,7 +1869,7 @@ int grid_prepare(HaB200Plan *P) {
 	return P->scrT64.ensure((size_t)maxT);
 }
 
-size_t pchol_smem(int rpl) { return (size_t)kPcholNb * 32 * rpl * sizeof(float); }
+size_t pchol_smem(int rpl, size_t esz) { return (size_t)kPcholNb * 32 * rpl * esz; }
 
 JacobiParams eig_params(bool only_flagged) {
 	JacobiParams jp;
@@ -1963,7 +1964,7 @@ int grid_chunk_launch(HaB200Plan *P, Chunk &ch, const double *d_X, const double 
 				// Gram into the V scratch, its pivoted Cholesky factor into the A scratch
 				{ HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<Real><<<dim3(x1 - x0, xrows_tiles(32 * b.rpl, 0)), kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_X, nt, tr, md.tr_n, V, G, gp, 0); }
 				{ HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<Real><<<dim3(x1 - x0, xrows_tiles(32 * b.rpl, 1)), kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_Y, nt, tr, md.tr_n, A, G, gp, 1); }
-				{ HA_LAUNCH(kHaB200KRidge, bs); k_pchol<Real><<<x1 - x0, kBlock, pchol_smem(b.rpl), bs>>>(wk, V, A, P->stats.p); }
+				{ HA_LAUNCH(kHaB200KRidge, bs); k_pchol<Real><<<x1 - x0, kBlock, pchol_smem(b.rpl, sizeof(float)), bs>>>(wk, V, A, P->stats.p); }
 				{
 					HA_LAUNCH(kHaB200KJacobi32, bs);
 					if ((rc = launch_jacobi<Real>(b.rpl, x1 - x0, b.threads, b.smem, bs, wk, A, V, P->scrT.p, P->stats.p, P->uv.p, jp)) != kHaSuccess)
@@ -2415,7 +2416,7 @@ int eigen_chunk32(HaB200Plan *P, Chunk &ch, const double *d_X, const double *d_Y
 		const SlWork *wk = ch.d_weig32 + b.first;
 		{ HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<float><<<dim3(b.count, xrows_tiles(32 * b.rpl, 0)), kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_X, P->nt, d_rows, n_rows, V, nullptr, gp, 0); }
 		if (d_Y) { HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<float><<<dim3(b.count, xrows_tiles(32 * b.rpl, 2)), kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_Y, P->nt, d_rows, n_rows, P->scrT.p, nullptr, gp, 2); }
-		{ HA_LAUNCH(kHaB200KRidge, bs); k_pchol<float><<<b.count, kBlock, pchol_smem(b.rpl), bs>>>(wk, V, A, P->stats.p); }
+		{ HA_LAUNCH(kHaB200KRidge, bs); k_pchol<float><<<b.count, kBlock, pchol_smem(b.rpl, sizeof(float)), bs>>>(wk, V, A, P->stats.p); }
 		{
 			HA_LAUNCH(kHaB200KJacobi32, bs);
 			if ((rc = launch_jacobi<float>(b.rpl, b.count, b.threads, b.smem, bs, wk, A, V, P->scrT.p, P->stats.p, P->uv.p, jp)) != kHaSuccess)
@@ -2985,13 +2986,14 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 		nn[s] = n;
 		mg[s] = n > 0 ? m : nt;
 		if (n == 0) { region[s] = ptot[s] = 0; bytes[s] = 0; continue; }
-		int bp, kp;
-		size_t mp;
+		int be, ke, bp, kp;
+		size_t me, mp;
+		jacobi_layout(m, true, be, ke, me, kSmemMax, false);
 		jacobi_layout(n, true, bp, kp, mp);
-		int64_t r = std::max<int64_t>((int64_t)m * m, (int64_t)n * kp * bp);
+		int64_t r = std::max<int64_t>((int64_t)m * std::max(m, be * ke), (int64_t)n * kp * bp);
 		region[s] = (r + 31) & ~(int64_t)31;
 		ptot[s] = PcaLayout::make(nt, n, m, m != nt).total;
-		bytes[s] = (size_t)(2 * region[s] + ptot[s] + m + 2 * n + EigScratch::make(m).total) * 8 + (size_t)n * n * 4 +
+		bytes[s] = (size_t)(2 * region[s] + ptot[s] + m + 2 * n + 3 * (int64_t)n * n) * 8 + (size_t)n * n * 4 +
 		           2 * sizeof(SlStats);
 	}
 	// batches of consecutive searchlights
@@ -3014,7 +3016,7 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 		int64_t R = 0, Pt = 0, Tt = 0, U = 0, E = 0;
 		for (int s = bstart[b]; s < bstart[b + 1]; s++) {
 			R += region[s];
-			E += nn[s] > 0 ? EigScratch::make(mg[s]).total : 0;
+			E += (3 * (int64_t)nn[s] * nn[s] + 3) & ~(int64_t)3;
 			Pt += ptot[s];
 			Tt += (int64_t)nn[s] * nn[s];
 			U += nn[s] > 0 ? mg[s] + 2 * nn[s] : 0;
@@ -3029,15 +3031,14 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 	const size_t m1 = (size_t)nt * nv;
 	DevArr<double> D, eA, eV, eS, Pw, uvb, tpl;
 	DevArr<float> T;
-	DevArr<SlStats> stP;
-	DevArr<SlWork> dwe, dwp, dwps;
-	DevArr<EigWork> deig;
+	DevArr<SlStats> stE, stP;
+	DevArr<SlWork> dwe, dwp, dwes, dwps;
 	PolarBufs polar;
 	DevArr<int64_t> dpofs;
 	DevArr<int32_t> dmg;
 	auto done = [&](int code) {
 		D.release(); eA.release(); eV.release(); eS.release(); Pw.release(); uvb.release(); tpl.release(); T.release();
-		stP.release(); dwe.release(); dwp.release(); dwps.release(); deig.release(); polar.release();
+		stE.release(); stP.release(); dwe.release(); dwp.release(); dwes.release(); dwps.release(); polar.release();
 		dpofs.release(); dmg.release();
 		return code;
 	};
@@ -3046,7 +3047,7 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 	    (rc = Pw.ensure((size_t)maxP)) != kHaSuccess || (rc = uvb.ensure((size_t)maxUV)) != kHaSuccess ||
 	    (rc = T.ensure((size_t)maxT)) != kHaSuccess || (rc = eS.ensure((size_t)maxE)) != kHaSuccess ||
 	    (rc = stP.ensure((size_t)maxS)) != kHaSuccess || (rc = dwe.ensure((size_t)maxS)) != kHaSuccess ||
-	    (rc = dwp.ensure((size_t)maxS)) != kHaSuccess || (rc = deig.ensure((size_t)maxS)) != kHaSuccess ||
+	    (rc = dwp.ensure((size_t)maxS)) != kHaSuccess || (rc = dwes.ensure((size_t)maxS)) != kHaSuccess || (rc = stE.ensure((size_t)maxS)) != kHaSuccess ||
 	    (rc = dwps.ensure((size_t)maxS)) != kHaSuccess || (rc = dpofs.ensure((size_t)maxS)) != kHaSuccess ||
 	    (rc = dmg.ensure((size_t)maxS)) != kHaSuccess)
 		return done(rc);
@@ -3054,6 +3055,7 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 	if (cudaMemcpyAsync(D.p, dms, m1 * ns * 8, cudaMemcpyHostToDevice, st) != cudaSuccess ||
 	    cudaMemsetAsync(tpl.p, 0, m1 * 8, st) != cudaSuccess)
 		return done(kHaErrorInternal);
+	const JacobiParams jpe = eig_params(false);
 	JacobiParams jpp;
 	jpp.max_sweeps = 40;
 	jpp.t_rowmajor = 0;
@@ -3069,7 +3071,6 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 		std::vector<SlWork> we, wp;
 		std::vector<int64_t> pofs(s_hi - s_lo, 0);
 		std::vector<int32_t> mgb(s_hi - s_lo);
-		std::vector<EigWork> eig;
 		std::vector<PolarWork> pol;
 		int64_t ro = 0, po = 0, to = 0, uo = 0, eo = 0;
 		for (int s = s_lo; s < s_hi; s++) {
@@ -3087,13 +3088,13 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 			{
 				int bb, kk;
 				size_t mm;
+				jacobi_layout(m, true, bb, kk, mm, kSmemMax, false);
+				e.bsz = bb; e.nblk = kk;
 				jacobi_layout(n, true, bb, kk, mm);
-				p.bsz = e.bsz = bb;
-				p.nblk = e.nblk = kk;
+				p.bsz = bb; p.nblk = kk;
 			}
-			eig.push_back({ro, ro, eo, uo, m, 0});
 			pol.push_back({ro, eo, eo + (int64_t)n * n, eo + 2 * (int64_t)n * n, to, n, q, 0, 0});
-			eo += EigScratch::make(m).total;
+			eo += (3 * (int64_t)n * n + 3) & ~(int64_t)3;  // the iterates of the polar factor
 			e.uvofs = uo;
 			p.uvofs = uo + m;
 			we.push_back(e);
@@ -3106,18 +3107,16 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 		}
 		const int nb = (int)we.size();
 		if (nb == 0) continue;
-		std::vector<SlWork> wps = wp;
-		const std::vector<Bucket> bp = bucketize(wps, 1);
-		std::stable_sort(eig.begin(), eig.end(), [](const EigWork &a, const EigWork &b) { return a.p > b.p; });
+		std::vector<SlWork> wes = we, wps = wp;
+		const std::vector<Bucket> be = bucketize(wes, 3), bp = bucketize(wps, 1);
 		std::stable_sort(pol.begin(), pol.end(), [](const PolarWork &a, const PolarWork &b) { return a.n > b.n; });
-		std::vector<int> orders(eig.size());
-		for (size_t k = 0; k < eig.size(); k++) orders[k] = eig[k].p;
 		if (cudaMemcpyAsync(dwe.p, we.data(), nb * sizeof(SlWork), cudaMemcpyHostToDevice, st) != cudaSuccess ||
 		    cudaMemcpyAsync(dwp.p, wp.data(), nb * sizeof(SlWork), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-		    cudaMemcpyAsync(deig.p, eig.data(), nb * sizeof(EigWork), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+		    cudaMemcpyAsync(dwes.p, wes.data(), nb * sizeof(SlWork), cudaMemcpyHostToDevice, st) != cudaSuccess ||
 		    cudaMemcpyAsync(dwps.p, wps.data(), nb * sizeof(SlWork), cudaMemcpyHostToDevice, st) != cudaSuccess ||
 		    cudaMemcpyAsync(dpofs.p, pofs.data(), pofs.size() * 8, cudaMemcpyHostToDevice, st) != cudaSuccess ||
 		    cudaMemcpyAsync(dmg.p, mgb.data(), mgb.size() * 4, cudaMemcpyHostToDevice, st) != cudaSuccess ||
+		    cudaMemsetAsync(stE.p, 0, (size_t)(s_hi - s_lo) * sizeof(SlStats), st) != cudaSuccess ||
 		    cudaMemsetAsync(stP.p, 0, (size_t)(s_hi - s_lo) * sizeof(SlStats), st) != cudaSuccess)
 			return done(kHaErrorInternal);
 		int nw = 1, mw = 1;  // widest searchlight and Gram order of the batch
@@ -3130,13 +3129,18 @@ int pca_template_impl(const double *dms, int ns, int nt, int nv, const int32_t *
 			HA_LAUNCH(kHaB200KPca, st);
 			k_pca_gram<<<dim3(tm * (tm + 1) / 2, std::min(nb - x, 65535)), kDgThreads, kDgSmem, st>>>(dwe.p + x, P->idx.p, P->off.p, D.p, ns, nt, nv, eV.p);
 		}
-		if ((rc = launch_eig(deig.p, orders, eV.p, eA.p, eS.p, uvb.p, st)) != kHaSuccess) return done(rc);
+		for (const Bucket &k : be) {
+			const SlWork *wk = dwes.p + k.first;
+			{ HA_LAUNCH(kHaB200KRidge, st); k_pchol<double><<<k.count, kBlock, pchol_smem(k.rpl, sizeof(double)), st>>>(wk, eV.p, eA.p, stE.p); }
+			HA_LAUNCH(kHaB200KJacobi64, st);
+			if ((rc = launch_jacobi<double>(k.rpl, k.count, k.threads, k.smem, st, wk, eA.p, eV.p, T.p, stE.p, uvb.p, jpe)) != kHaSuccess)
+				return done(rc);
+		}
 		{ HA_LAUNCH(kHaB200KPca, st); k_pca_tmpl<<<nb, kBlock, 0, st>>>(dwe.p, dwp.p, P->idx.p, D.p, ns, nt, nv, eV.p, uvb.p, dpofs.p, Pw.p); }
 		for (int x = 0; x < nb; x += 65535) {
 			HA_LAUNCH(kHaB200KPca, st);
 			k_pca_b<<<dim3(tn * tn, std::min(nb - x, 65535)), kDgThreads, kDgSmem, st>>>(dwe.p + x, dwp.p + x, nt, dpofs.p, Pw.p, eA.p);
 		}
-		// the eigen decomposition's scratch holds the iterates (it is at least 4 m^2 per searchlight)
 		if ((rc = polar_solve(polar, pol, eA.p, eS.p, T.p, stP.p, st)) != kHaSuccess) return done(rc);
 		// the flagged ones by Jacobi
 		for (const Bucket &k : bp) {

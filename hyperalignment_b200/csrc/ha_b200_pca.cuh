@@ -128,7 +128,9 @@ __global__ void __launch_bounds__(kDgThreads) k_pca_gram(const SlWork *__restric
 	}
 	double *G = Gscr + w.aofs;
 	dg_each(acc, [&](int i, int j, double v) {
-		if (i0 + i < m && j0 + j < m) G[(int64_t)(j0 + j) * m + i0 + i] = v;
+		if (i0 + i >= m || j0 + j >= m) return;
+		G[(int64_t)(j0 + j) * m + i0 + i] = v;
+		if (i0 != j0) G[(int64_t)(i0 + i) * m + j0 + j] = v;
 	});
 }
 

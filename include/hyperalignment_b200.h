@@ -238,7 +238,7 @@ int ha_searchlight_template_b200(
  * tmpl = U_n S_n / sqrt(n_subj) from the top n singular pairs of X; R = polar(tmpl^T sum_s
  * dms_s[:, sl]) (reflection allowed, no scaling); tpl_out[:, sl] += (tmpl R) diag(w) with the
  * searchlight weights of sl_dists and radius (ha_compute_weights).  The singular pairs are exact
- * (float64 Gram of the smaller side, eigen decomposition by tridiagonalisation and implicit QL): they agree with the
+ * (float64 Gram of the smaller side, eigen decomposition by Jacobi rotations): they agree with the
  * reference's randomized SVD where the top-n singular subspace is separated from the rest.
  * dms: n_subj consecutive nt x nv float64 column-major matrices (host); tpl_out: nt x nv float64
  * column-major (host, overwritten).  kHaErrorArg when a searchlight holds more than nt vertices
