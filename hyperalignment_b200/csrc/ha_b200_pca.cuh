@@ -7,7 +7,7 @@
 //   the top n singular pairs of X from the smaller Gram (m = min(nt, ns n) <= 512):
 //     time side   (m = nt):   X X^T = U diag(lambda) U^T,   tmpl = U_n diag(sqrt(lambda_n)) / sqrt(ns)
 //     vertex side (m = ns n): X^T X = W diag(lambda) W^T,   tmpl = X W_n / sqrt(ns)
-//   both by the batched eigen decomposition (ha_b200_eig.cuh); then M = sum_j D_j[:, sl],
+//   both by pivoted Cholesky and one-sided Jacobi (k_pchol, k_jacobi); then M = sum_j D_j[:, sl],
 //   R = polar(tmpl^T M) by the float64 Newton-Schulz iteration (ha_b200_polar.cuh), and
 //   template[:, sl] += (tmpl R) diag(w_s) with the searchlight weights, reduced per vertex in
 //   searchlight order.
