@@ -422,6 +422,9 @@ __global__ void __launch_bounds__(32) k_eig_ql(const EigWork *__restrict__ work,
 		for (int i = m - 1; i >= l; i--) {
 			const int ip = max(i - 1, l);
 			const double en = e[ip], dp = d[ip];  // read ahead of this step's stores
+			// lane 0 stores entries i + 1 below: every lane has read them (a sweep ago, or before the loop) by
+			// now, whatever the pace of the lanes
+			__syncwarp();
 			const double f = s * ei, b = c * ei;
 			const double h = fma(f, f, g * g);
 			const double gg = dn - q;
