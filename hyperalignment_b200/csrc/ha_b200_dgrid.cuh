@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kDgThreads) k_dg_project(const DgItem *__restr
 	});
 }
 
-// The eigenvalues as squared column norms of W or N, a warp a column (zero columns stay zero).
+// The eigenvalues as squared column norms of W or N, a warp a column.
 __global__ void __launch_bounds__(256) k_dg_lambda(const DgItem *__restrict__ items, double *S, const DgParams dp) {
 	const DgItem it = items[blockIdx.y];
 	const int rows = it.dual ? it.n : dp.mdl[it.model].d_n, lane = threadIdx.x & 31;
@@ -205,6 +205,22 @@ __global__ void __launch_bounds__(kDgThreads) k_dg_q(const DgItem *__restrict__ 
 	});
 }
 
+// Whether component k is rounding noise: its singular value, the column norm of W or N, is below p eps of
+// the largest, where a singular vector of a zero singular value ends up (its column of W is the sum of the
+// others' rounding).  The bound is on the column norm: the same bound on the Gram matrix's eigenvalue
+// drops true singular values up to sqrt(p eps) of the largest, which a small penalty still lets count (100
+// rows, 100 columns of which 50 repeat the others to 1e-5, alpha = 1e-3: beta 3e-3 off; here 1.4e-10).
+// NaN counts as a value.
+__device__ __forceinline__ bool dg_noise(const double *lam, int p, int k) {
+	const double r = p * Eps<double>::v();
+	return lam[k] <= r * r * lam[0];
+}
+
+// 1 / (alpha + l_k); 0 for noise, so that alpha = 0 gives the pseudoinverse.
+__device__ __forceinline__ double dg_coef(const double *lam, int p, int k, double alpha) {
+	return dg_noise(lam, p, k) ? 0.0 : 1.0 / (alpha + lam[k]);
+}
+
 // Features of the searchlights of a one-model batch: the 64 largest singular values divided by the
 // largest (zero-padded), then log n.
 __global__ void __launch_bounds__(kFeatSv) k_dg_features(const DgItem *__restrict__ items, const DgSl *__restrict__ sls,
@@ -214,19 +230,8 @@ __global__ void __launch_bounds__(kFeatSv) k_dg_features(const DgItem *__restric
 	float *f = feat + (int64_t)sls[blockIdx.x].s * (kFeatSv + 1);
 	const int k = threadIdx.x;
 	const double s1 = sqrt(lam[0]);
-	f[k] = (k < it.p && s1 > 0.0) ? (float)(sqrt(lam[k]) / s1) : 0.0f;
+	f[k] = (k < it.p && s1 > 0.0 && !dg_noise(lam, it.p, k)) ? (float)(sqrt(lam[k]) / s1) : 0.0f;
 	if (k == 0) f[kFeatSv] = logf((float)it.n);
-}
-
-// Components with a nonzero eigenvalue (they lead).
-__device__ __forceinline__ int dg_rank(const double *lam, int p) {
-	int lo = 0, hi = p;
-	while (lo < hi) {
-		const int mid = (lo + hi) >> 1;
-		if (lam[mid] > 0.0 || isnan(lam[mid])) lo = mid + 1;
-		else hi = mid;
-	}
-	return lo;
 }
 
 // Position in the PC chunks: slice [k, min(k + 16, hi)) of chunk p (csrc/ha_ridge.c:187-210: chunk p
@@ -275,8 +280,8 @@ __global__ void __launch_bounds__(kDgThreads) k_dg_eval(const DgItem *__restrict
 	const int g = lane >> 2, t = lane & 3, wm = 32 * (warp & 1), wn = 32 * (warp >> 1);
 	const double *lam = S + it.lam;
 	const double alpha = dp.alphas[a];
-	const int K = min(min(md.tr_n, n), dg_rank(lam, p));
-	for (int k = tid; k < K; k += kDgThreads) cv[k] = 1.0 / (alpha + lam[k]);
+	const int K = p;  // at most min(rows, n), where the reference clips: the components past p are zero
+	for (int k = tid; k < K; k += kDgThreads) cv[k] = dg_coef(lam, p, k, alpha);
 	const DgSl sl = sls[it.sl];
 	double acc[2][4][4];
 	const double *Yt = S + it.yte;
@@ -463,7 +468,7 @@ __global__ void __launch_bounds__(kDgThreads) k_dg_beta(const DgItem *__restrict
 	for (int mo = 0; mo < dp.models; mo++) {
 		const DgItem it = items[sl.item0 + mo];
 		const double *lam = S + it.lam;
-		const int K = min(min(dp.mdl[mo].tr_n, n), dg_rank(lam, it.p));
+		const int K = it.p;
 		__syncthreads();
 		if (tid == 0) s_top = 0;
 		__syncthreads();
@@ -474,7 +479,7 @@ __global__ void __launch_bounds__(kDgThreads) k_dg_beta(const DgItem *__restrict
 				pc_chunk(dp.npcs, p, K, r0, r1);
 				mult += (k >= r0 && k < r1) ? 1 : 0;
 			}
-			cv[k] = mult ? (double)mult / (alpha + lam[k]) : 0.0;
+			cv[k] = mult ? (double)mult * dg_coef(lam, it.p, k, alpha) : 0.0;
 			if (mult) atomicMax(&s_top, k + 1);
 		}
 		__syncthreads();

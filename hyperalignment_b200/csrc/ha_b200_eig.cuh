@@ -24,9 +24,10 @@ constexpr int kEigSweeps = 8;    // QL sweeps applied together
 constexpr int kEigRounds = 2;    // QL launches; the second finishes what the first had no room for
 
 // One matrix.  A (p x p, the lower triangle is read, column-major) is overwritten by the eigenvectors, columns
-// in decreasing order of the eigenvalues; Q is p x p scratch; lam receives the eigenvalues.
-// Eigenvalues at or below p eps lambda_max are numerically zero: they are written as 0 and their
-// eigenvectors as zero columns.
+// in decreasing order of the eigenvalues; Q is p x p scratch; lam receives the eigenvalues, each with
+// an error of a few eps lambda_max (those of a singular matrix are rounding of either sign).  No
+// eigenvector is dropped for it: of X^T X, a singular value of X down to sqrt(eps) of the largest ends
+// there, and its component still counts for a ridge fit at a small penalty.
 struct EigWork {
 	int64_t a, q, s, lam;  // element offsets from the launch's four base pointers
 	int32_t p, pad_;
@@ -459,14 +460,10 @@ __global__ void __launch_bounds__(32) k_eig_ql(const EigWork *__restrict__ work,
 		__syncwarp();
 		ns++;
 	}
-	// eigenvalues in decreasing order (ties by index), numerically zero ones as 0
+	// eigenvalues in decreasing order (ties by index)
 	int *rank = reinterpret_cast<int *>(S + L.rank);
 	const bool last = !full || round == kEigRounds;
 	if (last) {
-		double mx = 0.0;
-		for (int i = lane; i < p; i += 32) mx = fmax(mx, d[i]);
-		for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-		const double zero = p * Eps<double>::v() * mx;
 		for (int i = lane; i < p; i += 32) {
 			const double x = d[i];
 			const double kx = isnan(x) ? INFINITY : x;  // NaN first, so that the ranks stay a permutation
@@ -475,9 +472,8 @@ __global__ void __launch_bounds__(32) k_eig_ql(const EigWork *__restrict__ work,
 				const double ky = isnan(d[o]) ? INFINITY : d[o];
 				k += (ky > kx || (ky == kx && o < i)) ? 1 : 0;
 			}
-			const bool null = x <= zero;
-			rank[i] = null ? -1 - k : k;
-			lamb[w.lam + k] = null ? 0.0 : x * scale;
+			rank[i] = k;
+			lamb[w.lam + k] = x * scale;
 		}
 	}
 	for (int i = lane; i < p; i += 32) {
@@ -586,10 +582,7 @@ __global__ void __launch_bounds__(32) k_eig_rotate(const EigWork *__restrict__ w
 	}
 	if (st.done != round || !own) return;
 	const int *rank = reinterpret_cast<const int *>(S + L.rank);
-	for (int c = 0; c < p; c++) {
-		const int k = rank[c];
-		A[(int64_t)(k < 0 ? -1 - k : k) * p + r0 + lane] = k < 0 ? 0.0 : z[(int64_t)c * p];
-	}
+	for (int c = 0; c < p; c++) A[(int64_t)rank[c] * p + r0 + lane] = z[(int64_t)c * p];
 }
 
 }  // namespace hab200

@@ -37,3 +37,30 @@ def test_eigen_solver_repeats_bit_for_bit(gpu):
     for r in runs[1:]:
         assert r.tobytes() == runs[0].tobytes()
     np.testing.assert_allclose(runs[0], O.ridge_features(X, idx, off, np.arange(nt)), rtol=0, atol=2.5e-7)
+
+
+# A float64 Gram matrix carries eps lambda_max, which a fit at penalty alpha feels as a few eps lambda_max /
+# alpha of its norm: with at most 300 rows of 130 unit columns (lambda_max about 2,000 where half of them repeat) and
+# alpha = 1e-3 some 1e-9 at worst.  The repository's bound for this search is 1e-8.
+@pytest.mark.parametrize("noise", [1e-5, 1e-7, 1e-9, 0.0])
+@pytest.mark.parametrize("nt,n", [(100, 100), (300, 130), (90, 130), (65, 64)])
+def test_nearly_repeated_columns_at_a_small_penalty(gpu, noise, nt, n):
+    """Columns that repeat others up to a little noise: singular values far below the largest, but above
+    the rounding of X, count for the fit and its predictions; exactly repeated ones give no noise."""
+    from hyperalignment_b200 import hyperalignment_c as H
+    rng = np.random.default_rng(nt + n)
+    ntot = nt + 40
+    X = rng.standard_normal((ntot, n))
+    X[:, n // 2:] = X[:, :n - n // 2] + noise * X[:, n // 2:]
+    Y = X @ (0.1 * rng.standard_normal((n, n))) + rng.standard_normal((ntot, n))
+    tr = [np.arange(nt, dtype=np.int32)]
+    te = [np.arange(nt, ntot, dtype=np.int32)]
+    sls = [np.arange(n, dtype=np.int32)]
+    indptr, indices = H.sparse_pattern(sls, n)
+    alphas, npcs = np.array([1e-3]), [n]
+    data = np.zeros(indices.size)
+    _, costs = H.searchlight_ridge_grid(X, Y, sls, indptr, indices, data, alphas, npcs, tr, te, return_costs=True)
+    ref, _, rcosts = O.searchlight_ridge_grid_csc(X, Y, sls[0], np.array([0, n]), indptr, indices, np.zeros(indices.size),
+                                                  alphas, npcs, tr, te, None)
+    np.testing.assert_allclose(costs, rcosts, rtol=1e-8, atol=0)
+    assert np.linalg.norm(data - ref) <= 1e-8 * np.linalg.norm(ref)
