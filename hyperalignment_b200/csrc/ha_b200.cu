@@ -1998,6 +1998,13 @@ __global__ void k_dg_flags(const EigWork *__restrict__ eig, const int32_t *__res
 // go to *fit.
 int dgrid_upload(HaB200Plan *P, const GridSpec &gs, cudaStream_t st, DgParams &dp, const int32_t *rows = nullptr,
                  int n_rows = 0, DgParams *fit = nullptr) {
+	// no capture by the caller: the lists are copied from host memory that is freed, which a replay would read
+	cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+	if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+		cudaGetLastError();
+		fprintf(stderr, "ha_b200: the float64 grid search cannot be captured on the caller's stream\n");
+		return kHaErrorInternal;
+	}
 	const int models = (int)gs.mdl.size();
 	std::vector<DgModel> mdl(models + (fit ? 1 : 0));
 	std::vector<int32_t> drow, terow, ovrow, ovptr, ovent;

@@ -64,3 +64,44 @@ def test_nearly_repeated_columns_at_a_small_penalty(gpu, noise, nt, n):
                                                   alphas, npcs, tr, te, None)
     np.testing.assert_allclose(costs, rcosts, rtol=1e-8, atol=0)
     assert np.linalg.norm(data - ref) <= 1e-8 * np.linalg.norm(ref)
+
+
+def test_grid_search_refuses_a_callers_stream_capture(gpu):
+    """The search uploads lists from host memory that it frees: captured into a caller's graph, a replay would read
+    freed memory.  The call fails instead (nothing is replayed here), and the plan works on afterwards."""
+    import ctypes
+    import torch
+    rng = np.random.default_rng(3)
+    n, nt = 20, 60
+    X, Y = rng.standard_normal((nt, n)), rng.standard_normal((nt, n))
+    plan = Plan(nt, n, np.arange(n), np.array([0, n]), weights=np.ones(n))
+    dX, dY = upload(X), upload(Y)
+    best = torch.zeros(1, dtype=torch.int32, device="cuda")
+    vals = torch.zeros(plan.nnz, dtype=torch.float64, device="cuda")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+
+    def run():
+        plan.ridge_grid_device(dX.data_ptr(), dY.data_ptr(), vals.data_ptr(), best.data_ptr(), [1.0, 10.0], [5, n],
+                               [np.arange(40)], [np.arange(40, nt)], stream=stream.cuda_stream)
+
+    run()
+    stream.synchronize()
+    first = vals.cpu().numpy()
+    rt = ctypes.CDLL("libcudart.so.12")
+    rt.cudaStreamBeginCapture.argtypes = [ctypes.c_void_p, ctypes.c_int]
+    rt.cudaStreamEndCapture.argtypes = [ctypes.c_void_p, ctypes.POINTER(ctypes.c_void_p)]
+    graph = ctypes.c_void_p()
+    assert rt.cudaStreamBeginCapture(stream.cuda_stream, 1) == 0  # thread-local mode
+    try:
+        with pytest.raises(RuntimeError):
+            run()
+    finally:
+        rt.cudaStreamEndCapture(stream.cuda_stream, ctypes.byref(graph))
+        rt.cudaGetLastError()
+    vals.zero_()
+    torch.cuda.synchronize()
+    run()
+    stream.synchronize()
+    assert vals.cpu().numpy().tobytes() == first.tobytes()
+    plan.close()
