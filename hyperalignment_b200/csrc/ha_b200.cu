@@ -302,17 +302,24 @@ int launch_eig(const EigWork *d_work, const std::vector<int> &orders, double *A,
 	return g_fan.end(st);
 }
 
+// Searchlights for the eigen solve by pivoted Cholesky and one-sided Jacobi, bucketed.
+struct EigItems {
+	std::vector<SlWork> work;
+	std::vector<Bucket> buckets;
+	SlWork *d = nullptr;
+};
+
 struct Chunk {
 	int s0, s1;
 	std::vector<SlWork> w32, w64;  // float32 polar, float64 polar
 	std::vector<Bucket> b32, b64;
-	std::vector<SlWork> weig32;  // float32 eigenvector mode (the plain FP32 grid search)
-	std::vector<Bucket> beig32;
+	EigItems eig32;  // the plain FP32 grid search
+	EigItems eig64;  // the float64 search's badly scaled searchlights are taken from it (built on first use, no device copy)
 	std::vector<int64_t> tofs;  // per slot
 	int64_t scratch_elems8;     // scratch size in 8-byte units (A and V each)
 	int64_t t_elems;            // T scratch floats
 	int64_t uv_elems;
-	SlWork *d_w32 = nullptr, *d_w64 = nullptr, *d_weig32 = nullptr;
+	SlWork *d_w32 = nullptr, *d_w64 = nullptr;
 	int64_t *d_tofs = nullptr;
 	// tensor-core solve: one work item per searchlight (slot order), 128-row tiles in two size
 	// classes (np <= 256: two CTAs per SM; np > 256), largest searchlights first
@@ -407,9 +414,11 @@ struct HaB200Plan {
 	DevArr<DgModel> dgmdl;
 	DevArr<int32_t> dgint;
 	DevArr<double> dgdbl, eigscr;
+	DevArr<double> dgnorm;     // squared column norms per model
+	DevArr<int32_t> dgscaled;  // per searchlight: badly scaled
 	DevArr<int32_t> gfit;      // fit rows of the learned form / the features
 	DevArr<float> gfeat;       // features of the learned form
-	DevArr<SlWork> gwork;      // fallback work list of the learned form
+	DevArr<SlWork> gwork;      // work list of a part of a chunk's searchlights
 	int last_chunk = -1;
 	int last_rowmajor = 1;
 };
@@ -546,8 +555,11 @@ int build_chunks(HaB200Plan *P) {
 			jacobi_layout(n, false, be32, ke32, me, fp32_jacobi_budget(), false);
 			int64_t e32 = ((int64_t)n * k32 * b32 * 4 + 7) / 8;
 			int64_t e64 = (int64_t)n * k64 * b64;
+			int be, ke;
+			jacobi_layout(n, true, be, ke, me, kSmemMax, false);
 			int64_t eeig32 = ((int64_t)n * ke32 * be32 * 4 + 7) / 8;
-			int64_t region = std::max<int64_t>(std::max(std::max(e32, e64), eeig32), (int64_t)n * n);
+			int64_t eeig = (int64_t)n * ke * be;
+			int64_t region = std::max<int64_t>(std::max(std::max(e32, e64), std::max(eeig, eeig32)), (int64_t)n * n);
 			region = (region + 31) & ~(int64_t)31;
 			size_t bytes_if = (size_t)(acc8 + region) * 8 * 2 + (size_t)(tacc + (int64_t)n * n) * 4;
 			if (!tofs.empty() && bytes_if > budget) break;
@@ -590,7 +602,7 @@ int build_chunks(HaB200Plan *P) {
 			std::vector<Bucket> buckets = bucketize(items, prec);
 			if (prec == 0) { ch.w32 = items; ch.b32 = buckets; }
 			else if (prec == 1) { ch.w64 = items; ch.b64 = buckets; }
-			else { ch.weig32 = items; ch.beig32 = buckets; }
+			else { ch.eig32.work = items; ch.eig32.buckets = buckets; }
 		}
 		P->chunks.push_back(std::move(ch));
 	}
@@ -599,8 +611,8 @@ int build_chunks(HaB200Plan *P) {
 		size_t n32 = ch.w32.size(), n64 = ch.w64.size();
 		if (cudaMalloc(&ch.d_w32, n32 * sizeof(SlWork)) != cudaSuccess) return kHaErrorAlloc;
 		if (cudaMalloc(&ch.d_w64, n64 * sizeof(SlWork)) != cudaSuccess) return kHaErrorAlloc;
-		if (cudaMalloc(&ch.d_weig32, ch.weig32.size() * sizeof(SlWork)) != cudaSuccess) return kHaErrorAlloc;
-		HA_CUDA(cudaMemcpy(ch.d_weig32, ch.weig32.data(), ch.weig32.size() * sizeof(SlWork), cudaMemcpyHostToDevice));
+		if (cudaMalloc(&ch.eig32.d, ch.eig32.work.size() * sizeof(SlWork)) != cudaSuccess) return kHaErrorAlloc;
+		HA_CUDA(cudaMemcpy(ch.eig32.d, ch.eig32.work.data(), ch.eig32.work.size() * sizeof(SlWork), cudaMemcpyHostToDevice));
 		if (cudaMalloc(&ch.d_tofs, ch.tofs.size() * sizeof(int64_t)) != cudaSuccess) return kHaErrorAlloc;
 		HA_CUDA(cudaMemcpy(ch.d_w32, ch.w32.data(), n32 * sizeof(SlWork), cudaMemcpyHostToDevice));
 		HA_CUDA(cudaMemcpy(ch.d_w64, ch.w64.data(), n64 * sizeof(SlWork), cudaMemcpyHostToDevice));
@@ -1895,23 +1907,56 @@ int reduce_chunk64(HaB200Plan *P, Chunk &ch, int out_kind, double *d_vals, cudaS
 	return kHaSuccess;
 }
 
-// The grid search of one chunk: per sub-batch of searchlights (bounded by the grid scratch budget)
-// and CV model, the Gram and cross-covariance over the model's training rows, the pivoted Cholesky
-// factor and its float64 Jacobi eigen decomposition, and the per-model products; then the grid
-// evaluation, the winners (d_best) and their betas in the float64 T scratch.  The chunk's work list
-// may be a subset of the plan chunk's (the learned form's fallback searchlights).
-// Sub-batches of a chunk's grid search: searchlights [i0, i1) of the eigenvector-mode work list,
-// as many as fit the grid scratch budget, and each one's per-slot scratch base offsets.
+// The float64 items of a chunk for the pivoted-Cholesky and Jacobi eigen solve.
+const EigItems &eig64_items(Chunk &ch) {
+	if (ch.eig64.work.empty()) {
+		ch.eig64.work = ch.w64;
+		for (SlWork &w : ch.eig64.work) {
+			size_t smem;
+			jacobi_layout(w.n, true, w.bsz, w.nblk, smem, kSmemMax, false);
+		}
+		ch.eig64.buckets = bucketize(ch.eig64.work, 3);
+	}
+	return ch.eig64;
+}
+
+// The items that `keep` takes, uploaded as a work list of their own (same buckets, same scratch slots).
+template <typename F>
+int eig_subset(HaB200Plan *P, const EigItems &all, F keep, EigItems &out, cudaStream_t st) {
+	out.work.clear();
+	out.buckets.clear();
+	for (const Bucket &b : all.buckets) {
+		Bucket nb = b;
+		nb.first = (int)out.work.size();
+		for (int i = b.first; i < b.first + b.count; i++)
+			if (keep(all.work[i])) out.work.push_back(all.work[i]);
+		nb.count = (int)out.work.size() - nb.first;
+		if (nb.count > 0) out.buckets.push_back(nb);
+	}
+	const int rc = upload_vec(P->gwork, out.work, st);
+	out.d = P->gwork.p;
+	return rc;
+}
+
+// The grid search of a chunk's searchlights by pivoted Cholesky and Jacobi eigen solves: per sub-batch of
+// searchlights (bounded by the grid scratch budget) and CV model, the Gram and cross-covariance over the
+// model's training rows, the pivoted Cholesky factor and its eigen decomposition, and the per-model
+// products; then the grid evaluation, the winners (d_best) and their betas in the float64 T scratch.
+// Real is the arithmetic: float for the plain FP32 search, double for the badly scaled searchlights of
+// the float64 one.  The items may be a part of the chunk's.
+// Sub-batches: items [i0, i1), as many as fit the grid scratch budget, and each one's per-slot scratch
+// base offsets.
 struct GridBatch {
 	int i0, i1;
-	int64_t total;  // float32 elements of grid scratch
+	int64_t total;  // elements of grid scratch
 };
 
-void grid_plan_chunk(const Chunk &ch, const GridParams &gp, std::vector<GridBatch> &bt, std::vector<int64_t> &gbase_all) {
-	const int nsl = ch.s1 - ch.s0;
+template <typename Real>
+void grid_plan_chunk(const EigItems &it, int nsl, const GridParams &gp, std::vector<GridBatch> &bt,
+                     std::vector<int64_t> &gbase_all) {
 	const int grid = gp.n_alphas * gp.n_npcs;
 	const size_t budget = grid_budget_bytes();
-	const std::vector<SlWork> &items = ch.weig32;
+	const std::vector<SlWork> &items = it.work;
 	const int nitems = (int)items.size();
 	bt.clear();
 	int i0 = 0;
@@ -1923,7 +1968,7 @@ void grid_plan_chunk(const Chunk &ch, const GridParams &gp, std::vector<GridBatc
 		while (i1 < nitems) {
 			const SlWork &wi = items[i1];
 			const GridLayout Lg = GridLayout::make(wi.n, gp.models, gp.mte, gp.ntu, gp.n_alphas, grid);
-			if (i1 > i0 && (size_t)(total + Lg.total) * sizeof(float) > budget) break;
+			if (i1 > i0 && (size_t)(total + Lg.total) * sizeof(Real) > budget) break;
 			gbase_all[g0 + wi.slot] = total;
 			total += Lg.total;
 			i1++;
@@ -1933,18 +1978,16 @@ void grid_plan_chunk(const Chunk &ch, const GridParams &gp, std::vector<GridBatc
 	}
 }
 
-// The launches of one chunk's plain FP32 grid search (no host copies or allocations: capturable);
-// the sub-batches' base offsets are at d_gbase (nsl per sub-batch).  The A / V / grid scratch are
-// read as float; the winners' betas still go to the float64 T scratch for the reduction.
-int grid_chunk_launch(HaB200Plan *P, Chunk &ch, const double *d_X, const double *d_Y, const GridSpec &gs,
+// The launches (no host copies or allocations: capturable); the sub-batches' base offsets are at d_gbase
+// (nsl per sub-batch).  The A / V / grid scratch are read as Real.
+template <typename Real>
+int grid_chunk_launch(HaB200Plan *P, const EigItems &it, int nsl, const double *d_X, const double *d_Y, const GridSpec &gs,
                       GridParams gp, const std::vector<GridBatch> &bt, const int64_t *d_gbase, int rowmajor,
                       int32_t *d_best, double *d_cost, cudaStream_t st) {
-	using Real = float;
+	constexpr bool f32 = sizeof(Real) == 4;
+	constexpr int kx = f32 ? kHaB200KXcov32 : kHaB200KXcov64, kj = f32 ? kHaB200KJacobi32 : kHaB200KJacobi64;
 	const int nt = P->nt;
-	const int nsl = ch.s1 - ch.s0;
 	const JacobiParams jp = eig_params(false);
-	const std::vector<Bucket> &beig = ch.beig32;
-	SlWork *d_work = ch.d_weig32;
 	Real *A = reinterpret_cast<Real *>(P->scrA.p), *V = reinterpret_cast<Real *>(P->scrV.p);
 	Real *G = reinterpret_cast<Real *>(P->gridscr.p);
 	int rc;
@@ -1955,30 +1998,47 @@ int grid_chunk_launch(HaB200Plan *P, Chunk &ch, const double *d_X, const double 
 			const GridModel &md = gs.mdl[mo];
 			const int32_t *tr = P->grows.p + md.tr_ofs;
 			if ((rc = g_fan.begin(st)) != kHaSuccess) return rc;
-			for (size_t bi = 0; bi < beig.size(); bi++) {
-				const Bucket &b = beig[bi];
+			for (size_t bi = 0; bi < it.buckets.size(); bi++) {
+				const Bucket &b = it.buckets[bi];
 				const int x0 = std::max(i0, b.first), x1 = std::min(i1, b.first + b.count);
 				if (x1 <= x0) continue;
 				const cudaStream_t bs = g_fan.at((int)bi);
-				const SlWork *wk = d_work + x0;
+				const SlWork *wk = it.d + x0;
 				// Gram into the V scratch, its pivoted Cholesky factor into the A scratch
-				{ HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<Real><<<dim3(x1 - x0, xrows_tiles(32 * b.rpl, 0)), kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_X, nt, tr, md.tr_n, V, G, gp, 0); }
-				{ HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<Real><<<dim3(x1 - x0, xrows_tiles(32 * b.rpl, 1)), kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_Y, nt, tr, md.tr_n, A, G, gp, 1); }
-				{ HA_LAUNCH(kHaB200KRidge, bs); k_pchol<Real><<<x1 - x0, kBlock, pchol_smem(b.rpl, sizeof(float)), bs>>>(wk, V, A, P->stats.p); }
+				{ HA_LAUNCH(kx, bs); k_xcov_rows<Real><<<dim3(x1 - x0, xrows_tiles(32 * b.rpl, 0)), kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_X, nt, tr, md.tr_n, V, G, gp, 0); }
+				{ HA_LAUNCH(kx, bs); k_xcov_rows<Real><<<dim3(x1 - x0, xrows_tiles(32 * b.rpl, 1)), kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_Y, nt, tr, md.tr_n, A, G, gp, 1); }
+				{ HA_LAUNCH(kHaB200KRidge, bs); k_pchol<Real><<<x1 - x0, kBlock, pchol_smem(b.rpl, sizeof(Real)), bs>>>(wk, V, A, P->stats.p); }
 				{
-					HA_LAUNCH(kHaB200KJacobi32, bs);
+					HA_LAUNCH(kj, bs);
 					if ((rc = launch_jacobi<Real>(b.rpl, x1 - x0, b.threads, b.smem, bs, wk, A, V, P->scrT.p, P->stats.p, P->uv.p, jp)) != kHaSuccess)
 						return rc;
 				}
 			}
 			if ((rc = g_fan.end(st)) != kHaSuccess) return rc;
-			{ HA_LAUNCH(kHaB200KGrid, st); k_grid_model<Real><<<i1 - i0, kBlock, 0, st>>>(d_work + i0, P->idx.p, d_X, d_Y, V, P->uv.p, mo, G, gp); }
+			{ HA_LAUNCH(kHaB200KGrid, st); k_grid_model<Real><<<i1 - i0, kBlock, 0, st>>>(it.d + i0, P->idx.p, d_X, d_Y, V, P->uv.p, mo, G, gp); }
 		}
-		{ HA_LAUNCH(kHaB200KGrid, st); k_grid_eval<Real><<<dim3(i1 - i0, gp.n_alphas), kBlock, 0, st>>>(d_work + i0, G, gp); }
-		{ HA_LAUNCH(kHaB200KGrid, st); k_grid_final<Real><<<i1 - i0, kBlock, 0, st>>>(d_work + i0, P->idx.p, d_Y, G, gp, P->scrT64.p, rowmajor, d_best, d_cost); }
+		{ HA_LAUNCH(kHaB200KGrid, st); k_grid_eval<Real><<<dim3(i1 - i0, gp.n_alphas), kBlock, 0, st>>>(it.d + i0, G, gp); }
+		{ HA_LAUNCH(kHaB200KGrid, st); k_grid_final<Real><<<i1 - i0, kBlock, 0, st>>>(it.d + i0, P->idx.p, d_Y, G, gp, P->scrT64.p, rowmajor, d_best, d_cost); }
 		HA_CUDA(cudaGetLastError());
 	}
 	return kHaSuccess;
+}
+
+// The same enqueued directly (sub-batch plan, scratch and offsets, launches).
+template <typename Real>
+int grid_chunk(HaB200Plan *P, const EigItems &it, int nsl, const double *d_X, const double *d_Y, const GridSpec &gs,
+               const GridParams &gp, int rowmajor, int32_t *d_best, double *d_cost, cudaStream_t st) {
+	std::vector<GridBatch> bt;
+	std::vector<int64_t> gbase;
+	grid_plan_chunk<Real>(it, nsl, gp, bt, gbase);
+	int64_t mx = 1;
+	for (const auto &b : bt) mx = std::max(mx, b.total);
+	int rc;
+	if ((rc = P->gridscr.ensure((size_t)mx)) != kHaSuccess) return rc;
+	if ((rc = P->gbase.ensure(std::max<size_t>(gbase.size(), 1))) != kHaSuccess) return rc;
+	HA_CUDA(cudaMemcpyAsync(P->gbase.p, gbase.data(), gbase.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+	HA_CUDA(cudaStreamSynchronize(st));  // the host vector goes out of scope
+	return grid_chunk_launch<Real>(P, it, nsl, d_X, d_Y, gs, gp, bt, P->gbase.p, rowmajor, d_best, d_cost, st);
 }
 
 // ---- float64 grid search (ha_b200_dgrid.cuh) ----
@@ -2093,6 +2153,24 @@ int dgrid_upload(HaB200Plan *P, const GridSpec &gs, cudaStream_t st, DgParams &d
 		fit->nov = fit->entries = fit->n_untested = 0;
 	}
 	P->dg_models = std::move(mdl);
+	return kHaSuccess;
+}
+
+// Per searchlight whether its columns are badly scaled over the rows of some model (k_dg_scaled): those go
+// the way of pivoted Cholesky and Jacobi.  Waits for the stream.
+int dgrid_scaled(HaB200Plan *P, const double *d_X, const DgParams &dp, std::vector<int32_t> &scaled, cudaStream_t st) {
+	int rc;
+	if ((rc = P->dgnorm.ensure((size_t)P->nv * dp.models)) != kHaSuccess) return rc;
+	if ((rc = P->dgscaled.ensure((size_t)P->count)) != kHaSuccess) return rc;
+	for (int m = 0; m < dp.models; m += 65535) {
+		HA_LAUNCH(kHaB200KGrid, st);
+		k_dg_norms<<<dim3((P->nv + 7) / 8, std::min(dp.models - m, 65535)), kBlock, 0, st>>>(d_X, P->nv, dp, m, P->dgnorm.p);
+	}
+	{ HA_LAUNCH(kHaB200KGrid, st); k_dg_scaled<<<(P->count + 7) / 8, kBlock, 0, st>>>(P->off.p, P->idx.p, P->count, P->nv, dp.models, P->dgnorm.p, P->dgscaled.p); }
+	HA_CUDA(cudaGetLastError());
+	scaled.resize((size_t)P->count);
+	HA_CUDA(cudaMemcpyAsync(scaled.data(), P->dgscaled.p, scaled.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+	HA_CUDA(cudaStreamSynchronize(st));
 	return kHaSuccess;
 }
 
@@ -2263,10 +2341,11 @@ int dgrid_factor(HaB200Plan *P, const DgPlan &pl, const DgBatch &b, const double
 	});
 }
 
-// The float64 grid search of the searchlights `work` (slots of the current chunk): betas to the
-// float64 T scratch, winners and costs to d_best / d_cost.
-int dgrid_run(HaB200Plan *P, const std::vector<SlWork> &work, const double *d_X, const double *d_Y, const DgParams &dp,
+// The float64 grid search of the searchlights `work` (slots of the current chunk) by tile products: betas
+// to the float64 T scratch, winners and costs to d_best / d_cost.
+int dgrid_tiles(HaB200Plan *P, const std::vector<SlWork> &work, const double *d_X, const double *d_Y, const DgParams &dp,
               int rowmajor, int32_t *d_best, double *d_cost, cudaStream_t st) {
+	if (work.empty()) return kHaSuccess;
 	DgPlan pl;
 	int rc = dgrid_plan(P, work, dp, pl, st);
 	if (rc != kHaSuccess) return rc;
@@ -2290,20 +2369,25 @@ int dgrid_run(HaB200Plan *P, const std::vector<SlWork> &work, const double *d_X,
 	return kHaSuccess;
 }
 
-// One chunk's plain FP32 grid search enqueued directly (sub-batch plan, scratch and offsets, launches).
-int grid_chunk32(HaB200Plan *P, Chunk &ch, const double *d_X, const double *d_Y, const GridSpec &gs,
-                 const GridParams &gp, int rowmajor, int32_t *d_best, double *d_cost, cudaStream_t st) {
-	std::vector<GridBatch> bt;
-	std::vector<int64_t> gbase;
-	grid_plan_chunk(ch, gp, bt, gbase);
-	int64_t mx = 1;
-	for (const auto &b : bt) mx = std::max(mx, b.total);
-	int rc;
-	if ((rc = P->gridscr.ensure((size_t)mx)) != kHaSuccess) return rc;
-	if ((rc = P->gbase.ensure(std::max<size_t>(gbase.size(), 1))) != kHaSuccess) return rc;
-	HA_CUDA(cudaMemcpyAsync(P->gbase.p, gbase.data(), gbase.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-	HA_CUDA(cudaStreamSynchronize(st));  // the host vector goes out of scope
-	return grid_chunk_launch(P, ch, d_X, d_Y, gs, gp, bt, P->gbase.p, rowmajor, d_best, d_cost, st);
+// The float64 grid search of the searchlights of a chunk that `take` takes: by tile products, the badly
+// scaled ones by pivoted Cholesky and Jacobi.
+template <typename F>
+int dgrid_run(HaB200Plan *P, Chunk &ch, F take, const std::vector<int32_t> &scaled, const double *d_X, const double *d_Y,
+              const GridSpec &gs, const DgParams &dp, int rowmajor, int32_t *d_best, double *d_cost, cudaStream_t st) {
+	std::vector<SlWork> fw;
+	bool general = false;
+	for (const SlWork &w : ch.w64)
+		if (take(w)) {
+			if (scaled[w.s]) general = true;
+			else fw.push_back(w);
+		}
+	int rc = dgrid_tiles(P, fw, d_X, d_Y, dp, rowmajor, d_best, d_cost, st);
+	if (rc != kHaSuccess || !general) return rc;
+	EigItems it;
+	if ((rc = eig_subset(P, eig64_items(ch), [&](const SlWork &w) { return take(w) && scaled[w.s]; }, it, st)) != kHaSuccess) return rc;
+	GridParams gp;
+	if ((rc = grid_upload(P, gs, st, gp)) != kHaSuccess) return rc;
+	return grid_chunk<double>(P, it, ch.s1 - ch.s0, d_X, d_Y, gs, gp, rowmajor, d_best, d_cost, st);
 }
 
 int run_ridge_grid(HaB200Plan *P, const double *d_X, const double *d_Y, const GridSpec &gs, int out_kind,
@@ -2315,10 +2399,13 @@ int run_ridge_grid(HaB200Plan *P, const double *d_X, const double *d_Y, const Gr
 	if (!fp32) {
 		DgParams dp;
 		if ((rc = dgrid_upload(P, gs, st, dp)) != kHaSuccess) return rc;
+		std::vector<int32_t> scaled;
+		if ((rc = dgrid_scaled(P, d_X, dp, scaled, st)) != kHaSuccess) return rc;
 		HA_CUDA(cudaMemsetAsync(P->counters.p, 0, 5 * sizeof(int32_t), st));
 		for (Chunk &ch : P->chunks) {
 			HA_CUDA(cudaMemsetAsync(P->stats.p, 0, (size_t)(ch.s1 - ch.s0) * sizeof(SlStats), st));
-			if ((rc = dgrid_run(P, ch.w64, d_X, d_Y, dp, rowmajor, d_best, d_cost, st)) != kHaSuccess) return rc;
+			if ((rc = dgrid_run(P, ch, [](const SlWork &) { return true; }, scaled, d_X, d_Y, gs, dp, rowmajor, d_best, d_cost, st)) != kHaSuccess)
+				return rc;
 			if ((rc = reduce_chunk64(P, ch, out_kind, d_vals, st)) != kHaSuccess) return rc;
 		}
 		P->last_chunk = (int)P->chunks.size() - 1;
@@ -2336,7 +2423,7 @@ int run_ridge_grid(HaB200Plan *P, const double *d_X, const double *d_Y, const Gr
 	int64_t mx = 1;
 	for (size_t c = 0; c < P->chunks.size(); c++) {
 		gofs[c] = gbase.size();
-		grid_plan_chunk(P->chunks[c], gp, bts[c], gbase);
+		grid_plan_chunk<float>(P->chunks[c].eig32, P->chunks[c].s1 - P->chunks[c].s0, gp, bts[c], gbase);
 		for (const auto &b : bts[c]) mx = std::max(mx, b.total);
 	}
 	if ((rc = P->gridscr.ensure((size_t)mx)) != kHaSuccess) return rc;
@@ -2348,7 +2435,8 @@ int run_ridge_grid(HaB200Plan *P, const double *d_X, const double *d_Y, const Gr
 		for (size_t c = 0; c < P->chunks.size(); c++) {
 			Chunk &ch = P->chunks[c];
 			HA_CUDA(cudaMemsetAsync(P->stats.p, 0, (size_t)(ch.s1 - ch.s0) * sizeof(SlStats), ls));
-			int r = grid_chunk_launch(P, ch, d_X, d_Y, gs, gp, bts[c], P->gbase.p + gofs[c], rowmajor, d_best, d_cost, ls);
+			int r = grid_chunk_launch<float>(P, ch.eig32, ch.s1 - ch.s0, d_X, d_Y, gs, gp, bts[c], P->gbase.p + gofs[c], rowmajor,
+			                                 d_best, d_cost, ls);
 			if (r != kHaSuccess) return r;
 			if ((r = reduce_chunk64(P, ch, out_kind, d_vals, ls)) != kHaSuccess) return r;
 		}
@@ -2406,32 +2494,51 @@ int run_ridge_grid(HaB200Plan *P, const double *d_X, const double *d_Y, const Gr
 	return kHaSuccess;
 }
 
-// Plain FP32 eigen decomposition of every searchlight's Gram over the given rows (device list, n_rows
-// entries): the pivoted Cholesky factor and the eigenvector-mode Jacobi leave the eigenvectors in
-// the V scratch and the eigenvalues in the u/v buffer; with d_Y, C = X^T Y over the same rows goes
-// to the float32 T scratch.  Then the features of the chunk's searchlights.
-int eigen_chunk32(HaB200Plan *P, Chunk &ch, const double *d_X, const double *d_Y, const int32_t *d_rows, int n_rows,
-                  float *d_feat, cudaStream_t st) {
+// Eigen decomposition of the items' Grams over the given rows (device list, n_rows entries) in Real: the
+// pivoted Cholesky factor and the eigenvector-mode Jacobi leave the eigenvectors in the V scratch and
+// the eigenvalues in the u/v buffer; with d_Y, C = X^T Y over the same rows goes to the T scratch of
+// the arithmetic.  Then the items' features.
+template <typename Real>
+int eigen_chunk(HaB200Plan *P, const EigItems &it, const double *d_X, const double *d_Y, const int32_t *d_rows, int n_rows,
+                float *d_feat, cudaStream_t st) {
+	constexpr bool f32 = sizeof(Real) == 4;
+	constexpr int kx = f32 ? kHaB200KXcov32 : kHaB200KXcov64, kj = f32 ? kHaB200KJacobi32 : kHaB200KJacobi64;
 	GridParams gp = {};
 	const JacobiParams jp = eig_params(false);
-	float *A = reinterpret_cast<float *>(P->scrA.p), *V = reinterpret_cast<float *>(P->scrV.p);
+	Real *A = reinterpret_cast<Real *>(P->scrA.p), *V = reinterpret_cast<Real *>(P->scrV.p);
+	Real *Cs = f32 ? reinterpret_cast<Real *>(P->scrT.p) : reinterpret_cast<Real *>(P->scrT64.p);
 	int rc;
 	if ((rc = g_fan.begin(st)) != kHaSuccess) return rc;
-	for (size_t bi = 0; bi < ch.beig32.size(); bi++) {
-		const Bucket &b = ch.beig32[bi];
+	for (size_t bi = 0; bi < it.buckets.size(); bi++) {
+		const Bucket &b = it.buckets[bi];
 		const cudaStream_t bs = g_fan.at((int)bi);
-		const SlWork *wk = ch.d_weig32 + b.first;
-		{ HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<float><<<dim3(b.count, xrows_tiles(32 * b.rpl, 0)), kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_X, P->nt, d_rows, n_rows, V, nullptr, gp, 0); }
-		if (d_Y) { HA_LAUNCH(kHaB200KXcov32, bs); k_xcov_rows<float><<<dim3(b.count, xrows_tiles(32 * b.rpl, 2)), kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_Y, P->nt, d_rows, n_rows, P->scrT.p, nullptr, gp, 2); }
-		{ HA_LAUNCH(kHaB200KRidge, bs); k_pchol<float><<<b.count, kBlock, pchol_smem(b.rpl, sizeof(float)), bs>>>(wk, V, A, P->stats.p); }
+		const SlWork *wk = it.d + b.first;
+		{ HA_LAUNCH(kx, bs); k_xcov_rows<Real><<<dim3(b.count, xrows_tiles(32 * b.rpl, 0)), kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_X, P->nt, d_rows, n_rows, V, nullptr, gp, 0); }
+		if (d_Y) { HA_LAUNCH(kx, bs); k_xcov_rows<Real><<<dim3(b.count, xrows_tiles(32 * b.rpl, 2)), kBlock, 0, bs>>>(wk, P->idx.p, d_X, d_Y, P->nt, d_rows, n_rows, Cs, nullptr, gp, 2); }
+		{ HA_LAUNCH(kHaB200KRidge, bs); k_pchol<Real><<<b.count, kBlock, pchol_smem(b.rpl, sizeof(Real)), bs>>>(wk, V, A, P->stats.p); }
 		{
-			HA_LAUNCH(kHaB200KJacobi32, bs);
-			if ((rc = launch_jacobi<float>(b.rpl, b.count, b.threads, b.smem, bs, wk, A, V, P->scrT.p, P->stats.p, P->uv.p, jp)) != kHaSuccess)
+			HA_LAUNCH(kj, bs);
+			if ((rc = launch_jacobi<Real>(b.rpl, b.count, b.threads, b.smem, bs, wk, A, V, P->scrT.p, P->stats.p, P->uv.p, jp)) != kHaSuccess)
 				return rc;
 		}
 	}
 	if ((rc = g_fan.end(st)) != kHaSuccess) return rc;
-	{ HA_LAUNCH(kHaB200KGrid, st); k_features<<<(int)ch.weig32.size(), kBlock, 0, st>>>(ch.d_weig32, P->uv.p, d_feat); }
+	{ HA_LAUNCH(kHaB200KGrid, st); k_features<<<(int)it.work.size(), kBlock, 0, st>>>(it.d, P->uv.p, d_feat); }
+	HA_CUDA(cudaGetLastError());
+	return kHaSuccess;
+}
+
+// Betas of the items whose proposal has at least min_prob, from what eigen_chunk left.
+template <typename Real>
+int proposed_chunk(HaB200Plan *P, const EigItems &it, const int32_t *d_choice, const float *d_prob, float min_prob,
+                   const double *d_alphas, const int32_t *d_npcs, int n_npcs, int n_rows, int rowmajor, cudaStream_t st) {
+	constexpr bool f32 = sizeof(Real) == 4;
+	const Real *V = reinterpret_cast<const Real *>(P->scrV.p);
+	Real *Q = reinterpret_cast<Real *>(P->scrA.p);
+	const Real *Cs = f32 ? reinterpret_cast<const Real *>(P->scrT.p) : reinterpret_cast<const Real *>(P->scrT64.p);
+	const dim3 grid((unsigned)it.work.size(), kProposedParts);
+	{ HA_LAUNCH(kHaB200KGrid, st); k_proposed_q<Real><<<grid, kBlock, 0, st>>>(it.d, V, Q, Cs, d_prob, min_prob); }
+	{ HA_LAUNCH(kHaB200KGrid, st); k_proposed_beta<Real><<<grid, kBlock, 0, st>>>(it.d, V, P->uv.p, Q, P->scrT64.p, d_choice, d_prob, min_prob, d_alphas, d_npcs, n_npcs, n_rows, rowmajor); }
 	HA_CUDA(cudaGetLastError());
 	return kHaSuccess;
 }
@@ -2447,6 +2554,16 @@ int upload_rows(HaB200Plan *P, const int32_t *rows, int n_rows, cudaStream_t st)
 	return kHaSuccess;
 }
 
+// A chunk's searchlights for the tile products, and the badly scaled ones.
+int dgrid_split(HaB200Plan *P, Chunk &ch, const std::vector<int32_t> &scaled, std::vector<SlWork> &tiles, EigItems &general,
+                cudaStream_t st) {
+	tiles.clear();
+	for (const SlWork &w : ch.w64)
+		if (!scaled[w.s]) tiles.push_back(w);
+	if (tiles.size() == ch.w64.size()) return kHaSuccess;
+	return eig_subset(P, eig64_items(ch), [&](const SlWork &w) { return scaled[w.s] != 0; }, general, st);
+}
+
 // Features of every searchlight over the given rows (no fit).
 int run_ridge_features(HaB200Plan *P, const double *d_X, const int32_t *rows, int n_rows, float *d_feat,
                        cudaStream_t st) {
@@ -2454,16 +2571,23 @@ int run_ridge_features(HaB200Plan *P, const double *d_X, const int32_t *rows, in
 	if ((rc = grid_prepare(P)) != kHaSuccess) return rc;
 	if ((rc = upload_rows(P, rows, n_rows, st)) != kHaSuccess) return rc;
 	DgParams dp, fit;
-	if (P->grid_bits != 32 && (rc = dgrid_upload(P, GridSpec(), st, dp, rows, n_rows, &fit)) != kHaSuccess) return rc;
+	std::vector<int32_t> scaled;
+	if (P->grid_bits != 32 && ((rc = dgrid_upload(P, GridSpec(), st, dp, rows, n_rows, &fit)) != kHaSuccess ||
+	                           (rc = dgrid_scaled(P, d_X, fit, scaled, st)) != kHaSuccess))
+		return rc;
 	for (size_t c = 0; c < P->chunks.size(); c++) {
 		Chunk &ch = P->chunks[c];
 		HA_CUDA(cudaMemsetAsync(P->stats.p, 0, (size_t)(ch.s1 - ch.s0) * sizeof(SlStats), st));
 		if (P->grid_bits == 32) {
-			if ((rc = eigen_chunk32(P, ch, d_X, nullptr, P->gfit.p, n_rows, d_feat, st)) != kHaSuccess) return rc;
+			if ((rc = eigen_chunk<float>(P, ch.eig32, d_X, nullptr, P->gfit.p, n_rows, d_feat, st)) != kHaSuccess) return rc;
 			continue;
 		}
+		EigItems gen;
+		std::vector<SlWork> fw;
+		if ((rc = dgrid_split(P, ch, scaled, fw, gen, st)) != kHaSuccess) return rc;
+		if (!gen.work.empty() && (rc = eigen_chunk<double>(P, gen, d_X, nullptr, P->gfit.p, n_rows, d_feat, st)) != kHaSuccess) return rc;
 		DgPlan pl;
-		if ((rc = dgrid_plan(P, ch.w64, fit, pl, st)) != kHaSuccess) return rc;
+		if (!fw.empty() && (rc = dgrid_plan(P, fw, fit, pl, st)) != kHaSuccess) return rc;
 		for (const DgBatch &b : pl.batches) {
 			if ((rc = dgrid_factor(P, pl, b, d_X, nullptr, fit, st)) != kHaSuccess) return rc;
 			HA_LAUNCH(kHaB200KGrid, st);
@@ -2490,7 +2614,11 @@ int run_ridge_learned(HaB200Plan *P, const double *d_X, const double *d_Y, const
 	GridParams gp;
 	DgParams dp, fit;
 	if (fp32 && (rc = grid_upload(P, gs, st, gp)) != kHaSuccess) return rc;
-	if (!fp32 && (rc = dgrid_upload(P, gs, st, dp, rows, n_rows, &fit)) != kHaSuccess) return rc;
+	std::vector<int32_t> scaled, fit_scaled;  // over the rows of the CV models, over the fit rows
+	if (!fp32 && ((rc = dgrid_upload(P, gs, st, dp, rows, n_rows, &fit)) != kHaSuccess ||
+	              (rc = dgrid_scaled(P, d_X, dp, scaled, st)) != kHaSuccess ||
+	              (rc = dgrid_scaled(P, d_X, fit, fit_scaled, st)) != kHaSuccess))
+		return rc;
 	const size_t nfeat = (size_t)P->count * (kFeatSv + 1);
 	if ((rc = P->gfeat.ensure(nfeat)) != kHaSuccess) return rc;
 	HA_CUDA(cudaMemsetAsync(P->gfeat.p, 0, nfeat * sizeof(float), st));
@@ -2505,18 +2633,24 @@ int run_ridge_learned(HaB200Plan *P, const double *d_X, const double *d_Y, const
 			                         d_prob + ch.s0, st);
 		};
 		if (fp32) {
-			if ((rc = eigen_chunk32(P, ch, d_X, d_Y, P->gfit.p, n_rows, P->gfeat.p, st)) != kHaSuccess) return rc;
+			if ((rc = eigen_chunk<float>(P, ch.eig32, d_X, d_Y, P->gfit.p, n_rows, P->gfeat.p, st)) != kHaSuccess) return rc;
 			if ((rc = propose()) != kHaSuccess) return rc;
-			const float *V = reinterpret_cast<const float *>(P->scrV.p);
-			float *Q = reinterpret_cast<float *>(P->scrA.p);
-			const dim3 grid((unsigned)ch.weig32.size(), kProposedParts);
-			{ HA_LAUNCH(kHaB200KGrid, st); k_proposed_q<float><<<grid, kBlock, 0, st>>>(ch.d_weig32, V, Q, P->scrT.p, d_prob, min_prob); }
-			{ HA_LAUNCH(kHaB200KGrid, st); k_proposed_beta<float><<<grid, kBlock, 0, st>>>(ch.d_weig32, V, P->uv.p, Q, P->scrT64.p, d_choice, d_prob, min_prob, gp.alphas, gp.npcs, gp.n_npcs, n_rows, rowmajor); }
+			if ((rc = proposed_chunk<float>(P, ch.eig32, d_choice, d_prob, min_prob, gp.alphas, gp.npcs, gp.n_npcs, n_rows, rowmajor, st)) != kHaSuccess)
+				return rc;
 		} else {
 			// a batch's factors are at hand only until the next one's: the proposals are taken after every
 			// batch (those of searchlights without features yet are overwritten later)
+			EigItems gen;
+			std::vector<SlWork> fw;
+			if ((rc = dgrid_split(P, ch, fit_scaled, fw, gen, st)) != kHaSuccess) return rc;
+			if (!gen.work.empty()) {
+				if ((rc = eigen_chunk<double>(P, gen, d_X, d_Y, P->gfit.p, n_rows, P->gfeat.p, st)) != kHaSuccess) return rc;
+				if ((rc = propose()) != kHaSuccess) return rc;
+				if ((rc = proposed_chunk<double>(P, gen, d_choice, d_prob, min_prob, fit.alphas, fit.npcs, fit.n_npcs, n_rows, rowmajor, st)) != kHaSuccess)
+					return rc;
+			}
 			DgPlan pl;
-			if ((rc = dgrid_plan(P, ch.w64, fit, pl, st)) != kHaSuccess) return rc;
+			if (!fw.empty() && (rc = dgrid_plan(P, fw, fit, pl, st)) != kHaSuccess) return rc;
 			for (const DgBatch &b : pl.batches) {
 				if ((rc = dgrid_factor(P, pl, b, d_X, d_Y, fit, st)) != kHaSuccess) return rc;
 				const DgItem *it = P->dgitem.p + b.sl0;
@@ -2535,31 +2669,14 @@ int run_ridge_learned(HaB200Plan *P, const double *d_X, const double *d_Y, const
 		hprob.resize((size_t)nsl);
 		HA_CUDA(cudaMemcpyAsync(hprob.data(), d_prob + ch.s0, (size_t)nsl * 4, cudaMemcpyDeviceToHost, st));
 		HA_CUDA(cudaStreamSynchronize(st));
-		// the fallback searchlights as a work list of their own (same scratch slots)
 		auto below = [&](const SlWork &w) { return hprob[(size_t)(w.s - ch.s0)] < min_prob; };
 		if (fp32) {
-			Chunk fb;  // same buckets
-			fb.s0 = ch.s0;
-			fb.s1 = ch.s1;
-			for (const Bucket &b : ch.beig32) {
-				Bucket nb = b;
-				nb.first = (int)fb.weig32.size();
-				for (int i = b.first; i < b.first + b.count; i++)
-					if (below(ch.weig32[i])) fb.weig32.push_back(ch.weig32[i]);
-				nb.count = (int)fb.weig32.size() - nb.first;
-				if (nb.count > 0) fb.beig32.push_back(nb);
-			}
-			if (!fb.weig32.empty()) {
-				if ((rc = P->gwork.ensure(fb.weig32.size())) != kHaSuccess) return rc;
-				HA_CUDA(cudaMemcpyAsync(P->gwork.p, fb.weig32.data(), fb.weig32.size() * sizeof(SlWork), cudaMemcpyHostToDevice, st));
-				fb.d_weig32 = P->gwork.p;
-				if ((rc = grid_chunk32(P, fb, d_X, d_Y, gs, gp, rowmajor, d_choice, nullptr, st)) != kHaSuccess) return rc;
-			}
-		} else {
-			std::vector<SlWork> fw;
-			for (const SlWork &w : ch.w64)
-				if (below(w)) fw.push_back(w);
-			if (!fw.empty() && (rc = dgrid_run(P, fw, d_X, d_Y, dp, rowmajor, d_choice, nullptr, st)) != kHaSuccess) return rc;
+			EigItems fb;
+			if ((rc = eig_subset(P, ch.eig32, below, fb, st)) != kHaSuccess) return rc;
+			if (!fb.work.empty() && (rc = grid_chunk<float>(P, fb, nsl, d_X, d_Y, gs, gp, rowmajor, d_choice, nullptr, st)) != kHaSuccess)
+				return rc;
+		} else if ((rc = dgrid_run(P, ch, below, scaled, d_X, d_Y, gs, dp, rowmajor, d_choice, nullptr, st)) != kHaSuccess) {
+			return rc;
 		}
 		if ((rc = reduce_chunk64(P, ch, out_kind, d_vals, st)) != kHaSuccess) return rc;
 	}
@@ -3360,7 +3477,7 @@ void ha_b200_plan_destroy(HaB200Plan *P) {
 	for (auto &ch : P->chunks) {
 		if (ch.d_w32) cudaFree(ch.d_w32);
 		if (ch.d_w64) cudaFree(ch.d_w64);
-		if (ch.d_weig32) cudaFree(ch.d_weig32);
+		if (ch.eig32.d) cudaFree(ch.eig32.d);
 		if (ch.d_tofs) cudaFree(ch.d_tofs);
 		if (ch.d_tclists) cudaFree(ch.d_tclists);
 		if (ch.tc_graph) cudaGraphExecDestroy(ch.tc_graph);
@@ -3373,7 +3490,7 @@ void ha_b200_plan_destroy(HaB200Plan *P) {
 	P->grows.release(); P->gtpos.release(); P->gurows.release(); P->guntested.release(); P->gmdl.release();
 	P->gfit.release(); P->gfeat.release(); P->gwork.release();
 	P->dgitem.release(); P->dgsl.release(); P->dgeig.release(); P->dgslot.release(); P->dgmdl.release();
-	P->dgint.release(); P->dgdbl.release(); P->eigscr.release();
+	P->dgint.release(); P->dgdbl.release(); P->eigscr.release(); P->dgnorm.release(); P->dgscaled.release();
 	P->tcXb.release(); P->tcYb.release(); P->tcXp.release(); P->tcXq.release(); P->tcPp.release(); P->tcA.release(); P->tcRes.release();
 	P->tcSt.release(); P->tcSched.release(); P->tcPlain.release(); P->tcQueue.release();
 	if (P->grid_graph) cudaGraphExecDestroy(P->grid_graph);

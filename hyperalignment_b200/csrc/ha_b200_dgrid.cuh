@@ -77,6 +77,58 @@ struct DgSl {
 	int32_t sofs, pad_;
 };
 
+// Squared norms of X's columns over the distinct training rows of models m0, m0 + 1, .. (with their
+// multiplicities), a warp a (vertex, model).
+__global__ void __launch_bounds__(256) k_dg_norms(const double *__restrict__ X, int nv, const DgParams dp, int m0,
+                                                  double *__restrict__ norms) {
+	const int v = (int)blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, m = m0 + (int)blockIdx.y;
+	if (v >= nv) return;
+	const DgModel md = dp.mdl[m];
+	const double *x = X + (int64_t)v * dp.nt;
+	double s = 0.0;
+	for (int t = lane; t < md.d_n; t += 32) {
+		const double y = dp.dsq[md.d_ofs + t] * x[dp.drow[md.d_ofs + t]];
+		s = fma(y, y, s);
+	}
+	s = warp_sum(s);
+	if (lane == 0) norms[(int64_t)m * nv + v] = s;
+}
+
+// Whether the nonzero columns of a searchlight differ in norm by more than kDgMaxScale over the rows of some
+// model, or are not finite, a warp a searchlight.  The tridiagonal reduction's error is eps ||G||, whatever
+// a column's own size, and the kernel matrix keeps no column scale at all, so both lose the square of the
+// ratio; pivoted Cholesky and one-sided Jacobi are accurate relative to every column and take such
+// searchlights.  Error of beta at alpha = 1e-3, tile products / Jacobi, median over ten draws of 120 x 60,
+// 60 x 120 and 100 x 100 with some columns scaled by r: 3.9e-15 / 1.1e-14, 3.6e-15 / 1.2e-14 and 4.1e-12 /
+// 2.5e-12 at r = 1; 3.1e-14 / 2.2e-14, 2.7e-14 / 2.0e-14 and 8.1e-12 / 1.2e-12 at 8; 8.1e-13 / 9.0e-14, 3.8e-13 /
+// 6.2e-14 and 1.7e-10 / 9.4e-12 at 32; at 1e4 up to 1e-4 / 2e-8.  z-scored series lie below 2 over the rows of
+// a bootstrap and series with a standard deviation of 1.02-6.1 over the sphere below 6.1; the way by Jacobi
+// takes nine times as long (512 searchlights of 50-500 vertices: 835 against 89 ms).
+constexpr double kDgMaxScale = 8.0;
+__global__ void __launch_bounds__(256) k_dg_scaled(const int32_t *__restrict__ off, const int32_t *__restrict__ sl_idx, int count,
+                                                   int nv, int models, const double *__restrict__ norms,
+                                                   int32_t *__restrict__ scaled) {
+	const int s = (int)blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+	if (s >= count) return;
+	bool bad = false;
+	for (int m = 0; m < models; m++) {
+		double mn = INFINITY, mx = 0.0;
+		for (int i = off[s] + lane; i < off[s + 1]; i += 32) {
+			const double x = norms[(int64_t)m * nv + sl_idx[i]];
+			if (x > 0.0) mn = fmin(mn, x);
+			mx = fmax(mx, x);
+			bad = bad || !isfinite(x);
+		}
+		for (int o = 16; o > 0; o >>= 1) {
+			mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+			mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+		}
+		bad = bad || mx > kDgMaxScale * kDgMaxScale * mn;
+	}
+	bad = __any_sync(0xffffffffu, bad);
+	if (lane == 0) scaled[s] = bad ? 1 : 0;
+}
+
 // Gathered rows of one item (Y may be null when there are no test rows): the distinct training rows of X and Y, the test rows of X and Y, and (by
 // the first model's CTA) the targets of the several-model rows.
 __global__ void __launch_bounds__(256) k_dg_gather(const DgItem *__restrict__ items, const DgSl *__restrict__ sls,
