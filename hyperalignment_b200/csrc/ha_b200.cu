@@ -2157,15 +2157,17 @@ int dgrid_upload(HaB200Plan *P, const GridSpec &gs, cudaStream_t st, DgParams &d
 }
 
 // Per searchlight whether its columns are badly scaled over the rows of some model (k_dg_scaled): those go
-// the way of pivoted Cholesky and Jacobi.  Waits for the stream.
+// the way of pivoted Cholesky and Jacobi.  So does everything whose models or several-model rows would not fit
+// the grid of one launch of the tile products.  Waits for the stream.
 int dgrid_scaled(HaB200Plan *P, const double *d_X, const DgParams &dp, std::vector<int32_t> &scaled, cudaStream_t st) {
+	if (dp.models > 65535 || (dp.nov + kDgRows - 1) / kDgRows > 65535) {
+		scaled.assign((size_t)P->count, 1);
+		return kHaSuccess;
+	}
 	int rc;
 	if ((rc = P->dgnorm.ensure((size_t)P->nv * dp.models)) != kHaSuccess) return rc;
 	if ((rc = P->dgscaled.ensure((size_t)P->count)) != kHaSuccess) return rc;
-	for (int m = 0; m < dp.models; m += 65535) {
-		HA_LAUNCH(kHaB200KGrid, st);
-		k_dg_norms<<<dim3((P->nv + 7) / 8, std::min(dp.models - m, 65535)), kBlock, 0, st>>>(d_X, P->nv, dp, m, P->dgnorm.p);
-	}
+	if (dp.models) { HA_LAUNCH(kHaB200KGrid, st); k_dg_norms<<<dim3((P->nv + 7) / 8, dp.models), kBlock, 0, st>>>(d_X, P->nv, dp, P->dgnorm.p); }
 	{ HA_LAUNCH(kHaB200KGrid, st); k_dg_scaled<<<(P->count + 7) / 8, kBlock, 0, st>>>(P->off.p, P->idx.p, P->count, P->nv, dp.models, P->dgnorm.p, P->dgscaled.p); }
 	HA_CUDA(cudaGetLastError());
 	scaled.resize((size_t)P->count);
@@ -2199,7 +2201,7 @@ int dgrid_plan(HaB200Plan *P, std::vector<SlWork> work, const DgParams &dp, DgPl
 	pl.tt = dg_tiles_of(max_te);
 	pl.rows = (dp.nov + kDgRows - 1) / kDgRows;
 	// two penalties' predictions need about the scratch that the eigen solves had
-	pl.na = std::max(1, std::min({2, dp.n_alphas, 65535 / std::max(1, dp.n_npcs)}));
+	pl.na = std::max(1, std::min(2, dp.n_alphas));
 	std::vector<DgItem> items;
 	std::vector<EigWork> eig;
 	std::vector<int32_t> slot;
@@ -2359,7 +2361,7 @@ int dgrid_tiles(HaB200Plan *P, const std::vector<SlWork> &work, const double *d_
 			for (int a0 = 0; a0 < dp.n_alphas; a0 += pl.na) {
 				const int ca = std::min(pl.na, dp.n_alphas - a0);
 				if (pl.tt) { HA_LAUNCH(kHaB200KGrid, bs); k_dg_eval<<<dim3(pl.tt * tn, ca, cnt * dp.models), kDgThreads, kDgSmem, bs>>>(ci, sl, S, dp, a0); }
-				if (pl.rows) { HA_LAUNCH(kHaB200KGrid, bs); k_dg_cost<<<dim3(cnt, ca * dp.n_npcs, pl.rows), kBlock, 0, bs>>>(sl + i, S, dp, a0); }
+				if (pl.rows) { HA_LAUNCH(kHaB200KGrid, bs); k_dg_cost<<<dim3(ca * dp.n_npcs, cnt, pl.rows), kBlock, 0, bs>>>(sl + i, S, dp, a0); }
 			}
 			{ HA_LAUNCH(kHaB200KGrid, bs); k_dg_best<<<cnt, kBlock, 0, bs>>>(sl + i, P->idx.p, d_Y, S, dp, d_best, d_cost); }
 			{ HA_LAUNCH(kHaB200KGrid, bs); k_dg_beta<<<dim3(tn * tn, cnt), kDgThreads, kDgSmem, bs>>>(it, sl + i, S, dp, d_best, nullptr, 0.0f, P->scrT64.p, rowmajor); }

@@ -77,11 +77,11 @@ struct DgSl {
 	int32_t sofs, pad_;
 };
 
-// Squared norms of X's columns over the distinct training rows of models m0, m0 + 1, .. (with their
-// multiplicities), a warp a (vertex, model).
-__global__ void __launch_bounds__(256) k_dg_norms(const double *__restrict__ X, int nv, const DgParams dp, int m0,
+// Squared norms of X's columns over every model's distinct training rows (with their multiplicities), a warp
+// a (vertex, model).
+__global__ void __launch_bounds__(256) k_dg_norms(const double *__restrict__ X, int nv, const DgParams dp,
                                                   double *__restrict__ norms) {
-	const int v = (int)blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, m = m0 + (int)blockIdx.y;
+	const int v = (int)blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, m = (int)blockIdx.y;
 	if (v >= nv) return;
 	const DgModel md = dp.mdl[m];
 	const double *x = X + (int64_t)v * dp.nt;
@@ -430,14 +430,14 @@ __global__ void __launch_bounds__(kDgThreads) k_dg_eval(const DgItem *__restrict
 	emit(dp.n_npcs);
 }
 
-// Squared error of kDgRows several-model rows (blockIdx.z) of one searchlight at one grid point
-// (penalty a0 + blockIdx.y / n_npcs), a warp a row: one more partial of the grid point.
+// Squared error of kDgRows several-model rows (blockIdx.z) of one searchlight (blockIdx.y) at one grid point
+// (penalty a0 + blockIdx.x / n_npcs), a warp a row: one more partial of the grid point.
 constexpr int kDgRows = 16;
 __global__ void __launch_bounds__(256) k_dg_cost(const DgSl *__restrict__ sls, double *S, const DgParams dp, int a0) {
 	__shared__ double red[32];
-	const DgSl sl = sls[blockIdx.x];
+	const DgSl sl = sls[blockIdx.y];
 	const int n = sl.n, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const double *P = S + sl.pov + (int64_t)blockIdx.y * dp.entries * n, *Yov = S + sl.yov;
+	const double *P = S + sl.pov + (int64_t)blockIdx.x * dp.entries * n, *Yov = S + sl.yov;
 	double s = 0.0;
 	for (int u = kDgRows * blockIdx.z + warp; u < min(kDgRows * ((int)blockIdx.z + 1), dp.nov); u += 8) {
 		const int e0 = dp.ovptr[u], e1 = dp.ovptr[u + 1];
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(256) k_dg_cost(const DgSl *__restrict__ sls, d
 	}
 	s = grid_block_sum(s, red);
 	if (threadIdx.x == 0)
-		S[sl.part + ((int64_t)a0 * dp.n_npcs + blockIdx.y) * sl.nparts + sl.nparts - gridDim.z + blockIdx.z] = s;
+		S[sl.part + ((int64_t)a0 * dp.n_npcs + blockIdx.x) * sl.nparts + sl.nparts - gridDim.z + blockIdx.z] = s;
 }
 
 // The grid points' costs (their partials in order, a warp a grid point), the winner (first minimum of the

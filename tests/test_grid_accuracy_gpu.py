@@ -216,3 +216,33 @@ def test_learned_form_on_badly_scaled_columns(gpu, r):
     c.plan.ridge_grid_device(c.dX.data_ptr(), c.dY.data_ptr(), vals.data_ptr(), best.data_ptr(), alphas, npcs, c.train, c.test)
     assert v.tobytes() == vals.cpu().numpy().tobytes() and choice.tobytes() == best.cpu().numpy().tobytes()
     c.plan.close()
+
+
+def _grid_costs(X, Y, alphas, npcs, train, test):
+    from hyperalignment_b200 import hyperalignment_c as H
+    sls = [np.arange(X.shape[1], dtype=np.int32)]
+    indptr, indices = H.sparse_pattern(sls, X.shape[1])
+    data = np.zeros(indices.size)
+    best, costs = H.searchlight_ridge_grid(X, Y, sls, indptr, indices, data, alphas, npcs, train, test, return_costs=True)
+    return data, int(best[0]), costs.reshape(len(alphas), len(npcs))
+
+
+def test_more_pc_counts_than_a_launch_dimension(gpu):
+    """70,000 PC counts (a launch's second dimension holds 65,535): the repeated ones add no component."""
+    rng = np.random.default_rng(2)
+    X, Y = rng.standard_normal((60, 6)), rng.standard_normal((60, 6))
+    train, test = [np.arange(40, dtype=np.int32)] * 2, [np.arange(40, 56, dtype=np.int32), np.arange(48, 60, dtype=np.int32)]
+    d0, b0, c0 = _grid_costs(X, Y, np.array([0.5, 2.0]), [3], train, test)
+    d1, b1, c1 = _grid_costs(X, Y, np.array([0.5, 2.0]), [3] * 70000, train, test)
+    assert (c1 == c0).all() and b1 == b0 * 70000 and d1.tobytes() == d0.tobytes()
+
+
+def test_more_models_than_a_launch_dimension(gpu):
+    """65,537 models of the same rows give one model's fit (their mean: 65,537 additions of float64)."""
+    rng = np.random.default_rng(2)
+    X, Y = rng.standard_normal((12, 3)), rng.standard_normal((12, 3))
+    train, test = np.arange(8, dtype=np.int32), np.arange(8, 12, dtype=np.int32)
+    d0, _, c0 = _grid_costs(X, Y, np.array([1.0]), [3], [train], [test])
+    d1, _, c1 = _grid_costs(X, Y, np.array([1.0]), [3], [train] * 65537, [test] + [test[:0]] * 65536)
+    np.testing.assert_allclose(c1, c0, rtol=1e-10)
+    np.testing.assert_allclose(d1, d0, rtol=1e-10, atol=1e-12)
