@@ -246,3 +246,57 @@ def test_more_models_than_a_launch_dimension(gpu):
     d1, _, c1 = _grid_costs(X, Y, np.array([1.0]), [3], [train] * 65537, [test] + [test[:0]] * 65536)
     np.testing.assert_allclose(c1, c0, rtol=1e-10)
     np.testing.assert_allclose(d1, d0, rtol=1e-10, atol=1e-12)
+
+
+@pytest.mark.parametrize("csr", [False, True])
+def test_small_scratch_batches_match_one_batch(gpu, monkeypatch, csr):
+    """With 2 MB of grid scratch (HA_B200_GRID_GB) the searchlights of a chunk are worked off in many batches, some
+    of one searchlight: features, winners, costs, values and the learned form's choices keep their bits, since every
+    searchlight is computed by itself.  Some searchlights are badly scaled, and some proposals fall back."""
+    import ctypes
+    import torch
+    from hyperalignment_b200 import _lib as L
+    rng = np.random.default_rng(21)
+    nv, nt, out = 200, 110, L.OUT_CSR if csr else L.OUT_CSC
+    X = rng.standard_normal((nt, nv))
+    X[:, 7::40] *= 50.0
+    Y = 0.3 * X + rng.standard_normal((nt, nv))
+    sizes = np.concatenate([rng.integers(1, 90, 40), [200, 64, 65]])
+    idx = np.concatenate([np.sort(rng.choice(nv, n, replace=False)) if k % 3 else np.setdiff1d(np.arange(nv), np.arange(7, nv, 40))[:n]
+                          for k, n in enumerate(sizes)]).astype(np.int32)
+    off = np.concatenate([[0], np.cumsum([min(n, 195) if k % 3 == 0 else n for k, n in enumerate(sizes)])]).astype(np.int32)
+    S = sizes.size
+    alphas, npcs = np.array([1e-2, 1.0, 100.0]), [5, 20, 1 << 30]
+    train = [rng.integers(0, nt, 90).astype(np.int32) for _ in range(3)]
+    test = [np.setdiff1d(np.arange(nt), t).astype(np.int32) for t in train]
+    fit = rng.integers(0, nt, 100).astype(np.int32)
+    prm = torch.zeros(L.lib().ha_b200_mlp_param_count(9), dtype=torch.float32, device="cuda")
+    assert L.lib().ha_b200_mlp_init(ctypes.c_void_p(prm.data_ptr()), 9, 5) == 0
+    prm *= 8.0
+    dX, dY = upload(X), upload(Y)
+
+    def run(thr):
+        plan = Plan(nt, nv, idx, off, weights=np.ones(idx.size))
+        f = torch.zeros((S, 65), dtype=torch.float32, device="cuda")
+        plan.ridge_features_device(dX.data_ptr(), fit, f.data_ptr())
+        v = torch.zeros(plan.nnz, dtype=torch.float64, device="cuda")
+        best = torch.full((S,), -1, dtype=torch.int32, device="cuda")
+        cost = torch.zeros((S, 9), dtype=torch.float64, device="cuda")
+        plan.ridge_grid_device(dX.data_ptr(), dY.data_ptr(), v.data_ptr(), best.data_ptr(), alphas, npcs, train, test,
+                               d_cost=cost.data_ptr(), out_kind=out)
+        lv = torch.zeros_like(v)
+        choice = torch.full((S,), -1, dtype=torch.int32, device="cuda")
+        prob = torch.zeros(S, dtype=torch.float32, device="cuda")
+        plan.ridge_learned_device(dX.data_ptr(), dY.data_ptr(), fit, alphas, npcs, prm.data_ptr(), thr, train, test,
+                                  lv.data_ptr(), choice.data_ptr(), prob.data_ptr(), out_kind=out)
+        res = [t.cpu().numpy() for t in (f, v, best, cost, lv, choice, prob)]
+        plan.close()
+        return res
+
+    thr = float(np.median(run(2.0)[-1]))
+    one = run(thr)
+    monkeypatch.setenv("HA_B200_GRID_GB", "0.002")
+    many = run(thr)
+    assert 0 < (one[-1] < thr).sum() < S
+    for a, b in zip(one, many):
+        assert np.isfinite(a).all() and a.tobytes() == b.tobytes()
