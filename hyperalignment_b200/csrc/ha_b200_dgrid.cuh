@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(256) k_dg_norms(const double *__restrict__ X, 
 }
 
 // Whether the nonzero columns of a searchlight differ in norm by more than kDgMaxScale over the rows of some
-// model, or are not finite, a warp a searchlight.  The tridiagonal reduction's error is eps ||G||, whatever
+// model, or are not finite (or beyond the range below), a warp a searchlight.  The tridiagonal reduction's error is eps ||G||, whatever
 // a column's own size, and the kernel matrix keeps no column scale at all, so both lose the square of the
 // ratio; pivoted Cholesky and one-sided Jacobi are accurate relative to every column and take such
 // searchlights.  Error of beta at alpha = 1e-3, tile products / Jacobi, median over ten draws of 120 x 60,
@@ -104,7 +104,9 @@ __global__ void __launch_bounds__(256) k_dg_norms(const double *__restrict__ X, 
 // 6.2e-14 and 1.7e-10 / 9.4e-12 at 32; at 1e4 up to 1e-4 / 2e-8.  z-scored series lie below 2 over the rows of
 // a bootstrap and series with a standard deviation of 1.02-6.1 over the sphere below 6.1; the way by Jacobi
 // takes nine times as long (512 searchlights of 50-500 vertices: 835 against 89 ms).
-constexpr double kDgMaxScale = 8.0;
+// So do searchlights whose squared norms leave 1e-100 .. 1e100: the reduction squares entries of G, which from
+// 2^256 times unit columns on overflowed (and at 2^-270 vanished); Jacobi gives the same bits there up to 2^500.
+constexpr double kDgMaxScale = 8.0, kDgMinNorm = 1e-100, kDgMaxNorm = 1e100;
 __global__ void __launch_bounds__(256) k_dg_scaled(const int32_t *__restrict__ off, const int32_t *__restrict__ sl_idx, int count,
                                                    int nv, int models, const double *__restrict__ norms,
                                                    int32_t *__restrict__ scaled) {
@@ -117,13 +119,13 @@ __global__ void __launch_bounds__(256) k_dg_scaled(const int32_t *__restrict__ o
 			const double x = norms[(int64_t)m * nv + sl_idx[i]];
 			if (x > 0.0) mn = fmin(mn, x);
 			mx = fmax(mx, x);
-			bad = bad || !isfinite(x);
+			bad = bad || !(x <= kDgMaxNorm);
 		}
 		for (int o = 16; o > 0; o >>= 1) {
 			mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
 			mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
 		}
-		bad = bad || mx > kDgMaxScale * kDgMaxScale * mn;
+		bad = bad || mx > kDgMaxScale * kDgMaxScale * mn || (mx > 0.0 && mx < kDgMinNorm);
 	}
 	bad = __any_sync(0xffffffffu, bad);
 	if (lane == 0) scaled[s] = bad ? 1 : 0;

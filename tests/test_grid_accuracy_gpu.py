@@ -300,3 +300,20 @@ def test_small_scratch_batches_match_one_batch(gpu, monkeypatch, csr):
     assert 0 < (one[-1] < thr).sum() < S
     for a, b in zip(one, many):
         assert np.isfinite(a).all() and a.tobytes() == b.tobytes()
+
+
+@pytest.mark.parametrize("k", [150, 180, 270, 500])
+def test_grid_search_at_the_ends_of_the_number_range(gpu, k):
+    """X times 2^k with the penalties times 4^k: the same costs and winners, beta times 2^-k, to the bound of the
+    search (powers of two are exact; the largest and smallest go through another eigen solver)."""
+    rng = np.random.default_rng(0)
+    X = rng.standard_normal((100, 70))
+    Y = 0.3 * X + rng.standard_normal((100, 70))
+    train = [rng.integers(0, 60, 60).astype(np.int32) for _ in range(2)]
+    test = [np.arange(60, 90, dtype=np.int32), np.arange(80, 100, dtype=np.int32)]
+    alphas, npcs = np.array([1e-2, 1.0, 30.0]), [5, 20, 70]
+    d0, b0, c0 = _grid_costs(X, Y, alphas, npcs, train, test)
+    for c in (2.0 ** k, 2.0 ** -k):
+        d, b, cost = _grid_costs(X * c, Y, alphas * c * c, npcs, train, test)
+        np.testing.assert_allclose(cost, c0, rtol=1e-8)
+        assert b == b0 and np.linalg.norm(d * c - d0) <= 1e-8 * np.linalg.norm(d0)
