@@ -719,7 +719,7 @@ def run_b200(args):
         peak = float(peaks.get("bf16_tflops_sustained", peaks.get("bf16_tflops")))
         executed = tc_executed_flops(sizes, tc_iters) * KT / max(1, cnt[dom]) / (avg_ms / 1e3)
         useful = 23.0 * float((sizes.astype(np.float64) ** 3).sum()) * KT / max(1, cnt[dom]) / (avg_ms / 1e3)
-        roof = {"bound": "tensor", "kernel": "tc_ns (k_tc_gemm Gram + update, k_tc_ns_init)", "achieved": achieved / 1e12,
+        roof = {"bound": "tensor", "kernel": "tc_ns (k_tc_resident, k_tc_wide, k_tc_ns_init, k_tc_ns_finish)", "achieved": achieved / 1e12,
                 "peak": peak, "unit": "TFLOP/s", "frac": achieved / 1e12 / peak, "traffic": None,
                 "peak_source": f"{peak_src} bf16 sustained",
                 "algorithmic": "12 n^3 tensor flops per searchlight and iteration (two n^3 products, three FP16 "

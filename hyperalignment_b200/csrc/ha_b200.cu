@@ -405,7 +405,7 @@ struct HaB200Plan {
 	DevArr<int64_t> gbase;
 	DevArr<int32_t> gnpcs, grows, gtpos, gurows, guntested;
 	DevArr<GridModel> gmdl;
-	// float64 grid search: work lists and the CV description of its kernels; scratch of the eigen solves
+	// float64 grid search: work lists and the CV description of its kernels
 	std::vector<DgModel> dg_models;
 	DevArr<DgItem> dgitem;
 	DevArr<DgSl> dgsl;
@@ -413,7 +413,7 @@ struct HaB200Plan {
 	DevArr<int32_t> dgslot;
 	DevArr<DgModel> dgmdl;
 	DevArr<int32_t> dgint;
-	DevArr<double> dgdbl, eigscr;
+	DevArr<double> dgdbl;
 	DevArr<double> dgnorm;     // squared column norms per model
 	DevArr<int32_t> dgscaled;  // per searchlight: badly scaled
 	DevArr<int32_t> gfit;      // fit rows of the learned form / the features
@@ -988,8 +988,9 @@ int polar_solve(PolarBufs &pb, std::vector<PolarWork> &items, const double *B, d
 // largest |1 - sigma^2| is then below 1e-4 sqrt(n); the final step squares it.
 double ns_tol() { return env_double("HA_B200_NS_TOL", 1e-4, 1e-7, 1e-1); }
 
-// One launch per phase and iteration (default), or the persistent solve (HA_B200_TC_PERSIST=1: one
-// CTA runs whole searchlights, their planes stay in L2; measured 3% slower on the template pair).
+// HA_B200_TC_PERSIST=1: in place of the resident and wide kernels the persistent solve, one CTA running
+// whole searchlights whose planes stay in L2 (3% slower on the template pair than one launch per phase
+// and iteration, HA_B200_TC_RESIDENT=0, which the resident and wide kernels beat in turn).
 bool tc_persistent() {
 	static int v = -1;
 	if (v < 0) {
@@ -2074,7 +2075,6 @@ int dgrid_upload(HaB200Plan *P, const GridSpec &gs, cudaStream_t st, DgParams &d
 	int entries = 0;
 	auto distinct = [&](DgModel &d, const int32_t *tr, int n) {
 		d = {};
-		d.tr_n = n;
 		d.d_ofs = (int32_t)drow.size();
 		std::fill(count.begin(), count.end(), 0);
 		for (int i = 0; i < n; i++) count[tr[i]]++;
@@ -3492,7 +3492,7 @@ void ha_b200_plan_destroy(HaB200Plan *P) {
 	P->grows.release(); P->gtpos.release(); P->gurows.release(); P->guntested.release(); P->gmdl.release();
 	P->gfit.release(); P->gfeat.release(); P->gwork.release();
 	P->dgitem.release(); P->dgsl.release(); P->dgeig.release(); P->dgslot.release(); P->dgmdl.release();
-	P->dgint.release(); P->dgdbl.release(); P->eigscr.release(); P->dgnorm.release(); P->dgscaled.release();
+	P->dgint.release(); P->dgdbl.release(); P->dgnorm.release(); P->dgscaled.release();
 	P->tcXb.release(); P->tcYb.release(); P->tcXp.release(); P->tcXq.release(); P->tcPp.release(); P->tcA.release(); P->tcRes.release();
 	P->tcSt.release(); P->tcSched.release(); P->tcPlain.release(); P->tcQueue.release();
 	if (P->grid_graph) cudaGraphExecDestroy(P->grid_graph);

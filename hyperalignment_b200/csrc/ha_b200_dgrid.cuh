@@ -17,6 +17,7 @@
 //   * a grid point's cost is accumulated in the registers that hold the predictions (they start at
 //     -Y, and every PC chunk adds its components), so predictions go to memory only for the rows that
 //     several models test, whose average is formed afterwards.
+// Badly scaled searchlights are left to ha_b200_grid.cuh (k_dg_scaled).
 // All products are 64 x 64 tiles, one CTA a tile.  512 searchlights of 50-500 vertices, 500 rows, 5 folds,
 // 10 penalties x 4 PC counts: 89 ms (eigen solves 41, evaluation 28, other products 17); one CTA a
 // searchlight with Jacobi eigen solves on the n x n Gram matrices took 835 ms, and its costs were up to
@@ -33,7 +34,7 @@ namespace hab200 {
 // terow / tew [te_ofs, te_ofs + te_n), the te1 rows that no other model tests first.  The others are the
 // searchlight's entries entry0, entry0 + 1, .. of predictions to be averaged.
 struct DgModel {
-	int32_t d_ofs, d_n, te_ofs, te_n, te1, tr_n, entry0, pad_;
+	int32_t d_ofs, d_n, te_ofs, te_n, te1, entry0;
 };
 
 struct DgParams {

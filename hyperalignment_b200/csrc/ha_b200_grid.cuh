@@ -1,6 +1,7 @@
-// ha_b200_grid.cuh -- per-searchlight ridge grid search with cross-validated ensembles, the plain FP32
-// form: the kernels are templated on the arithmetic type Real and instantiated with float (inputs,
-// alphas and the output betas stay float64).  The float64 search is ha_b200_dgrid.cuh.
+// ha_b200_grid.cuh -- per-searchlight ridge grid search with cross-validated ensembles by pivoted Cholesky
+// and one-sided Jacobi.  The kernels are templated on the arithmetic type Real: float for the plain FP32
+// search (inputs, alphas and the output betas stay float64), double for the searchlights of the float64
+// search whose columns are badly scaled; ha_b200_dgrid.cuh solves the others.
 //
 // Composition of the reference's ha_ridge_grid (csrc/ha_ridge.c:97-227) and ha_ensemble_ridge
 // (csrc/ha_ridge.c:229-345) applied to every searchlight: X = X[:, sl] and the searchlight's n

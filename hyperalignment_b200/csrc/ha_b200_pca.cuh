@@ -23,7 +23,7 @@
 
 namespace hab200 {
 
-constexpr int kPcaMaxM = 512;  // Gram order limit (kEigMaxP)
+constexpr int kPcaMaxM = 512;  // Gram order limit (the pivoted Cholesky's rank arrays and the widest Jacobi instance)
 
 // Per-searchlight scratch of the PCA template (float64 elements from the searchlight's base):
 // tmpl (nt x n), M (nt x n), then a work area that first holds the gathered X (nt x m) and the

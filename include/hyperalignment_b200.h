@@ -180,8 +180,10 @@ int ha_searchlight_ridge_csc_b200(
  * model-averaged beta (n_s x n_s) is scattered like ha_searchlight_ridge_csc_b200.  PC chunks
  * follow the reference: [npcs[p-1], npcs[p]) clipped at min(train rows, n_s), summed over p.
  * cost_out (count x n_alphas x n_npcs float64, may be NULL) receives every grid cost.
- * Computed in float64 (eigen decomposition of the smaller side's Gram of the distinct training rows by
- * tridiagonalisation and implicit QL).  kHaErrorArg for
+ * Computed in float64: eigen decomposition of the smaller side's Gram of the distinct training rows by
+ * tridiagonalisation and implicit QL; for a searchlight whose nonzero columns differ in norm by more
+ * than 8 over some model's rows (or lie beyond about 1e-50 .. 1e50), of X^T X by pivoted Cholesky and one-sided
+ * Jacobi, which keeps small columns' accuracy and takes about nine times as long.  kHaErrorArg for
  * negative PC counts, non-finite alphas, empty training lists, rows outside [0, nt), a row
  * repeated within one test list, or a searchlight of more than 512 vertices.
  */
@@ -291,8 +293,8 @@ int ha_b200_plan_pattern(const HaB200Plan *plan, int64_t *indptr, int32_t *indic
 int ha_b200_plan_device_pattern(const HaB200Plan *plan, const int64_t **d_indptr, const int32_t **d_indices);
 /* Searchlights of the last run that were solved in FP64, and that hit the sweep limit. */
 int ha_b200_plan_stats(const HaB200Plan *plan, int32_t *n_fp64, int32_t *n_jacobi_unconverged);
-/* Jacobi sweeps of the last run: sum over searchlights (final solve of each) and maximum (0 after a
- * float64 grid search, which has none). */
+/* Jacobi sweeps of the last run: sum over searchlights (final solve of each) and maximum (searchlights that
+ * the float64 grid search solves without Jacobi count 0). */
 int ha_b200_plan_sweep_stats(const HaB200Plan *plan, int64_t *sweeps_sum, int32_t *sweeps_max);
 /*
  * Per-searchlight solve record of the last run, searchlights [first, first + n) of its last
@@ -325,7 +327,8 @@ int ha_b200_plan_ridge_device(
 /*
  * Ridge grid search on device-resident data (conventions of ha_b200_plan_ridge_device; grid and
  * CV lists in host memory as ha_searchlight_ridge_grid_b200).  d_best (count int32) and d_cost
- * (count x n_alphas x n_npcs float64, may be NULL) are DEVICE memory, overwritten.
+ * (count x n_alphas x n_npcs float64, may be NULL) are DEVICE memory, overwritten.  Waits for the work
+ * that is already on the stream; fails on a stream that is being captured.
  */
 int ha_b200_plan_ridge_grid_device(
 	HaB200Plan *plan, const double *d_X, const double *d_Y,
@@ -461,7 +464,7 @@ enum {
 	kHaB200KJacobi32 = 3,   /* Jacobi polar, float32 */
 	kHaB200KFormT32 = 4,    /* T = U V^T for blocked float32 searchlights */
 	kHaB200KXcov64 = 5,
-	kHaB200KJacobi64 = 6,
+	kHaB200KJacobi64 = 6,   /* Jacobi, float64, and the grid's tridiagonal eigen solves */
 	kHaB200KFormT64 = 7,
 	kHaB200KRefine = 8,     /* Newton-Schulz orthogonality refinement */
 	kHaB200KReflect = 9,    /* det(T) < 0 fix */
