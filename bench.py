@@ -1662,8 +1662,8 @@ def run_pca(args):
                 "path": "ha_searchlight_pca_template_b200, wall clock per call"},
         "kernel_ms_per_step": {L.KERNEL_KINDS[i]: round(float(kms[i]), 3) for i in range(len(L.KERNEL_KINDS))
                                if kcnt[i] > 0},
-        "kernel_kinds": "pca: k_pca_gram, k_pca_tmpl, k_pca_contrib, k_pca_reduce; ridge: k_pchol; jacobi64: "
-                        "k_jacobi<double> (eigenvector mode on the Gram factors, then the polar); formT64: "
+        "kernel_kinds": "pca: k_pca_*, k_polar_*; ridge: k_pchol; jacobi64: k_jacobi<double> (eigenvector mode on the "
+                        "Gram factors, then the polar of the flagged searchlights); formT64: "
                         "k_form_t_global<double>",
         "error_vs_oracle": {"template_relfrob": err, "sample": int(sub.count)},
         "cpu_baseline": {"value": sub.count / cpu_s, "unit": "searchlights/s", "cores": int(blas), "kind": "port",
